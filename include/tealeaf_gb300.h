@@ -210,10 +210,10 @@ int tea_gb300_configure(int halo_depth, int solver, int preconditioner,
  * value. */
 int tea_gb300_set_arithmetic(int form);
 /* How the driver's device-resident CG loop runs (TEA_DRIVER_RESIDENT):
- * 0 (default) and 1 replay batches of iterations, three kernels each, from a
- * CUDA graph; 2 runs the whole loop as one cooperative (persistent) launch
- * with grid barriers between its phases.  The results are identical; on
- * GB300 the persistent launch measured no faster at 512^2 to 4096^2.
+ * 1 replays batches of iterations, two kernels each, from a CUDA graph; 2 runs
+ * the whole loop as one cooperative (persistent) launch with two grid barriers
+ * per iteration; 0 (default) takes 2 on small and middle grids and 1 on large
+ * ones, whichever measured faster.  The results are identical.
  * Returns 0, or -1 for another value. */
 int tea_gb300_set_resident_mode(int mode);
 int tea_gb300_get_arithmetic(void);

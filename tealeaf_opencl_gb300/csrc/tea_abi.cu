@@ -232,7 +232,8 @@ static void free_chunk(Chunk& c) {
   cudaFree(c.r2.base);
   cudaFree(c.sd2.base);
   cudaFree(c.u2.base);
-  c.r2 = c.sd2 = c.u2 = Field();
+  cudaFree(c.p2.base);
+  c.r2 = c.sd2 = c.u2 = c.p2 = Field();
   c.pending_inner = -1;
   tb_release();
   if (c.stream) cudaStreamDestroy(c.stream);
@@ -409,6 +410,7 @@ bool ensure_alt_fields(Chunk& c) {
 }
 
 bool ensure_u_alt(Chunk& c) { return c.u2.base || alloc_field(c, c.u2); }
+bool ensure_p_alt(Chunk& c) { return c.p2.base || alloc_field(c, c.p2); }
 
 void swap_alt_fields(Chunk& c) {
   std::swap(c.r, c.r2);

@@ -1,0 +1,558 @@
+// The device-resident CG loop as one cooperative launch: tea_solve.f90:270-330
+// with w = A p, the u/r/z update and p = z + beta p of tea_leaf_cg_cl.cl
+// folded into two passes per iteration.
+//
+//   pass A  p' = z + beta p formed where w = A p' needs it (own cells and the
+//           cells around them), u += alpha p of the iteration before, w and
+//           the tile sums of p'.w
+//   pass B  r -= alpha w, z = M^-1 r, the tile sums of r.z
+//
+// Every value is computed by the expressions of the three kernels of the
+// graph loop from the same operands, and every sum takes the fixed order of
+// tea_device.cuh, so the results are theirs bit for bit.
+#include <string.h>
+
+#include <algorithm>
+
+#include "tea_cg.cuh"
+#include "tea_device.cuh"
+
+namespace tea {
+
+namespace {
+
+constexpr int kLoopThreads = 512;               // one block per SM, 128 registers
+constexpr int kLoopWarps = kLoopThreads / 32;
+constexpr int kLoopSlots = kLoopWarps / kTilesPerSuper;  // supertiles in flight
+constexpr int kLoopBatch = 4;                   // rounds whose tile sums share a sweep
+
+// why the loop left
+enum { kStopConverged = 1, kStopLoopMax, kStopLaunch, kStopPw, kStopRz };
+
+struct LoopShared {
+  double lanes[kLoopBatch * kLoopThreads];  // lane sums of a batch of rounds
+  double tiles[kLoopBatch * kLoopWarps];    // its tile sums, supertile by supertile
+  double alpha, beta;
+  int go;      // barrier passed
+  int stop;    // the loop ends after this iteration
+};
+
+// t + 0.0 without the FP64 pipe: only -0 changes (a signalling NaN, which no
+// arithmetic makes, would be quieted)
+__device__ __forceinline__ double plus_zero(double t) {
+  const long long b = __double_as_longlong(t);
+  return __longlong_as_double(b == (long long)0x8000000000000000ull ? 0 : b);
+}
+
+// The least non-negative x with sqrt(x) >= t, so that sqrt(x) < t can be
+// tested without the square root (monotonic), or -1 where t^2 leaves the
+// normal range and the root must be taken.
+__device__ __forceinline__ double square_limit(double t) {
+  double x = t * t;
+  if (!(x > 1e-290 && x < 1e290)) return -1.0;
+  for (int k = 0; k < 16 && sqrt(x) >= t; k++)
+    x = __longlong_as_double(__double_as_longlong(x) - 1);
+  for (int k = 0; k < 32 && sqrt(x) < t; k++)
+    x = __longlong_as_double(__double_as_longlong(x) + 1);
+  return sqrt(x) >= t && sqrt(__longlong_as_double(__double_as_longlong(x) - 1)) < t ? x : -1.0;
+}
+
+template <int F>
+__device__ __forceinline__ double p_next(double beta, double p, double z) {
+  return F ? __fma_rn(beta, p, z) : z + beta * p;
+}
+
+// Pass A on one tile: lane column x, rows y0 .. y0+TH-1.  p' of the rows
+// above and below and of the columns either side is formed here too (the
+// two columns by lanes 0-7, one multiply-add for four rows), so no pass and
+// no grid barrier separates p' from w.  Halo cells keep the p they were given
+// (they are read from d.p whichever buffer is current).  On the first
+// iteration of a launch p is current already (it stays in pin, or with COPY
+// goes to pout as it is) and u has nothing pending.
+// p and z are written by other SMs during the launch: they are read through
+// L2.  All loads of four rows are issued before anything waits for one; rows
+// past the interior are clamped to the halo row above it and lanes past the
+// last column read the row's padding, and neither is used.
+template <int TH, int F, bool COPY = false>
+__device__ __forceinline__ double loop_w_tile(const Dev& d, const double* __restrict__ pin,
+                                              double* __restrict__ pout,
+                                              const double* __restrict__ zsrc, int x, int y0,
+                                              double alpha, double beta, bool first) {
+  const int lane = threadIdx.x & 31;
+  const double* __restrict__ hal = d.p;
+  const double* __restrict__ kx = d.Kx;
+  const double* __restrict__ ky = d.Ky;
+  const double* __restrict__ dg = d.diag;
+  double* __restrict__ u = d.u;
+  double* __restrict__ w = d.w;
+  const long long S = d.S;
+  const long long c0 = cidx(d, x, y0);
+  const bool xin = x < d.x_max;
+  const int rows = min(TH, d.y_max - y0);
+  const bool top = y0 + rows == d.y_max;  // row `rows` is halo
+  const double* __restrict__ pcol = xin ? pin : hal;
+  // p' from the old p and z; halo cells keep p
+  auto fresh = [&](double po, double zv, bool in) {
+    return first || !in ? po : p_next<F>(beta, po, zv);
+  };
+  double acc = 0.0;
+  double pm = 0.0, pc = 0.0, pco = 0.0;  // p' of rows g-1 and g, old p of row g
+#pragma unroll 1
+  for (int g = 0; g < rows; g += 4) {
+    const bool bottom = TH == 4 || g == 0;
+    double po[6], zv[6], uv[4], kyv[5], kxc[4], kxe[4], dv[4];
+    const int er = min(g + (lane >> 1), rows - 1);
+    const int xe = (lane & 1) ? x - lane + 32 : x - lane - 1;
+    const bool ein = xe >= 0 && xe < d.x_max;
+    double ep = 0.0, ez = 0.0;
+#pragma unroll
+    for (int j = 0; j < 6; j++) {
+      po[j] = zv[j] = 0.0;
+      if (j < 2 && !bottom) continue;  // carried from the group below
+      const int row = min(g + j - 1, rows);
+      const bool rin = (row >= 0 || y0 > 0) && !(row == rows && top);
+      const long long c = c0 + row * S;
+      po[j] = __ldcg((rin ? pcol : hal) + c);
+      zv[j] = __ldcg(zsrc + c);
+    }
+    if (lane < 8) {
+      const long long c = cidx(d, xe, y0 + er);
+      ep = __ldcg((ein ? pin : hal) + c);
+      ez = __ldcg(zsrc + c);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const long long c = c0 + min(g + j, rows - 1) * S;
+      uv[j] = u[c];
+      kyv[j] = __ldg(ky + c);
+      kxc[j] = __ldg(kx + c);
+      kxe[j] = __ldg(kx + c + 1);
+      dv[j] = __ldg(dg + c);
+    }
+    kyv[4] = __ldg(ky + c0 + min(g + 4, rows) * S);
+    double pv[6];
+    pv[0] = pm;
+    pv[1] = pc;
+    if (!bottom) po[1] = pco;
+#pragma unroll
+    for (int j = 0; j < 6; j++) {
+      if (j < 2 && !bottom) continue;
+      const int row = min(g + j - 1, rows);
+      const bool rin = (row >= 0 || y0 > 0) && !(row == rows && top);
+      pv[j] = fresh(po[j], zv[j], rin && xin);
+    }
+    const double ev = fresh(ep, ez, ein);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const long long c = c0 + (g + j) * S;
+      const bool own = xin && g + j < rows;
+      if (own && !first)
+        u[c] = F ? __fma_rn(alpha, po[j + 1], uv[j]) : uv[j] + alpha * po[j + 1];
+      double pe = __shfl_down_sync(0xffffffffu, pv[j + 1], 1);
+      double pw = __shfl_up_sync(0xffffffffu, pv[j + 1], 1);
+      const double e = __shfl_sync(0xffffffffu, ev, 2 * j + 1);
+      const double wst = __shfl_sync(0xffffffffu, ev, 2 * j);
+      if (lane == 31) pe = e;
+      if (lane == 0) pw = wst;
+      const double kyn = j < 3 && g + j + 1 < rows ? kyv[j + 1] : kyv[4];
+      const double wv = smvp_v<F>(dv[j], kyn, kyv[j], kxe[j], kxc[j], pv[j + 1], pv[j + 2], pv[j],
+                                  pe, pw);
+      if (own) {
+        w[c] = wv;
+        if (COPY || !first) pout[c] = pv[j + 1];
+      }
+      acc = accum<F>(acc, own ? pv[j + 1] : 0.0, own ? wv : 0.0);
+    }
+    pm = pv[4];
+    pc = pv[5];
+    pco = po[5];
+  }
+  return acc;
+}
+
+// Pass B on one tile: r -= alpha w, z = M^-1 r and the lane's share of r.z
+// (cg_ur_tile_r without u, which pass A updates).  A lane reads back only
+// the r and w that it wrote itself.
+template <int TH, int F, int NV = 1>
+__device__ __forceinline__ void loop_r_tile(const Dev& d, int x, int y0, double alpha,
+                                            double* acc) {
+  double* __restrict__ r = d.r;
+  const double* __restrict__ w = d.w;
+  double* __restrict__ z = d.z;
+  const long long S = d.S;
+  if (x >= d.x_max) return;
+  const int rows = min(TH, d.y_max - y0);
+#pragma unroll 1
+  for (int g = 0; g < rows; g += 4) {
+    const long long c0 = cidx(d, x, y0 + g);
+    double rv[4], wv[4], mv[4], zv[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const long long c = c0 + min(j, rows - 1 - g) * S;
+      wv[j] = w[c];
+      rv[j] = r[c];
+      mv[j] = d.prec == PREC_JAC_DIAG ? __ldg(d.Mi + c) : 0.0;
+    }
+    if (d.prec == PREC_JAC_BLOCK) {
+      const int upper = strip_rows(d, y0 + g);
+      double bl[4], kl[4], cl[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const long long c = c0 + min(j, upper - 1) * S;
+        bl[j] = __ldg(d.bfp + c);
+        kl[j] = __ldg(d.Ky + c);
+        cl[j] = __ldg(d.cp + c);
+      }
+      const double d0 = F ? 0.0 : __ldg(d.diag + c0);
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        rv[j] = g + j >= rows ? 0.0 : F ? __fma_rn(-alpha, wv[j], rv[j]) : rv[j] - alpha * wv[j];
+      if (upper == 4)
+        strip_solve_v<F, false, true>(4, rv, bl, kl, cl, d0, zv);
+      else
+        strip_solve_v<F, false>(upper, rv, bl, kl, cl, d0, zv);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        rv[j] = F ? __fma_rn(-alpha, wv[j], rv[j]) : rv[j] - alpha * wv[j];
+        zv[j] = d.prec == PREC_JAC_DIAG ? mul_e<true>(rv[j], mv[j]) : rv[j];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (g + j < rows) {
+        r[c0 + j * S] = rv[j];
+        if (d.prec != PREC_NONE) z[c0 + j * S] = zv[j];
+        acc[0] = accum<F>(acc[0], rv[j], zv[j]);
+        if (NV > 1) acc[NV - 1] = accum<F>(acc[NV - 1], rv[j], rv[j]);
+      }
+    }
+  }
+}
+
+// Runs body(x, y0) -> lane sum over the block's supertiles and stores the
+// supertile partials.  A warp writes its lane sums to shared memory and
+// whole warps then sum four tiles each (bfly4) and four supertiles each
+// (the steps of supertile_partials4): 1.5 FP64 instructions per tile however
+// few tiles the block has.
+template <int TH, bool SUM, class Body>
+__device__ __forceinline__ void loop_pass(const Dev& d, double* partials, LoopShared& sh,
+                                          Body body) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int slot = warp / kTilesPerSuper, tile = warp % kTilesPerSuper;
+  const int nb = gridDim.x, b = blockIdx.x;
+  const int mine = b < d.ns ? (d.ns - 1 - b) / nb + 1 : 0;  // supertiles b, b+nb, ...
+  const int rounds = (mine + kLoopSlots - 1) / kLoopSlots;
+  for (int r0 = 0; r0 < rounds; r0 += kLoopBatch) {
+    const int nr = min(kLoopBatch, rounds - r0);
+    for (int k = 0; k < nr; k++) {
+      const long long s = b + (long long)nb * ((r0 + k) * kLoopSlots + slot);
+      double acc = 0.0;
+      if (s < d.ns) {
+        const int sy = (int)s / d.nsx, sx = (int)s - sy * d.nsx;
+        const int tx = sx * kTilesPerSuper + tile;
+        if (tx < d.ntx) acc = body(tx * kTileW + lane, sy * TH);
+      }
+      if (SUM) sh.lanes[k * kLoopThreads + threadIdx.x] = acc;
+    }
+    if (!SUM) continue;
+    __syncthreads();
+    if (warp < nr * (kLoopWarps / 4)) {
+      const double* a = sh.lanes + warp * 128 + lane;
+      const double t = bfly4(a[0], a[32], a[64], a[96]);
+      if ((lane & 7) == 0) sh.tiles[warp * 4 + bfly4_slot(lane)] = t;
+    }
+    __syncthreads();
+    if (warp * 4 < nr * kLoopSlots) {
+      double t = plus_zero(sh.tiles[warp * 32 + lane]);
+#pragma unroll
+      for (int off = 4; off >= 1; off >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, off);
+      const int q = warp * 4 + (lane >> 3);  // supertile of the batch
+      const long long s = b + (long long)nb * (r0 * kLoopSlots + q);
+      if ((lane & 7) == 0 && q < nr * kLoopSlots && s < d.ns) __stcg(partials + s, t);
+    }
+  }
+}
+
+// Grid barrier on a counter that only grows during the launch.  Bounded: a
+// block that polls spin_limit times, or sees another's error flag, sets the
+// flag and returns false, and the kernel must return.
+__device__ __forceinline__ bool loop_barrier(unsigned int* bar, int* err, unsigned int target,
+                                             long long spin_limit, LoopShared& sh) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int ok = 1;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    for (long long spins = 0;;) {
+      unsigned int v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      if ((int)(v - target) >= 0) break;
+      if (++spins > spin_limit || ((spins & 255) == 0 && *(volatile int*)err)) {
+        atomicExch(err, 1);
+        ok = 0;
+        break;
+      }
+    }
+    sh.go = ok;
+  }
+  __syncthreads();
+  return sh.go != 0;
+}
+
+// The reduced value (step 4 of the summation order) in lane 0 of warps 0 and
+// 1 of every block.
+__device__ __forceinline__ double loop_total(const double* partials, int ns, LoopShared& sh) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < kBlock) {
+    double a = 0.0;
+#pragma unroll 4
+    for (int k = threadIdx.x; k < ns; k += kBlock) a = a + __ldcg(partials + k);
+    sh.lanes[threadIdx.x] = a;
+  }
+  __syncthreads();
+  if (warp < 2) {
+    const double* a = sh.lanes + warp * 128 + lane;
+    const double t = bfly4(a[0], a[32], a[64], a[96]);
+    if ((lane & 7) == 0) sh.tiles[warp * 4 + bfly4_slot(lane)] = t;
+  }
+  __syncthreads();
+  double t = 0.0;
+  if (warp < 2) {
+    t = lane < 8 ? plus_zero(sh.tiles[lane]) : 0.0;
+#pragma unroll
+    for (int off = 4; off >= 1; off >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, off);
+  }
+  return t;
+}
+
+template <int TH, int F>
+__global__ void __launch_bounds__(kLoopThreads, 1)
+    k_cg_loop(Dev d, double* p2, Red red, ResState* st, unsigned int* bar, int* err,
+              long long spin_limit, unsigned int extra, int iters) {
+  __shared__ LoopShared sh;
+  double* const pw_parts = red.partials;
+  double* const rz_parts = red.partials + red.stride;
+  const double* zsrc = d.prec != PREC_NONE ? d.z : d.r;
+  const unsigned int arrivals = gridDim.x + extra;
+  unsigned int target = 0;
+  double* const alphas = st->alphas;
+  double* const betas = st->betas;
+  double rro = st->rro;  // kept up to date by thread 0
+  int n = st->n;
+  const int loop_max = st->loop_max, check = st->check;
+  const double eps_target = st->eps_target;
+  const double rr_limit = threadIdx.x == 32 ? square_limit(eps_target) : 0.0;
+  double alpha = 0.0, beta = 0.0;
+  int it = 0, stop = 0;
+  for (;; it++, n++) {
+    // p alternates between d.p and p2; the first iteration finds it in d.p
+    const double* pin = (it & 1) || !it ? d.p : p2;
+    double* pout = (it & 1) ? p2 : d.p;
+    const bool first = it == 0;
+    loop_pass<TH, true>(d, pw_parts, sh, [&](int x, int y0) {
+      return loop_w_tile<TH, F>(d, pin, pout, zsrc, x, y0, alpha, beta, first);
+    });
+    target += arrivals;
+    if (!loop_barrier(bar, err, target, spin_limit, sh)) return;
+    const double pw = loop_total(pw_parts, d.ns, sh);
+    if (threadIdx.x == 0) sh.alpha = rro / pw;
+    __syncthreads();
+    alpha = sh.alpha;
+    loop_pass<TH, true>(d, rz_parts, sh, [&](int x, int y0) {
+      double acc[1] = {0.0};
+      loop_r_tile<TH, F>(d, x, y0, alpha, acc);
+      return acc[0];
+    });
+    target += arrivals;
+    if (!loop_barrier(bar, err, target, spin_limit, sh)) return;
+    const double rrn = loop_total(rz_parts, d.ns, sh);
+    // the host steps of the iteration (cg_scalar_step): beta by thread 0, the
+    // exit test beside it by thread 32
+    if (threadIdx.x == 0) {
+      const double bt = rrn / rro;
+      sh.beta = bt;
+      if (blockIdx.x == 0) {
+        if (alphas) {
+          alphas[n] = alpha;
+          betas[n] = bt;
+        }
+      }
+      rro = rrn;
+    }
+    if (threadIdx.x == 32) {
+      const bool done = rr_limit > 0.0 ? rrn < rr_limit && rrn >= 0.0 : sqrt(rrn) < eps_target;
+      int s = done              ? kStopConverged
+              : n >= loop_max   ? kStopLoopMax
+              : it + 1 >= iters ? kStopLaunch
+                                : 0;
+      if (check) {
+        if (!(pw > 0.0) || isinf(pw))
+          s = kStopPw;
+        else if (!isfinite(rrn))
+          s = kStopRz;
+      }
+      if (blockIdx.x == 0 && s && s < kStopPw) st->error = sqrt(rrn);
+      sh.stop = s;
+    }
+    __syncthreads();
+    beta = sh.beta;
+    stop = sh.stop;
+    if (stop) break;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (stop >= kStopPw) {
+      st->breakdown = stop == kStopPw ? 1 : 2;
+      st->breakdown_n = n;
+    } else {
+      st->alpha = alpha;
+      st->beta = beta;
+      st->rro = st->rrn = rro;
+      st->converged = stop == kStopConverged;
+    }
+    st->n = stop == kStopLaunch ? n + 1 : n;
+    st->stop = stop != kStopLaunch;
+    st->p_pending = 0;
+  }
+  // u and p of the last iteration (p stays as it is after a breakdown)
+  const double* pc = (it & 1) ? p2 : d.p;
+  loop_pass<TH, false>(d, pw_parts, sh, [&](int x, int y0) {
+    if (x >= d.x_max) return 0.0;
+    const int rows = min(TH, d.y_max - y0);
+    for (int j = 0; j < rows; j++) {
+      const long long c = cidx(d, x, y0 + j);
+      const double po = __ldcg(pc + c), uv = d.u[c];
+      d.u[c] = F ? __fma_rn(alpha, po, uv) : uv + alpha * po;
+      if (stop < kStopPw) d.p[c] = p_next<F>(beta, po, __ldcg(zsrc + c));
+    }
+    return 0.0;
+  });
+}
+
+// ---- the two passes as separate kernels, for grids whose passes are long
+// beside a launch (replayed from a graph) ----
+
+// Pass A.  An iteration whose predecessor has run (p_pending) forms p' and
+// finishes u; the first one copies p, so that p alternates between the two
+// buffers whatever happens.
+template <int TH, int F>
+__global__ void __launch_bounds__(kBlock, 2)
+    k_cg_pass_w(Dev d, Red red, ResState* st, const double* pin, double* pout) {
+  if (*(volatile int*)&st->stop) return;
+  const bool first = !*(volatile int*)&st->p_pending;
+  const double alpha = st->alpha, beta = st->beta;
+  const double* zsrc = d.prec != PREC_NONE ? d.z : d.r;
+  const bool last = tile_driver<TH, 1>(d, red, [&](int x, int y0, bool, double* acc) {
+    acc[0] = loop_w_tile<TH, F, true>(d, pin, pout, zsrc, x, y0, alpha, beta, first);
+  });
+  if (last && threadIdx.x == 0) {
+    const double pw = red.result[0];
+    st->pw = pw;
+    st->alpha = st->rro / pw;
+  }
+}
+
+// Pass B and the scalar step; with NV = 2 also r.r for the exit test on the
+// unpreconditioned residual.
+template <int TH, int F, int NV>
+__global__ void __launch_bounds__(kBlock, 4) k_cg_pass_r(Dev d, Red red, ResState* st) {
+  if (*(volatile int*)&st->stop) return;
+  const double alpha = st->alpha;
+  const bool last = tile_driver<TH, NV>(d, red, [&](int x, int y0, bool, double* acc) {
+    loop_r_tile<TH, F, NV>(d, x, y0, alpha, acc);
+  });
+  if (last && threadIdx.x == 0) cg_scalar_step<NV>(st, alpha, red.result);
+}
+
+// u and p of the iteration that stopped the loop, p to d.p: it is in p2
+// after an odd number of iterations.
+template <int TH, int F>
+__global__ void __launch_bounds__(kBlock)
+    k_cg_pass_end(Dev d, Red red, ResState* st, const double* p2, unsigned int* counter) {
+  if (!*(volatile int*)&st->stop || st->ended) return;
+  const bool odd = ((st->n - st->n_first + 1) & 1) != 0;
+  const bool brk = st->breakdown != 0;
+  const double* pc = odd ? p2 : d.p;
+  const double alpha = st->alpha, beta = st->beta;
+  const double* z = d.prec != PREC_NONE ? d.z : d.r;
+  tile_driver<TH, 0>(d, red, [&](int x, int y0, bool xin, double*) {
+    if (!xin) return;
+    const int rows = min(TH, d.y_max - y0);
+    for (int j = 0; j < rows; j++) {
+      const long long c = cidx(d, x, y0 + j);
+      const double po = pc[c], uv = d.u[c];
+      d.u[c] = F ? __fma_rn(alpha, po, uv) : uv + alpha * po;
+      if (!brk) d.p[c] = p_next<F>(beta, po, z[c]);
+    }
+  });
+  if (last_block(counter) && threadIdx.x == 0) {
+    st->ended = 1;
+    st->p_pending = 0;
+  }
+}
+
+template <class... KArgs>
+int pass_grid(const LaunchCtx& l, const Dev& d, void (*kernel)(KArgs...)) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlock, 0) != cudaSuccess ||
+      per_sm < 1)
+    per_sm = 1;
+  return (int)std::max<long long>(1, std::min<long long>(d.ns, (long long)l.num_sms * per_sm));
+}
+
+template <int TH, int F, int NV>
+void enqueue_passes_t(const LaunchCtx& l, const Dev& d, double* p2, const Red& red,
+                      ResState* st, unsigned int* counter, int iters) {
+  const int gw = pass_grid(l, d, k_cg_pass_w<TH, F>);
+  const int gr = pass_grid(l, d, k_cg_pass_r<TH, F, NV>);
+  const int ge = pass_grid(l, d, k_cg_pass_end<TH, F>);
+  for (int i = 0; i < iters; i += 2) {
+    k_cg_pass_w<TH, F><<<gw, kBlock, 0, l.stream>>>(d, red, st, d.p, p2);
+    k_cg_pass_r<TH, F, NV><<<gr, kBlock, 0, l.stream>>>(d, red, st);
+    k_cg_pass_w<TH, F><<<gw, kBlock, 0, l.stream>>>(d, red, st, p2, d.p);
+    k_cg_pass_r<TH, F, NV><<<gr, kBlock, 0, l.stream>>>(d, red, st);
+  }
+  k_cg_pass_end<TH, F><<<ge, kBlock, 0, l.stream>>>(d, red, st, p2, counter);
+}
+
+template <int TH, int F>
+bool launch_loop_t(const LaunchCtx& l, Dev d, double* p2, Red red, ResState* st,
+                   unsigned int* bar, long long spin_limit, unsigned int extra, int iters) {
+  int grid = std::max(1, std::min(d.ns, l.num_sms));
+  int* err = (int*)(bar + 1);
+  void* args[] = {&d, &p2, &red, &st, &bar, &err, &spin_limit, &extra, &iters};
+  return check_cuda(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned int), l.stream),
+                    "CG loop barrier reset") &&
+         check_cuda(cudaLaunchCooperativeKernel((const void*)k_cg_loop<TH, F>, dim3(grid),
+                                                dim3(kLoopThreads), args, 0, l.stream),
+                    "CG loop launch");
+}
+
+}  // namespace
+
+void enqueue_cg_passes(const LaunchCtx& l, const Dev& d, double* p2, const Red& red,
+                       ResState* st, unsigned int* counter, int iters, bool true_exit) {
+#define TEA_PASSES(TH, NV)                                                           \
+  (l.arith == 2   ? enqueue_passes_t<TH, 2, NV>(l, d, p2, red, st, counter, iters) \
+   : l.arith == 1 ? enqueue_passes_t<TH, 1, NV>(l, d, p2, red, st, counter, iters) \
+                  : enqueue_passes_t<TH, 0, NV>(l, d, p2, red, st, counter, iters))
+  if (d.th == 16)
+    true_exit ? TEA_PASSES(16, 2) : TEA_PASSES(16, 1);
+  else
+    true_exit ? TEA_PASSES(4, 2) : TEA_PASSES(4, 1);
+#undef TEA_PASSES
+}
+
+bool launch_cg_loop(const LaunchCtx& l, const Dev& d, double* p2, const Red& red, ResState* st,
+                    unsigned int* bar, long long spin_limit, unsigned int extra) {
+  const int iters = kLoopLaunchIters;
+  count_launch("resident_cg_loop");
+  if (d.th == 16)
+    return l.arith == 2 ? launch_loop_t<16, 2>(l, d, p2, red, st, bar, spin_limit, extra, iters)
+         : l.arith == 1 ? launch_loop_t<16, 1>(l, d, p2, red, st, bar, spin_limit, extra, iters)
+                        : launch_loop_t<16, 0>(l, d, p2, red, st, bar, spin_limit, extra, iters);
+  return l.arith == 2 ? launch_loop_t<4, 2>(l, d, p2, red, st, bar, spin_limit, extra, iters)
+       : l.arith == 1 ? launch_loop_t<4, 1>(l, d, p2, red, st, bar, spin_limit, extra, iters)
+                      : launch_loop_t<4, 0>(l, d, p2, red, st, bar, spin_limit, extra, iters);
+}
+
+}  // namespace tea

@@ -70,6 +70,8 @@ struct ResState {
   int breakdown;   // 0, or 1 (p.w) / 2 (r.z) with check set
   int breakdown_n; // the iteration it happened in
   double rr_true;  // r.r of the last iteration (true-residual exit only)
+  int n_first;     // iteration the loop began at
+  int ended;       // u and p of the last iteration are in place
   double* alphas;  // indexed by iteration number n
   double* betas;
 };
@@ -122,10 +124,10 @@ struct Chunk {
   double* res_coef = nullptr;          // device alphas/betas
   int res_coef_n = 0;
   unsigned int* res_counter = nullptr;
-  unsigned int* res_bar = nullptr;     // grid barrier [2] + error flag
+  unsigned int* res_bar = nullptr;     // grid barrier: counter, error flag
   cudaGraphExec_t res_ppcg_graph = nullptr;  // resident PPCG iterations
   std::vector<double> res_ppcg_key;          // theta, coefficients, form of it
-  int resident_mode = 0;               // 0 auto, 1 graph replay, 2 persistent
+  int resident_mode = 0;               // 0 by size, 1 graph replay, 2 cooperative loop
   // second r and sd buffers for the fused pair of PPCG inner steps
   // (tea_ppcg_tb.cu), which writes r and sd to the pair it does not read;
   // allocated on first use, with the halos of the live pair
@@ -134,6 +136,7 @@ struct Chunk {
   // calc_p (block Jacobi), which writes the new u, halo included, to the
   // buffer it does not read; the two then trade places
   Field u2;
+  Field p2;  // second p buffer of the resident CG loop (tea_cg_loop.cu)
   int inner_pairs = 0;      // run PPCG inner steps in fused pairs where they apply
   int field_epoch = 0;      // bumped whenever r/sd and r2/sd2 trade places
   int pending_inner = -1;   // a per-call inner step (0-based) not launched yet
@@ -241,6 +244,19 @@ void dev_cg_init_p(const LaunchCtx& l, const Dev& d, const Red& r);
 // kernels return at once after it has stopped)
 void dev_cg_iteration(const LaunchCtx& l, const Dev& d, const Red& r, ResState* st,
                       unsigned int* counter);
+// The whole CG loop from the state in *st, at most kLoopLaunchIters
+// iterations, as one cooperative launch (tea_cg_loop.cu).  p2: a second p
+// buffer (interior only); bar: two words, the barrier's counter and its error
+// flag; red.partials holds at least two arrays of red.stride.  After it
+// st->stop is set, or the loop goes on with another launch.
+constexpr int kLoopLaunchIters = 1024;
+bool launch_cg_loop(const LaunchCtx& l, const Dev& d, double* p2, const Red& red, ResState* st,
+                    unsigned int* bar, long long spin_limit, unsigned int extra);
+// `iters` (even) iterations of the same loop as two kernels each, and the
+// kernel that finishes u and p once it has stopped, queued for a graph.
+// counter: one word, zero.
+void enqueue_cg_passes(const LaunchCtx& l, const Dev& d, double* p2, const Red& red,
+                       ResState* st, unsigned int* counter, int iters, bool true_exit);
 void dev_finalise(const LaunchCtx& l, const Dev& d, const Red& r);
 void dev_field_summary(const LaunchCtx& l, const Dev& d, const Red& r);
 // device-resident CG loop (tea_kernels.cu)
@@ -267,8 +283,9 @@ void tb_release();
 // the second r/sd buffers (tea_abi.cu): allocated and given the live
 // buffers' contents once; false on failure
 bool ensure_alt_fields(Chunk& c);
-// allocates u2 on first use
+// allocates u2 / p2 on first use
 bool ensure_u_alt(Chunk& c);
+bool ensure_p_alt(Chunk& c);
 // r/sd and r2/sd2 trade places (the fused pair has just written r2/sd2)
 void swap_alt_fields(Chunk& c);
 // launches a per-call PPCG inner step held back for pairing (tea_abi.cu)

@@ -1373,93 +1373,6 @@ static int tile_grid(Chunk& c, void (*kernel)(KArgs...), int ns = 0) {
   return (int)std::max<long long>(1, std::min<long long>(ns > 0 ? ns : c.dev().ns, cap));
 }
 
-// The whole remaining CG loop as one cooperative launch, for grids whose
-// iterations are short enough for kernel boundaries to dominate.  Every
-// block keeps the same supertiles in all three phases; grid barriers
-// separate w = A p, the u/r/z update and p = z + beta p.  After each
-// reducing phase every block forms the reduced value itself from the
-// supertile partials, in the fixed order of block_final_sum, so all blocks
-// agree bit for bit and no extra barrier is needed; block 0 keeps the loop
-// state (cg_scalar_step).  Fields written by other blocks are read through
-// L2 (CG = true).  Results are those of the three-kernel loop.
-template <int TH, int F>
-__global__ void __launch_bounds__(kBlock)
-    k_cg_persistent(Dev d, Red red, ResState* st, unsigned int* bar, int* err,
-                    long long spin_limit, unsigned int extra_arrivals) {
-  __shared__ double sh[16];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  Red rw = red, ru = red;
-  ru.partials = red.partials + red.stride;  // p.w and r.z partials apart
-  auto phase = [&](const Red& r, auto body, bool reduce) {
-    for (int s = blockIdx.x; s < d.ns; s += gridDim.x) {
-      const int sy = s / d.nsx, sx = s - sy * d.nsx;
-      const int tx = sx * kTilesPerSuper + warp;
-      double acc[1] = {0.0};
-      if (tx < d.ntx) {
-        const int x = tx * kTileW + lane;
-        body(x, sy * TH, x < d.x_max, acc);
-        if (reduce) acc[0] = bfly(acc[0]);
-      }
-      if (reduce) supertile_partial<1>(r, s, acc, sh);
-    }
-  };
-  for (;;) {
-    if (*(volatile int*)&st->stop) return;
-    const double rro = *(volatile double*)&st->rro;
-    phase(rw, [&](int x, int y0, bool xin, double* acc) {
-      cg_w_tile<TH, F, true>(d, x, y0, xin, acc);
-    }, true);
-    if (!grid_barrier(bar, err, spin_limit, extra_arrivals)) return;
-    const double pw = block_final_value(rw.partials, d.ns, sh);
-    const double alpha = rro / pw;
-    phase(ru, [&](int x, int y0, bool xin, double* acc) {
-      cg_ur_tile<TH, F, 1, true>(d, x, y0, xin, acc, alpha);
-    }, true);
-    if (!grid_barrier(bar, err, spin_limit, extra_arrivals)) return;
-    const double rrn = block_final_value(ru.partials, d.ns, sh);
-    const double beta = rrn / rro;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      st->pw = pw;
-      cg_scalar_step<1>(st, alpha, &rrn);
-      st->p_pending = 0;
-    }
-    phase(rw, [&](int x, int y0, bool xin, double* acc) {
-      cg_p_tile<TH, F, true>(d, x, y0, xin, beta);
-    }, false);
-    if (!grid_barrier(bar, err, spin_limit, extra_arrivals)) return;
-  }
-}
-
-// Cooperative launch of k_cg_persistent: as many blocks as can be resident
-// at once, at most one per supertile.  Returns false if the launch fails.
-template <int TH, int F>
-static bool launch_cg_persistent_t(Chunk& c) {
-  const void* fn = (const void*)k_cg_persistent<TH, F>;
-  const long long cap = (long long)c.num_sms * blocks_per_sm(fn);
-  const int grid = (int)std::max<long long>(1, std::min<long long>(c.dev().ns, cap));
-  Dev d = c.dev();
-  Red red = c.red();
-  ResState* st = c.res_state;
-  unsigned int* bar = c.res_bar;
-  int* err = (int*)(c.res_bar + 2);
-  long long spin_limit = c.barrier_spin_limit;
-  unsigned int extra = (unsigned int)c.barrier_extra;
-  void* args[] = {&d, &red, &st, &bar, &err, &spin_limit, &extra};
-  return check_cuda(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kBlock), args, 0,
-                                                c.stream),
-                    "persistent CG launch");
-}
-
-static bool launch_cg_persistent(Chunk& c) {
-  if (c.TH == 16)
-    return c.arith == 2 ? launch_cg_persistent_t<16, 2>(c)
-           : c.arith == 1 ? launch_cg_persistent_t<16, 1>(c)
-                          : launch_cg_persistent_t<16, 0>(c);
-  return c.arith == 2 ? launch_cg_persistent_t<4, 2>(c)
-         : c.arith == 1 ? launch_cg_persistent_t<4, 1>(c)
-                        : launch_cg_persistent_t<4, 0>(c);
-}
-
 // ---- device-resident PPCG iterations (tea_solve.f90:231-268 after the
 // switch from CG), scalars in the ResState as for CG ----
 
@@ -1599,45 +1512,9 @@ static void enqueue_ppcg_iterations(Chunk& c, int iters) {
   }
 }
 
-template <int TH, int F, int NV>
-static void enqueue_resident_iterations_t(Chunk& c, int iters) {
-  const Dev d = c.dev();
-  const Dev d4 = dev4(c);  // calc_p takes no sum
-  const Red red = c.red();
-  const int gw = tile_grid(c, k_cg_calc_w<TH, F>);
-  const int gu = tile_grid(c, k_cg_calc_ur<TH, F, NV>);
-  const int gp = tile_grid(c, k_cg_calc_p<4, F>, d4.ns);
-  for (int i = 0; i < iters; i++) {
-    k_cg_calc_w<TH, F><<<gw, kBlock, 0, c.stream>>>(d, red, c.res_state);
-    k_cg_calc_ur<TH, F, NV><<<gu, kBlock, 0, c.stream>>>(d, red, 0.0, c.res_state);
-    k_cg_calc_p<4, F><<<gp, kBlock, 0, c.stream>>>(d4, red, 0.0, c.res_state,
-                                                   c.res_counter);
-  }
-}
-
-template <int TH, int NV>
-static void enqueue_resident_iterations_th(Chunk& c, int iters) {
-  if (c.arith == 2)
-    enqueue_resident_iterations_t<TH, 2, NV>(c, iters);
-  else if (c.arith == 1)
-    enqueue_resident_iterations_t<TH, 1, NV>(c, iters);
-  else
-    enqueue_resident_iterations_t<TH, 0, NV>(c, iters);
-}
-
-template <int NV>
-static void enqueue_resident_iterations_nv(Chunk& c, int iters) {
-  if (c.TH == 16)
-    enqueue_resident_iterations_th<16, NV>(c, iters);
-  else
-    enqueue_resident_iterations_th<4, NV>(c, iters);
-}
-
 static void enqueue_resident_iterations(Chunk& c, int iters, bool true_exit) {
-  if (true_exit)
-    enqueue_resident_iterations_nv<2>(c, iters);
-  else
-    enqueue_resident_iterations_nv<1>(c, iters);
+  enqueue_cg_passes(LaunchCtx{c.stream, c.num_sms, c.arith}, c.dev(), c.p2.f, c.red(),
+                    c.res_state, c.res_counter, iters, true_exit);
 }
 
 void resident_release() {
@@ -1662,21 +1539,27 @@ void resident_release() {
 }
 
 // CG iterations n_begin..loop_max of tea_solve.f90:147-332 with all scalars
-// on the device.  The iterations are queued in batches replayed from a
-// captured CUDA graph; after each batch the host reads the loop state once.
-// Kernels queued after the loop has stopped return at once.  The arithmetic
-// and the exit test are those of the per-call path, so the results are
-// bit-identical to it.
-// The persistent loop runs when asked for (resident_mode 2).  The default
-// is the graph loop: measured per CG iteration (jac_diag, chain form), the
-// graph loop took 24.3 / 51.7 / 150 / 455 us at 512^2 / 1024^2 / 2048^2 /
-// 4096^2 and the persistent one 25.3 / 56.3 / 154 / 455 us.  At small grids
-// every phase is latency-bound either way, and three grid barriers cost
-// what three graph-replayed launches cost; removing the barrier's back-off
-// or using one block per SM changed nothing.  The persistent loop keeps the
-// r.z exit test only (the true-residual exit uses the graph loop).
-static bool use_persistent(const Chunk& c, bool true_exit) {
-  return !true_exit && !c.profiler_on && c.resident_mode == 2;
+// on the device (tea_cg_loop.cu): the whole loop as one cooperative launch, or
+// batches of iterations, two kernels each, replayed from a captured graph with
+// one read of the loop state per batch.  Kernels queued after the loop has
+// stopped return at once.  The arithmetic and the exit test are those of the
+// per-call path, so the results are bit-identical to it.
+//
+// The line between the two: a launch boundary costs a pass about 10 us (start,
+// drain, the last block's sum), a grid barrier with the sum in every block
+// about 3.5 us; but the cooperative kernel's passes share one register budget
+// (16 warps per SM), so pass B of long passes streams at 0.8 of the rate of its
+// own kernel.  us per iteration, cooperative / graph (three kernels per
+// iteration before them): 64^2 7.3 / 9.9 (11.7), 512^2 diagonal 15.3 / 21.6
+// (25.1), 960^2 33.0 / 38.9 (43.5), 1024^2 diagonal 34.7 / 39.7 (47.4),
+// 1501x1203 block 67.4 / 69.8 (71.8), 1700^2 diagonal 103 / 98, 2048^2
+// diagonal 134 / 121 (125), 4096^2 diagonal 419 / 391 (425), block 466 / 440
+// (463).  They cross between 12 and 20 supertiles per SM.  The true-residual
+// exit (r.r beside r.z) and profiling use the kernels.
+constexpr int kLoopSupertilesPerSM = 14;
+static bool use_cg_loop(const Chunk& c, bool true_exit) {
+  if (true_exit || c.profiler_on || c.resident_mode == 1) return false;
+  return c.resident_mode == 2 || c.dev().ns <= kLoopSupertilesPerSM * c.num_sms;
 }
 
 int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
@@ -1714,7 +1597,7 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
   memset(&h, 0, sizeof(h));
   h.rro = rro_in;
   h.eps_target = eps_target;
-  h.n = n_begin;
+  h.n = h.n_first = n_begin;
   h.loop_max = loop_max;
   h.check = c.solver_checks;
   h.alphas = c.res_coef;
@@ -1723,29 +1606,31 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
                                   cudaMemcpyHostToDevice, c.stream),
                   "resident state upload"))
     return -1;
-  if (use_persistent(c, true_exit)) {
-    // one cooperative launch runs the loop to its end
-    if (!check_cuda(cudaMemsetAsync(c.res_bar, 0, 3 * sizeof(unsigned int), c.stream),
-                    "barrier reset") ||
-        !launch_cg_persistent(c))
-      return -1;
-    count_launch("resident_cg_persistent");
-    int err = 0;
-    if (!check_cuda(cudaMemcpyAsync(&h, c.res_state, sizeof(ResState),
-                                    cudaMemcpyDeviceToHost, c.stream),
-                    "resident state read") ||
-        !check_cuda(cudaMemcpyAsync(&err, c.res_bar + 2, sizeof(int),
-                                    cudaMemcpyDeviceToHost, c.stream),
-                    "barrier flag read") ||
-        !check_cuda(cudaStreamSynchronize(c.stream), "persistent CG"))
-      return -1;
-    if (err) {
-      fail(25, "persistent CG: a grid barrier timed out");
-      return -1;
-    }
-    if (!h.stop) {
-      fail(24, "persistent CG loop ended before its exit test");
-      return -1;
+  if (!ensure_p_alt(c)) return -1;
+  if (use_cg_loop(c, true_exit)) {
+    const LaunchCtx l{c.stream, c.num_sms, c.arith};
+    const long long launches = (long long)(loop_max - n_begin) / kLoopLaunchIters + 2;
+    for (long long k = 0;; k++) {
+      int err = 0;
+      if (!launch_cg_loop(l, c.dev(), c.p2.f, c.red(), c.res_state, c.res_bar,
+                          c.barrier_spin_limit, (unsigned int)c.barrier_extra) ||
+          !check_cuda(cudaMemcpyAsync(&h, c.res_state, sizeof(ResState),
+                                      cudaMemcpyDeviceToHost, c.stream),
+                      "resident state read") ||
+          !check_cuda(cudaMemcpyAsync(&err, c.res_bar + 1, sizeof(int),
+                                      cudaMemcpyDeviceToHost, c.stream),
+                      "barrier flag read") ||
+          !check_cuda(cudaStreamSynchronize(c.stream), "resident CG loop"))
+        return -1;
+      if (err) {
+        fail(25, "resident CG loop: a grid barrier timed out");
+        return -1;
+      }
+      if (h.stop) break;
+      if (k >= launches) {
+        fail(24, "resident CG loop ended before its exit test");
+        return -1;
+      }
     }
   } else {
   if (!c.res_graph && !c.profiler_on) {
@@ -1777,7 +1662,7 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
       enqueue_resident_iterations(c, batch, true_exit);
       check_cuda(cudaGetLastError(), "resident launch");
     }
-    for (int i = 0; i < 3 * batch; i++) count_launch("resident_cg");
+    count_launches(2 * batch + 1);
     if (!check_cuda(cudaMemcpyAsync(&h, c.res_state, sizeof(ResState),
                                     cudaMemcpyDeviceToHost, c.stream),
                     "resident state read") ||
