@@ -28,8 +28,8 @@
 // step and u_{n+1} of the steps of the last segment; the backward pass
 // recomputes each earlier segment from its checkpoint before walking it
 // backwards.  Every solve is the device-resident CG loop of the single-chunk
-// path (dev_cg_iteration, graph-replayed), so the forward pass is
-// bit-identical to the driver's.
+// path (tea_cg_loop.cu), so the forward pass is bit-identical to the
+// driver's.
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
@@ -95,7 +95,7 @@ __global__ void k_adj_begin(ResState* st, const double* results, double eps,
   ResState s{};
   s.rro = results[0];
   s.eps_target = eps * sqrt(results[4]);
-  s.n = 1;
+  s.n = s.n_first = 1;
   s.loop_max = loop_max;
   *st = s;
 }
@@ -121,7 +121,8 @@ struct Adjoint {
   double* states = nullptr;        // checkpoints and the segment's u's
   int n_states = 0;
   double* partials = nullptr;
-  unsigned int* counters = nullptr;  // [0] reductions, [1] calc_p
+  unsigned int* counters = nullptr;  // [0] reductions, [1] end of the loop, [2..3] grid barrier
+  double* p2 = nullptr;              // second p buffer of the CG loop
   double* results = nullptr;
   ResState* st = nullptr;
   ResState* st_h = nullptr;        // pinned
@@ -208,19 +209,29 @@ long long solve(Adjoint& a, double eps, int max_iters) {
   dev_cg_init_p(l, a.d, a.red);
   k_adj_begin<<<1, 1, 0, a.stream>>>(a.st, a.red.result, eps, max_iters);
   count_launch("adjoint_begin");
-  const long long max_replays = (long long)max_iters / kReplayIters + 3;
+  const bool loop = cg_loop_fits(a.d, a.num_sms);
+  const int per_launch = loop ? kLoopLaunchIters : kReplayIters;
+  const long long max_launches = (long long)max_iters / per_launch + 3;
   for (long long nb = 0;; nb++) {
-    if (nb >= max_replays) {
-      fail(61, "adjoint: CG loop did not stop after %lld graph replays", nb);
+    if (nb >= max_launches) {
+      fail(61, "adjoint: CG loop did not stop after %lld launches", nb);
       return -1;
     }
-    if (!check_cuda(cudaGraphLaunch(a.graph, a.stream), "adjoint replay")) return -1;
-    count_launches(3 * kReplayIters);
+    if (loop) {
+      if (!launch_cg_loop(l, a.d, a.p2, a.red, a.st, a.counters + 2, kLoopSpins, 0)) return -1;
+    } else {
+      if (!check_cuda(cudaGraphLaunch(a.graph, a.stream), "adjoint replay")) return -1;
+      count_launches(2 * kReplayIters + 1);
+    }
     if (!check_cuda(cudaMemcpyAsync(a.st_h, a.st, sizeof(ResState),
                                     cudaMemcpyDeviceToHost, a.stream),
                     "adjoint state read") ||
         !check_cuda(cudaStreamSynchronize(a.stream), "adjoint solve"))
       return -1;
+    if (a.st_h->timed_out) {
+      fail(61, "adjoint: a grid barrier of the CG loop timed out");
+      return -1;
+    }
     if (a.st_h->stop && !a.st_h->p_pending) break;
   }
   return a.st_h->n;
@@ -281,7 +292,7 @@ extern "C" int tea_gb300_adjoint_create(int x_cells, int y_cells, double xmin,
   const long long S = ((long long)(x_cells + 2 + 1 + 31) / 32) * 32;
   const long long rows = y_cells + 2 + 1;
   a.fd = (size_t)((31 + rows * S + 32 + 31) / 32 * 32);
-  const int nf = 14;  // 12 solver fields, lambda, gradient
+  const int nf = 15;  // 12 solver fields, the second p, lambda, gradient
   const long long ntx = (x_cells + kTileW - 1) / kTileW;
   const long long nsx = (ntx + kTilesPerSuper - 1) / kTilesPerSuper;
   const long long stride = nsx * ((y_cells + 3) / 4) + 1;
@@ -289,8 +300,8 @@ extern "C" int tea_gb300_adjoint_create(int x_cells, int y_cells, double xmin,
       !check_cuda(cudaMemsetAsync(a.arena, 0, nf * a.fd * sizeof(double), a.stream),
                   "cudaMemset adjoint") ||
       !check_cuda(cudaMalloc(&a.partials, 4 * stride * sizeof(double)), "cudaMalloc partials") ||
-      !check_cuda(cudaMalloc(&a.counters, 2 * sizeof(unsigned int)), "cudaMalloc counters") ||
-      !check_cuda(cudaMemsetAsync(a.counters, 0, 2 * sizeof(unsigned int), a.stream),
+      !check_cuda(cudaMalloc(&a.counters, 4 * sizeof(unsigned int)), "cudaMalloc counters") ||
+      !check_cuda(cudaMemsetAsync(a.counters, 0, 4 * sizeof(unsigned int), a.stream),
                   "cudaMemset counters") ||
       !check_cuda(cudaMalloc(&a.results, 8 * sizeof(double)), "cudaMalloc results") ||
       !check_cuda(cudaMalloc(&a.st, sizeof(ResState)), "cudaMalloc state") ||
@@ -320,6 +331,7 @@ extern "C" int tea_gb300_adjoint_create(int x_cells, int y_cells, double xmin,
   d.z = next();
   d.diag = next();
   d.un = d.Mi;
+  a.p2 = next();
   a.lam = next();
   a.grad = next();
   a.d = make_dev_tiling(d);
@@ -327,7 +339,15 @@ extern "C" int tea_gb300_adjoint_create(int x_cells, int y_cells, double xmin,
   a.red.stride = stride;
   a.red.counter = a.counters;
   a.red.result = a.results;
-  // the graph of kReplayIters resident CG iterations on these fields
+  // the graph of kReplayIters resident CG iterations on these fields, for
+  // grids beyond the one-launch loop
+  if (cg_loop_fits(a.d, a.num_sms)) {
+    if (!check_cuda(cudaStreamSynchronize(a.stream), "adjoint create")) {
+      release_adjoint();
+      return -1;
+    }
+    return 0;
+  }
   const long long n0 = tea_gb300_kernel_launches();
   cudaGraph_t g = nullptr;
   if (!check_cuda(cudaStreamBeginCapture(a.stream, cudaStreamCaptureModeThreadLocal),
@@ -335,8 +355,7 @@ extern "C" int tea_gb300_adjoint_create(int x_cells, int y_cells, double xmin,
     release_adjoint();
     return -1;
   }
-  for (int i = 0; i < kReplayIters; i++)
-    dev_cg_iteration(ctx(a), a.d, a.red, a.st, a.counters + 1);
+  enqueue_cg_passes(ctx(a), a.d, a.p2, a.red, a.st, a.counters + 1, kReplayIters, false);
   const bool ok = check_cuda(cudaStreamEndCapture(a.stream, &g), "adjoint capture end") &&
                   check_cuda(cudaGraphInstantiate(&a.graph, g, 0), "adjoint instantiate");
   if (g) cudaGraphDestroy(g);

@@ -277,8 +277,9 @@ __device__ __forceinline__ void loop_pass(const Dev& d, double* partials, LoopSh
 // Grid barrier on a counter that only grows during the launch.  Bounded: a
 // block that polls spin_limit times, or sees another's error flag, sets the
 // flag and returns false, and the kernel must return.
-__device__ __forceinline__ bool loop_barrier(unsigned int* bar, int* err, unsigned int target,
-                                             long long spin_limit, LoopShared& sh) {
+__device__ __forceinline__ bool loop_barrier(unsigned int* bar, int* err, int* timed_out,
+                                             unsigned int target, long long spin_limit,
+                                             LoopShared& sh) {
   __syncthreads();
   if (threadIdx.x == 0) {
     int ok = 1;
@@ -289,6 +290,7 @@ __device__ __forceinline__ bool loop_barrier(unsigned int* bar, int* err, unsign
       if ((int)(v - target) >= 0) break;
       if (++spins > spin_limit || ((spins & 255) == 0 && *(volatile int*)err)) {
         atomicExch(err, 1);
+        *timed_out = 1;
         ok = 0;
         break;
       }
@@ -353,7 +355,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
       return loop_w_tile<TH, F>(d, pin, pout, zsrc, x, y0, alpha, beta, first);
     });
     target += arrivals;
-    if (!loop_barrier(bar, err, target, spin_limit, sh)) return;
+    if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, sh)) return;
     const double pw = loop_total(pw_parts, d.ns, sh);
     if (threadIdx.x == 0) sh.alpha = rro / pw;
     __syncthreads();
@@ -364,7 +366,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
       return acc[0];
     });
     target += arrivals;
-    if (!loop_barrier(bar, err, target, spin_limit, sh)) return;
+    if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, sh)) return;
     const double rrn = loop_total(rz_parts, d.ns, sh);
     // the host steps of the iteration (cg_scalar_step): beta by thread 0, the
     // exit test beside it by thread 32
@@ -528,6 +530,19 @@ bool launch_loop_t(const LaunchCtx& l, Dev d, double* p2, Red red, ResState* st,
 }
 
 }  // namespace
+
+// The line between the two: a launch boundary costs a pass about 10 us (start,
+// drain, the last block's sum), a grid barrier with the sum in every block
+// about 3.5 us; but the cooperative kernel's passes share one register budget
+// (16 warps per SM), so pass B of long passes streams at 0.8 of the rate of its
+// own kernel.  us per iteration, cooperative / graph (three kernels per
+// iteration before them): 64^2 7.3 / 9.9 (11.7), 512^2 diagonal 15.3 / 21.6
+// (25.1), 960^2 33.0 / 38.9 (43.5), 1024^2 diagonal 34.7 / 39.7 (47.4),
+// 1501x1203 block 67.4 / 69.8 (71.8), 1700^2 diagonal 103 / 98, 2048^2
+// diagonal 134 / 121 (125), 4096^2 diagonal 419 / 391 (425), block 466 / 440
+// (463).  They cross between 12 and 20 supertiles per SM.
+constexpr int kLoopSupertilesPerSM = 14;
+bool cg_loop_fits(const Dev& d, int num_sms) { return d.ns <= kLoopSupertilesPerSM * num_sms; }
 
 void enqueue_cg_passes(const LaunchCtx& l, const Dev& d, double* p2, const Red& red,
                        ResState* st, unsigned int* counter, int iters, bool true_exit) {

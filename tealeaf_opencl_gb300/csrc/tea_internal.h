@@ -72,6 +72,7 @@ struct ResState {
   double rr_true;  // r.r of the last iteration (true-residual exit only)
   int n_first;     // iteration the loop began at
   int ended;       // u and p of the last iteration are in place
+  int timed_out;   // a grid barrier of the loop gave up
   double* alphas;  // indexed by iteration number n
   double* betas;
 };
@@ -240,16 +241,15 @@ void dev_dot(const LaunchCtx& l, const Dev& d, const Red& r, const double* a,
 void dev_block_init(const LaunchCtx& l, const Dev& d);
 void dev_update_halo(const LaunchCtx& l, const Dev& d, int mask, int depth);
 void dev_cg_init_p(const LaunchCtx& l, const Dev& d, const Red& r);
-// one iteration of the device-resident CG loop (loop scalars in *st; the
-// kernels return at once after it has stopped)
-void dev_cg_iteration(const LaunchCtx& l, const Dev& d, const Red& r, ResState* st,
-                      unsigned int* counter);
 // The whole CG loop from the state in *st, at most kLoopLaunchIters
 // iterations, as one cooperative launch (tea_cg_loop.cu).  p2: a second p
 // buffer (interior only); bar: two words, the barrier's counter and its error
-// flag; red.partials holds at least two arrays of red.stride.  After it
+// flag (also in st->timed_out); red.partials holds at least two arrays of red.stride.  After it
 // st->stop is set, or the loop goes on with another launch.
 constexpr int kLoopLaunchIters = 1024;
+constexpr long long kLoopSpins = 1LL << 26;  // polls of a barrier before it gives up
+// true where the one launch is the faster form (by size, tea_cg_loop.cu)
+bool cg_loop_fits(const Dev& d, int num_sms);
 bool launch_cg_loop(const LaunchCtx& l, const Dev& d, double* p2, const Red& red, ResState* st,
                     unsigned int* bar, long long spin_limit, unsigned int extra);
 // `iters` (even) iterations of the same loop as two kernels each, and the

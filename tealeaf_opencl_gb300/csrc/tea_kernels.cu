@@ -1348,12 +1348,6 @@ void dev_update_halo(const LaunchCtx& l, const Dev& d, int mask, int depth) {
 void dev_cg_init_p(const LaunchCtx& l, const Dev& d, const Red& r) {
   CTX_DISPATCH(l, d, "tea_leaf_cg_solve_init_p", k_cg_init_p, d, r);
 }
-void dev_cg_iteration(const LaunchCtx& l, const Dev& d, const Red& r, ResState* st,
-                      unsigned int* counter) {
-  CTX_DISPATCH(l, d, "tea_leaf_cg_solve_calc_w", k_cg_calc_w, d, r, st);
-  CTX_DISPATCH(l, d, "tea_leaf_cg_solve_calc_ur", k_cg_calc_ur, d, r, 0.0, st);
-  CTX_DISPATCH(l, d, "tea_leaf_cg_solve_calc_p", k_cg_calc_p, d, r, 0.0, st, counter);
-}
 void dev_finalise(const LaunchCtx& l, const Dev& d, const Red& r) {
   CTX_DISPATCH(l, d, "tea_leaf_finalise", k_finalise, d, r);
 }
@@ -1543,23 +1537,11 @@ void resident_release() {
 // batches of iterations, two kernels each, replayed from a captured graph with
 // one read of the loop state per batch.  Kernels queued after the loop has
 // stopped return at once.  The arithmetic and the exit test are those of the
-// per-call path, so the results are bit-identical to it.
-//
-// The line between the two: a launch boundary costs a pass about 10 us (start,
-// drain, the last block's sum), a grid barrier with the sum in every block
-// about 3.5 us; but the cooperative kernel's passes share one register budget
-// (16 warps per SM), so pass B of long passes streams at 0.8 of the rate of its
-// own kernel.  us per iteration, cooperative / graph (three kernels per
-// iteration before them): 64^2 7.3 / 9.9 (11.7), 512^2 diagonal 15.3 / 21.6
-// (25.1), 960^2 33.0 / 38.9 (43.5), 1024^2 diagonal 34.7 / 39.7 (47.4),
-// 1501x1203 block 67.4 / 69.8 (71.8), 1700^2 diagonal 103 / 98, 2048^2
-// diagonal 134 / 121 (125), 4096^2 diagonal 419 / 391 (425), block 466 / 440
-// (463).  They cross between 12 and 20 supertiles per SM.  The true-residual
+// per-call path, so the results are bit-identical to it.  The true-residual
 // exit (r.r beside r.z) and profiling use the kernels.
-constexpr int kLoopSupertilesPerSM = 14;
 static bool use_cg_loop(const Chunk& c, bool true_exit) {
   if (true_exit || c.profiler_on || c.resident_mode == 1) return false;
-  return c.resident_mode == 2 || c.dev().ns <= kLoopSupertilesPerSM * c.num_sms;
+  return c.resident_mode == 2 || cg_loop_fits(c.dev(), c.num_sms);
 }
 
 int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
@@ -1611,18 +1593,14 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
     const LaunchCtx l{c.stream, c.num_sms, c.arith};
     const long long launches = (long long)(loop_max - n_begin) / kLoopLaunchIters + 2;
     for (long long k = 0;; k++) {
-      int err = 0;
       if (!launch_cg_loop(l, c.dev(), c.p2.f, c.red(), c.res_state, c.res_bar,
                           c.barrier_spin_limit, (unsigned int)c.barrier_extra) ||
           !check_cuda(cudaMemcpyAsync(&h, c.res_state, sizeof(ResState),
                                       cudaMemcpyDeviceToHost, c.stream),
                       "resident state read") ||
-          !check_cuda(cudaMemcpyAsync(&err, c.res_bar + 1, sizeof(int),
-                                      cudaMemcpyDeviceToHost, c.stream),
-                      "barrier flag read") ||
           !check_cuda(cudaStreamSynchronize(c.stream), "resident CG loop"))
         return -1;
-      if (err) {
+      if (h.timed_out) {
         fail(25, "resident CG loop: a grid barrier timed out");
         return -1;
       }

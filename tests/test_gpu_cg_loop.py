@@ -24,7 +24,13 @@ def run(deck, mode, resident_mode=0):
         L.tea_gb300_set_resident_mode(0)
     last = steps[-1]
     return ([s.iterations for s in steps], (last.vol, last.mass, last.ie, last.temp),
-            [f.view(np.int64) for f in fields])
+            fields)
+
+
+def same_bits(a, b):
+    """Equal bit patterns, any NaN equal to any NaN (a 1x1 grid divides 0 by
+    0, on the host or on the GPU, which give NaNs of different signs)."""
+    return np.all((a.view(np.int64) == b.view(np.int64)) | (np.isnan(a) & np.isnan(b)))
 
 
 @pytest.mark.parametrize("x,y,halo,prec,form,iters,extra", [
@@ -45,6 +51,7 @@ def test_loop_matches_per_call(x, y, halo, prec, form, iters, extra):
     ref = run(deck, lib.DRIVER_PER_CALL)
     for resident_mode in (0, 1, 2):
         got = run(deck, lib.DRIVER_RESIDENT, resident_mode)
-        assert got[0] == ref[0] and got[1] == ref[1], resident_mode
+        assert got[0] == ref[0], resident_mode
+        assert np.array_equal(got[1], ref[1], equal_nan=True), resident_mode
         for name, a, b in zip(FIELDS + ("z",), got[2], ref[2]):
-            assert np.array_equal(a, b), (resident_mode, name)
+            assert same_bits(a, b), (resident_mode, name)
