@@ -153,7 +153,7 @@ __device__ __forceinline__ double st_load(const double* p) {
 // written by other blocks in an earlier phase are read through L2).
 
 // w = A p and p.w of every active problem (tea_leaf_cg_cl.cl:45-69); the
-// finishing block stores pw in the problem's loop state.
+// finishing block stores pw and alpha = rro/pw in the problem's loop state.
 template <int F, bool CG>
 __device__ __forceinline__ void phase_w(const Dev* __restrict__ devs,
                                         const Red* __restrict__ reds, ResState* st,
@@ -184,7 +184,10 @@ __device__ __forceinline__ void phase_w(const Dev* __restrict__ devs,
     if (unit_done(red.counter, units_of(d.ns, wl.G), is_last)) {
       block_final_sum<1>(red.partials, red.stride, d.ns, red.result, sh);
       if (threadIdx.x == 0) {
+        // alpha once per problem: a division in every thread of phase_ur
+        // costs each unit there about 10 FP64 instructions per warp
         st[i].pw = red.result[0];
+        st[i].alpha = st_load<CG>(&st[i].rro) / red.result[0];
         __threadfence();
       }
       __syncthreads();
@@ -192,7 +195,7 @@ __device__ __forceinline__ void phase_w(const Dev* __restrict__ devs,
   }
 }
 
-// u, r, z updates and r.z (tea_leaf_cg_cl.cl:73-137) with alpha = rro/pw;
+// u, r, z updates and r.z (tea_leaf_cg_cl.cl:73-137);
 // the finishing block takes the problem's scalar step and exit test.
 template <int F, bool CG>
 __device__ __forceinline__ void phase_ur(const Dev* __restrict__ devs,
@@ -205,7 +208,7 @@ __device__ __forceinline__ void phase_ur(const Dev* __restrict__ devs,
     if (*(volatile int*)&st[i].stop) continue;
     const Dev d = devs[i];
     const Red red = reds[i];
-    const double alpha = st_load<CG>(&st[i].rro) / st_load<CG>(&st[i].pw);
+    const double alpha = st_load<CG>(&st[i].alpha);
     const int s0 = (u - wl.ustart[j]) * wl.G, s1 = min(s0 + wl.G, d.ns);
     unit_partials(d, red, s0, s1, sh, [&](int x, int y0, bool xin, double* a) {
       if constexpr (CG) {

@@ -433,8 +433,9 @@ __global__ void __launch_bounds__(kBlock) k_cg_init_p(Dev d, Red red) {
 }
 
 // tea_leaf_cg_solve_calc_w, tea_leaf_cg_cl.cl:45-69.  With st != nullptr
-// (device-resident loop) it does nothing once the loop has stopped and
-// leaves pw in st.
+// (device-resident PPCG loop) it does nothing once the loop has stopped and
+// leaves pw and alpha = rro/pw in st (one division: made by every thread of
+// the kernel that uses alpha it cost that kernel about 2.5 us).
 template <int TH, int F>
 __global__ void __launch_bounds__(kBlock, 4)
     k_cg_calc_w(Dev d, Red red, ResState* st) {
@@ -442,34 +443,18 @@ __global__ void __launch_bounds__(kBlock, 4)
   const bool last = tile_driver<TH, 1>(d, red, [&](int x, int y0, bool xin, double* acc) {
     cg_w_tile_r<TH, F>(d, x, y0, xin, acc);
   });
-  if (st && last && threadIdx.x == 0) st->pw = red.result[0];
+  if (st && last && threadIdx.x == 0) {
+    st->pw = red.result[0];
+    st->alpha = st->rro / red.result[0];
+  }
 }
 
-// tea_leaf_cg_solve_calc_ur, tea_leaf_cg_cl.cl:73-137.  In the
-// device-resident loop alpha = rro/pw is formed here, and the block that
-// finishes the reduction carries out the host steps of one CG iteration
-// (cg_scalar_step).  With NV = 2 it also sums r.r, for the resident loop's
-// optional exit test on the unpreconditioned residual.
-// With r.r as well (NV = 2) the restrict-qualified body needs more registers
-// than 4 blocks per SM leave (202.5 against 188.7 us at 4096^2, diagonal
-// Jacobi), so that variant keeps cg_ur_tile at 3 blocks per SM.
-template <int TH, int F, int NV = 1>
-__global__ void __launch_bounds__(kBlock, NV == 2 ? 3 : 4)
-    k_cg_calc_ur(Dev d, Red red, double alpha, ResState* st) {
-  if (st) {
-    if (*(volatile int*)&st->stop) return;
-    alpha = st->rro / st->pw;
-  }
-  const bool last = tile_driver<TH, NV>(d, red, [&](int x, int y0, bool xin, double* acc) {
-    if constexpr (NV == 2)
-      cg_ur_tile<TH, F, NV>(d, x, y0, xin, acc, alpha);
-    else
-      cg_ur_tile_r<TH, F, NV>(d, x, y0, xin, acc, alpha);
+// tea_leaf_cg_solve_calc_ur, tea_leaf_cg_cl.cl:73-137
+template <int TH, int F>
+__global__ void __launch_bounds__(kBlock, 4) k_cg_calc_ur(Dev d, Red red, double alpha) {
+  tile_driver<TH, 1>(d, red, [&](int x, int y0, bool xin, double* acc) {
+    cg_ur_tile_r<TH, F, 1>(d, x, y0, xin, acc, alpha);
   });
-  if (st && last && threadIdx.x == 0) {
-    cg_scalar_step<NV>(st, alpha, red.result);
-    __threadfence();
-  }
 }
 
 // tea_leaf_cg_solve_calc_ur with its r.z, and PPCG's init_sd
@@ -1153,8 +1138,7 @@ void launch_cg_calc_w(Chunk& c) {
 }
 
 void launch_cg_calc_ur(Chunk& c, double alpha) {
-  TH_DISPATCH(c, "tea_leaf_cg_solve_calc_ur", k_cg_calc_ur, c.dev(), c.red(),
-              alpha, (ResState*)nullptr);
+  TH_DISPATCH(c, "tea_leaf_cg_solve_calc_ur", k_cg_calc_ur, c.dev(), c.red(), alpha);
 }
 
 void launch_cg_calc_ur_sd(Chunk& c, double alpha, double theta, double* sd_out) {
@@ -1370,18 +1354,17 @@ static int tile_grid(Chunk& c, void (*kernel)(KArgs...), int ns = 0) {
 // ---- device-resident PPCG iterations (tea_solve.f90:231-268 after the
 // switch from CG), scalars in the ResState as for CG ----
 
-// tea_leaf_cg_calc_ur of a PPCG iteration with alpha = rro/pw from the loop
-// state, fused with tea_leaf_ppcg_init_sd: PPCG discards this r.z, so no
+// tea_leaf_cg_calc_ur of a PPCG iteration with alpha from the loop state,
+// fused with tea_leaf_ppcg_init_sd: PPCG discards this r.z, so no
 // sum is taken, and sd = M^-1 r / theta comes from the z formed here.
 template <int TH, int F>
 __global__ void __launch_bounds__(kBlock, 4)
     k_ppcg_ur_sd(Dev d, Red red, ResState* st, DivConst theta) {
   if (*(volatile int*)&st->stop) return;
-  const double alpha = st->rro / st->pw;
+  const double alpha = st->alpha;
   tile_driver<TH, 0>(d, red, [&](int x, int y0, bool xin, double* acc) {
     cg_ur_tile_r<TH, F, 0, true>(d, x, y0, xin, acc, alpha, theta);
   });
-  if (blockIdx.x == 0 && threadIdx.x == 0) st->alpha = alpha;
 }
 
 // tea_leaf_ppcg_calc_zrnorm (r.z with the z of the last calc_ur) with the

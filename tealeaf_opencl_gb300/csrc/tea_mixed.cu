@@ -108,8 +108,18 @@ __device__ __forceinline__ void acc_pair(float& hi, float& lo, float a,
   hi = s;
 }
 
+// (double)f from the bit pattern: conversions run on the FP64 pipe, whose
+// warp instruction costs an SM 19 cycles.  Subnormals, infinities and NaNs
+// take the hardware's conversion.
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t b = __float_as_uint(f), mag = b & 0x7fffffffu;
+  if (mag != 0 && (mag < 0x00800000u || mag >= 0x7f800000u)) return (double)f;
+  const uint32_t hi = (b & 0x80000000u) | (mag != 0 ? (mag >> 3) + 0x38000000u : 0u);
+  return __hiloint2double((int)hi, (int)(b << 29));
+}
+
 __device__ __forceinline__ double pair_value(float hi, float lo) {
-  return (double)hi + (double)lo;
+  return widen(hi) + widen(lo);
 }
 
 // FP32 copies of the operator over the whole padded array:
@@ -196,7 +206,10 @@ __global__ void __launch_bounds__(kBlock, kMixMinBlocks)
     }
     acc[0] = pair_value(hi, lo);
   });
-  if (last && threadIdx.x == 0) st->pw = red.result[0];
+  if (last && threadIdx.x == 0) {
+    st->pw = red.result[0];
+    st->alpha = st->rro / red.result[0];
+  }
 }
 
 // ---- FP32 iteration kernels with 16-byte accesses ----
@@ -242,12 +255,16 @@ __device__ __forceinline__ bool quad_driver(const Dev& d, const Red& red, Body b
       const int tx = sx * kTilesPerSuper + tile;
       if (tx < d.ntx) body(tx * kTileW + 4 * q, sy * TH, v);
     }
-#pragma unroll
-    for (int off = 4; off >= 1; off >>= 1) {
-#pragma unroll
-      for (int k = 0; k < 4; k++) v[k] = v[k] + __shfl_xor_sync(0xffffffffu, v[k], off);
-    }
-    const double t = (v[0] + v[2]) + (v[1] + v[3]);
+    // Each stage adds the pairs of the butterfly, but a lane carries on with
+    // half of its columns after the first two: 6 FP64 instructions in place
+    // of 15 (the last two stages add columns within a quad, k with k^2, k^1).
+    const bool h4 = q & 4, h2 = q & 2;
+    const double a0 = (h4 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, h4 ? v[0] : v[2], 4);
+    const double a1 = (h4 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, h4 ? v[1] : v[3], 4);
+    double t = (h2 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, h2 ? a0 : a1, 2);
+    t = t + __shfl_xor_sync(0xffffffffu, t, 1);
+    t = t + __shfl_xor_sync(0xffffffffu, t, 4);
+    t = t + __shfl_xor_sync(0xffffffffu, t, 2);
     if (q == 0) sh[grp * 8 + tile] = t;
     int s_k[4];
 #pragma unroll
@@ -304,7 +321,10 @@ __global__ void __launch_bounds__(kBlock, 4)
 #pragma unroll
     for (int k = 0; k < 4; k++) v[k] = pair_value(hi[k], lo[k]);
   });
-  if (last && threadIdx.x == 0) st->pw = red.result[0];
+  if (last && threadIdx.x == 0) {
+    st->pw = red.result[0];
+    st->alpha = st->rro / red.result[0];
+  }
 }
 
 // calc_p folded into calc_w (CG inner loop of the mixed solve): with the
@@ -408,6 +428,7 @@ __global__ void __launch_bounds__(kBlock, 4)
   });
   if (last && threadIdx.x == 0) {
     st->pw = red.result[0];
+    st->alpha = st->rro / red.result[0];
     st->p_pending = 0;
     __threadfence();
   }
@@ -419,7 +440,7 @@ template <int TH>
 __global__ void __launch_bounds__(kBlock, 4)
     k_mix_calc_ur4(Dev d, MixDev m, Red red, MixState* st) {
   if (*(volatile int*)&st->stop) return;
-  const double alpha = st->rro / st->pw;
+  const double alpha = st->alpha;
   const float af = (float)alpha;
   const bool last = quad_driver<TH>(d, red, [&](int x, int y0, double* v) {
     float hi[4] = {0.0f, 0.0f, 0.0f, 0.0f}, lo[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -463,7 +484,6 @@ __global__ void __launch_bounds__(kBlock, 4)
   });
   if (last && threadIdx.x == 0) {
     const double rrn = red.result[0];
-    st->alpha = alpha;
     st->beta = rrn / st->rro;
     if (st->alphas) {
       st->alphas[st->n] = alpha;
@@ -539,7 +559,7 @@ template <int TH>
 __global__ void __launch_bounds__(kBlock, kMixMinBlocks)
     k_mix_ppcg_ur(Dev d, MixDev m, Red red, MixState* st) {
   if (*(volatile int*)&st->stop) return;
-  const double alpha = st->rro / st->pw;
+  const double alpha = st->alpha;
   const float af = (float)alpha;
   tile_driver<TH, 0>(d, red, [&](int x, int y0, bool xin, double* acc) {
     if (!xin) return;
