@@ -12,8 +12,10 @@
 #include <algorithm>
 #include <fstream>
 #include <map>
+#include <mutex>
 #include <sstream>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/tealeaf_gb300.h"
@@ -509,6 +511,98 @@ static Field* field_by_id(Chunk& c, int id) {
   }
 }
 
+// Pinned staging for reads into pageable memory: two buffers of kStage bytes,
+// made by the first such read and given back by tea_gb300_finalise.
+constexpr size_t kStage = 8u << 20;
+static std::mutex g_stage_mutex;
+static char* g_stage = nullptr;
+static cudaEvent_t g_stage_ev[2] = {nullptr, nullptr};
+
+static void release_stage() {
+  std::lock_guard<std::mutex> lock(g_stage_mutex);
+  cudaFreeHost(g_stage);
+  g_stage = nullptr;
+  for (cudaEvent_t& e : g_stage_ev) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
+  }
+}
+
+static bool ensure_stage() {
+  if (g_stage) return true;
+  if (cudaMallocHost(&g_stage, 2 * kStage) != cudaSuccess) {
+    cudaGetLastError();
+    g_stage = nullptr;
+    return false;
+  }
+  for (cudaEvent_t& e : g_stage_ev)
+    if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      e = nullptr;
+      return false;
+    }
+  return true;
+}
+
+// memcpy on up to four threads: one faults fresh pages in at 11 GB/s
+static void copy_threaded(char* dst, const char* src, size_t bytes) {
+  const size_t parts = bytes >= (4u << 20) ? 4 : 1, part = (bytes / parts + 4095) & ~(size_t)4095;
+  std::thread t[4];
+  for (size_t k = 1; k < parts; k++) {
+    const size_t at = std::min(k * part, bytes), end = std::min(at + part, bytes);
+    try {
+      t[k] = std::thread([=] { memcpy(dst + at, src + at, end - at); });
+    } catch (...) {  // no thread to be had
+      memcpy(dst + at, src + at, end - at);
+    }
+  }
+  memcpy(dst, src, std::min(part, bytes));
+  for (std::thread& th : t)
+    if (th.joinable()) th.join();
+}
+
+// A w x h block of a field into a dense host array.  A strided device-to-host
+// copy into pageable memory faults fresh pages in from the copy engine's side:
+// 131 ms for the 134 MB of a 4096^2 field (6.7 ms for the 7.4 MB of 960^2).
+// So larger blocks for pageable memory go through the pinned buffers, one half
+// filling while the host empties the other.  Below 1 MB, and into pinned
+// memory, the strided copy is as fast.  Waits for the copy.
+static bool block_to_host(Chunk& c, double* host, const double* dev, int w, int h) {
+  const size_t row = (size_t)w * sizeof(double), bytes = row * (size_t)h;
+  const size_t pitch = (size_t)c.S * sizeof(double);
+  cudaPointerAttributes at;
+  const bool known = cudaPointerGetAttributes(&at, host) == cudaSuccess;
+  if (!known) cudaGetLastError();
+  const bool pageable = !known || at.type == cudaMemoryTypeUnregistered;
+  if (bytes >= (1u << 20) && row <= kStage && pageable) {
+    std::lock_guard<std::mutex> lock(g_stage_mutex);
+    if (ensure_stage()) {
+      const int per = (int)(kStage / row), chunks = (h + per - 1) / per;
+      for (int k = 0; k <= chunks; k++) {
+        if (k < chunks) {
+          const int r0 = k * per, n = std::min(per, h - r0);
+          if (!check_cuda(cudaMemcpy2DAsync(g_stage + (k & 1) * kStage, row,
+                                            dev + (long long)r0 * c.S, pitch, row, n,
+                                            cudaMemcpyDeviceToHost, c.stream),
+                          "field copy") ||
+              !check_cuda(cudaEventRecord(g_stage_ev[k & 1], c.stream), "field copy"))
+            return false;
+        }
+        if (k > 0) {
+          const int r0 = (k - 1) * per, n = std::min(per, h - r0);
+          if (!check_cuda(cudaEventSynchronize(g_stage_ev[(k - 1) & 1]), "field copy"))
+            return false;
+          copy_threaded((char*)host + r0 * row, g_stage + ((k - 1) & 1) * kStage, n * row);
+        }
+      }
+      return true;
+    }
+  }
+  return check_cuda(cudaMemcpy2DAsync(host, row, dev, pitch, row, h, cudaMemcpyDeviceToHost,
+                                      c.stream),
+                    "field copy");
+}
+
 static bool store_coefs(const double* a, const double* b, int n, double** ah,
                         double** bh) {
   free(*ah);
@@ -964,7 +1058,10 @@ extern "C" int tea_gb300_last_error(char* msg, int len) {
   return code;
 }
 
-extern "C" void tea_gb300_finalise(void) { free_chunk(chunk()); }
+extern "C" void tea_gb300_finalise(void) {
+  free_chunk(chunk());
+  release_stage();
+}
 
 static int copy_field(int id, double* host, const double* in, bool padded) {
   if (!need_chunk("field access")) return -1;
@@ -978,16 +1075,14 @@ static int copy_field(int id, double* host, const double* in, bool padded) {
   const int w = padded ? c.x_max + 2 * c.H : c.x_max;
   const int h = padded ? c.y_max + 2 * c.H : c.y_max;
   double* dev = f->f + (long long)off * c.S + off;
-  cudaError_t e;
-  if (in)
-    e = cudaMemcpy2DAsync(dev, c.S * sizeof(double), in, w * sizeof(double),
-                          w * sizeof(double), h, cudaMemcpyHostToDevice,
-                          c.stream);
-  else
-    e = cudaMemcpy2DAsync(host, w * sizeof(double), dev, c.S * sizeof(double),
-                          w * sizeof(double), h, cudaMemcpyDeviceToHost,
-                          c.stream);
-  if (!check_cuda(e, "field copy")) return -1;
+  if (in) {
+    if (!check_cuda(cudaMemcpy2DAsync(dev, c.S * sizeof(double), in, w * sizeof(double),
+                                      w * sizeof(double), h, cudaMemcpyHostToDevice, c.stream),
+                    "field copy"))
+      return -1;
+  } else if (!block_to_host(c, host, dev, w, h)) {
+    return -1;
+  }
   // the second r/sd buffer keeps the same halo (the fused PPCG inner steps
   // read halos from whichever buffer is live)
   Field* alt = f == &c.r ? &c.r2 : f == &c.sd ? &c.sd2 : nullptr;
