@@ -320,7 +320,8 @@ __device__ __forceinline__ void cg_scalar_step(ResState* st, double alpha,
   if (done) {
     st->converged = 1;
     st->stop = 1;
-  } else if (n >= st->loop_max) {
+  } else if (n >= st->loop_max ||
+             (st->switch_n > 0 && n + 1 >= st->switch_n && fabs(err) <= st->switch_eps)) {
     st->stop = 1;
   } else {
     st->n = n + 1;

@@ -27,7 +27,7 @@ constexpr int kLoopSlots = kLoopWarps / kTilesPerSuper;  // supertiles in flight
 constexpr int kLoopBatch = 4;                   // rounds whose tile sums share a sweep
 
 // why the loop left
-enum { kStopConverged = 1, kStopLoopMax, kStopLaunch, kStopPw, kStopRz };
+enum { kStopConverged = 1, kStopLoopMax, kStopSwitch, kStopLaunch, kStopPw, kStopRz };
 
 struct LoopShared {
   double lanes[kLoopBatch * kLoopThreads];  // lane sums of a batch of rounds
@@ -342,7 +342,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
   double rro = st->rro;  // kept up to date by thread 0
   int n = st->n;
   const int loop_max = st->loop_max, check = st->check;
-  const double eps_target = st->eps_target;
+  const double eps_target = st->eps_target, switch_eps = st->switch_eps;
+  const int switch_n = st->switch_n;
   const double rr_limit = threadIdx.x == 32 ? square_limit(eps_target) : 0.0;
   double alpha = 0.0, beta = 0.0;
   int it = 0, stop = 0;
@@ -383,8 +384,10 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
     }
     if (threadIdx.x == 32) {
       const bool done = rr_limit > 0.0 ? rrn < rr_limit && rrn >= 0.0 : sqrt(rrn) < eps_target;
+      const bool sw = switch_n > 0 && n + 1 >= switch_n && sqrt(rrn) <= switch_eps;
       int s = done              ? kStopConverged
               : n >= loop_max   ? kStopLoopMax
+              : sw              ? kStopSwitch
               : it + 1 >= iters ? kStopLaunch
                                 : 0;
       if (check) {

@@ -723,16 +723,20 @@ class Driver {
         }
         cheby_calc_steps++;
       } else if (use_cg || use_cheby || use_ppcg) {
-        if (mode == TEA_DRIVER_RESIDENT && use_cg) {
-          // The whole remaining CG loop runs on the device; it stops exactly
-          // where this loop would (same tests, same arithmetic).
+        if (mode == TEA_DRIVER_RESIDENT && (use_cg || !D.verbose)) {
+          // The whole remaining CG loop, or the CG iterations before the
+          // switch to Chebyshev or PPCG, on the device; it stops exactly
+          // where this loop would (same tests, same arithmetic).  PPCG
+          // switches after one iteration once the eigenvalues are known.
           int n_done = 0, conv = 0;
           tea::chunk().solver_checks = checks & TEA_CHECK_BREAKDOWN;
-          if (tea::resident_cg_iterations(n, loop_max, rro,
-                                          D.eps * initial_residual, &rro,
-                                          &error, &n_done, &conv,
-                                          cg_alphas.data(), cg_betas.data(),
-                                          D.true_exit) != 0 ||
+          const bool one = use_ppcg && !first;
+          if (tea::resident_cg_iterations(n, one ? std::min(loop_max, std::max(n, 1)) : loop_max,
+                                          rro, D.eps * initial_residual, &rro, &error, &n_done,
+                                          &conv, cg_alphas.data(), cg_betas.data(),
+                                          use_cg && D.true_exit,
+                                          use_cg || one ? 0 : std::max(D.presteps, 1),
+                                          D.epslim) != 0 ||
               !resident_breakdown_ok())
             return -1;
           n = n_done;
@@ -740,6 +744,7 @@ class Driver {
             exited = true;
             break;
           }
+          old_error = error;
           n++;
           continue;
         }

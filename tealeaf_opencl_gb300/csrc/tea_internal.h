@@ -71,6 +71,8 @@ struct ResState {
   int breakdown_n; // the iteration it happened in
   double rr_true;  // r.r of the last iteration (true-residual exit only)
   int n_first;     // iteration the loop began at
+  int switch_n;    // > 0: also stop once error <= switch_eps and the next
+  double switch_eps;  // iteration is at least switch_n (the switch from CG)
   int ended;       // u and p of the last iteration are in place
   int timed_out;   // a grid barrier of the loop gave up
   double* alphas;  // indexed by iteration number n
@@ -260,12 +262,14 @@ void enqueue_cg_passes(const LaunchCtx& l, const Dev& d, double* p2, const Red& 
 void dev_finalise(const LaunchCtx& l, const Dev& d, const Red& r);
 void dev_field_summary(const LaunchCtx& l, const Dev& d, const Red& r);
 // device-resident CG loop (tea_kernels.cu)
-// true_exit: stop on ||r||_2 < eps_target instead of sqrt(r.z)
+// true_exit: stop on ||r||_2 < eps_target instead of sqrt(r.z); switch_n > 0:
+// also stop where the driver would switch to Chebyshev or PPCG
 int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
                            double eps_target, double* rro_out,
                            double* error_out, int* n_done, int* converged,
                            double* cg_alphas, double* cg_betas,
-                           bool true_exit = false);
+                           bool true_exit = false, int switch_n = 0,
+                           double switch_eps = 0.0);
 // device-resident PPCG iterations n_begin..loop_max with the coefficients
 // of the last tea_leaf_ppcg_init_ocl_ (tea_solve.f90:231-268); the fused
 // calc_ur + init_sd kernel replaces the per-call pair

@@ -1530,7 +1530,8 @@ static bool use_cg_loop(const Chunk& c, bool true_exit) {
 int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
                            double eps_target, double* rro_out,
                            double* error_out, int* n_done, int* converged,
-                           double* cg_alphas, double* cg_betas, bool true_exit) {
+                           double* cg_alphas, double* cg_betas, bool true_exit, int switch_n,
+                           double switch_eps) {
   Chunk& c = chunk();
   flush_pending_inner(c);
   if (c.res_graph &&
@@ -1564,6 +1565,8 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
   h.eps_target = eps_target;
   h.n = h.n_first = n_begin;
   h.loop_max = loop_max;
+  h.switch_n = switch_n;
+  h.switch_eps = switch_eps;
   h.check = c.solver_checks;
   h.alphas = c.res_coef;
   h.betas = c.res_coef + c.res_coef_n;
