@@ -831,17 +831,12 @@ extern "C" void tea_leaf_cheby_iterate_kernel_ocl_(const int* cheby_calc_step) {
          *cheby_calc_step, c.n_cheby);
     return;
   }
-  if (c.prec == PREC_JAC_BLOCK) {
-    // calc_u folded into calc_p: the new u goes to the second buffer,
-    // which then becomes u
-    if (!ensure_u_alt(c)) return;
-    launch_cheby_calc_pu(c, c.cheby_alpha_h[s], c.cheby_beta_h[s], c.u2.f);
-    std::swap(c.u, c.u2);
-    c.field_epoch++;
-    return;
-  }
-  launch_cheby_calc_p(c, c.cheby_alpha_h[s], c.cheby_beta_h[s]);
-  launch_cheby_calc_u(c);
+  // calc_u folded into calc_p: the new u goes to the second buffer, which
+  // then becomes u
+  if (!ensure_u_alt(c)) return;
+  launch_cheby_calc_pu(c, c.cheby_alpha_h[s], c.cheby_beta_h[s], c.u2.f);
+  std::swap(c.u, c.u2);
+  c.field_epoch++;
 }
 
 extern "C" void tea_leaf_ppcg_init_ocl_(const double* ch_alphas,
@@ -914,17 +909,12 @@ extern "C" void tea_leaf_ppcg_inner_kernel_ocl_(int* inner_step,
     }
   }
   flush_pending_inner(c);
-  if (c.prec == PREC_JAC_BLOCK) {
-    // update_r and calc_sd in one pass (k_ppcg_step): the new sd goes to
-    // the second buffer, which then becomes sd
-    if (!ensure_alt_fields(c)) return;
-    launch_ppcg_step(c, c.ppcg_alpha_h[s], c.ppcg_beta_h[s], c.sd.f, c.sd2.f);
-    std::swap(c.sd, c.sd2);
-    c.field_epoch++;
-    return;
-  }
-  launch_ppcg_update_r(c);
-  launch_ppcg_calc_sd(c, c.ppcg_alpha_h[s], c.ppcg_beta_h[s]);
+  // update_r and calc_sd in one pass: the new sd goes to the second buffer,
+  // which then becomes sd
+  if (!ensure_alt_fields(c)) return;
+  launch_ppcg_step(c, c.ppcg_alpha_h[s], c.ppcg_beta_h[s], c.sd.f, c.sd2.f);
+  std::swap(c.sd, c.sd2);
+  c.field_epoch++;
 }
 
 extern "C" void tea_leaf_jacobi_solve_kernel_ocl_(double* error) {

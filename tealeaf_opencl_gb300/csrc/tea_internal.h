@@ -136,7 +136,7 @@ struct Chunk {
   // allocated on first use, with the halos of the live pair
   Field r2, sd2;
   // second u buffer of the Chebyshev iteration with calc_u folded into
-  // calc_p (block Jacobi), which writes the new u, halo included, to the
+  // calc_p, which writes the new u, halo included, to the
   // buffer it does not read; the two then trade places
   Field u2;
   Field p2;  // second p buffer of the resident CG loop (tea_cg_loop.cu)
@@ -205,15 +205,12 @@ void launch_cg_calc_ur(Chunk& c, double alpha);
 void launch_cg_calc_ur_sd(Chunk& c, double alpha, double theta, double* sd_out);
 void launch_cg_calc_p(Chunk& c, double beta);
 void launch_cheby_init_p(Chunk& c, double theta);
-void launch_cheby_calc_p(Chunk& c, double alpha, double beta);
 void launch_cheby_calc_u(Chunk& c);
-// calc_p and calc_u of one Chebyshev iteration in one pass (block Jacobi),
-// the new u into un
+// calc_p and calc_u of one Chebyshev iteration in one pass, the new u into un
 void launch_cheby_calc_pu(Chunk& c, double alpha, double beta, double* un);
 void launch_ppcg_init_sd(Chunk& c, double theta);
 void launch_ppcg_update_r(Chunk& c);
-// update_r and calc_sd of one inner step in one pass (block Jacobi), sd
-// read from sdi and the new sd written to sdo
+// update_r and calc_sd of one inner step in one pass, sd read from sdi and the new sd written to sdo
 void launch_ppcg_step(Chunk& c, double alpha, double beta, const double* sdi, double* sdo);
 void launch_ppcg_calc_sd(Chunk& c, double alpha, double beta);
 void launch_jacobi_copy_u(Chunk& c);

@@ -501,8 +501,8 @@ __device__ __forceinline__ double cheby_update(double a, double p, double bl,
 // One Chebyshev iteration with the block-Jacobi preconditioner alone, in
 // one pass: tea_leaf_cheby_solve_calc_p (tea_leaf_cheby_cl.cl:78-145) and
 // then tea_leaf_cheby_solve_calc_u (u = u + p, :66-76) on the p it has just
-// formed.  Only this path compiled in (k_cheby_p's mode-1 block path alone
-// took 72 registers against 80, 340 -> 326 us at 4096^2).  The product
+// formed.  Only this path compiled in (on its own it took 72 registers against
+// 80, 340 -> 326 us at 4096^2).  The product
 // beta z runs on the integer pipes (tea_emu.cuh, bit-identical): on non-zero
 // fields 340.2 -> 315.6 us; the operator's first product there as well was
 // slower (367.0 us), and so were the sweep's multiplies by bfp (388 us),
@@ -512,7 +512,7 @@ __device__ __forceinline__ double cheby_update(double a, double p, double bl,
 // ring to un, so un is exactly the in-place result.  One FP64 add per cell
 // more in this FP64-bound kernel against a separate pass over u and p:
 // 373.6 -> 350.6 us per iteration at 4096^2 (non-zero fields).
-template <int TH, int F, bool U>
+template <int TH, int F>
 __device__ __forceinline__ void cheby_block_body(const Dev& d, const Red& red, double alpha,
                                                  double beta, double* un) {
   tile_driver<TH, 0>(d, red, [&](int x, int y0, bool xin, double* acc) {
@@ -526,7 +526,7 @@ __device__ __forceinline__ void cheby_block_body(const Dev& d, const Red& red, d
         if (ys + i < d.y_max) {
           const long long c = c0 + i * d.S;
           wl[i] = smvp<F, false, false>(d, d.u, c);
-          if (U) ul[i] = d.u[c];
+          ul[i] = d.u[c];
           rl[i] = d.u0[c] - wl[i];
           pl[i] = d.p[c];
         }
@@ -545,7 +545,7 @@ __device__ __forceinline__ void cheby_block_body(const Dev& d, const Red& red, d
           const double pn = F ? __fma_rn(alpha, pl[i], emu_dmul(beta, zl[i]))
                               : alpha * pl[i] + emu_dmul(beta, zl[i]);
           d.p[c0 + i * d.S] = pn;
-          if (U) un[c0 + i * d.S] = ul[i] + pn;
+          un[c0 + i * d.S] = ul[i] + pn;
         }
     }
   });
@@ -554,89 +554,88 @@ __device__ __forceinline__ void cheby_block_body(const Dev& d, const Red& red, d
 template <int TH, int F>
 __global__ void __launch_bounds__(kBlock, 3)
     k_cheby_calc_pu_block(Dev d, Red red, double alpha, double beta, double* un) {
-  cheby_block_body<TH, F, true>(d, red, alpha, beta, un);
+  cheby_block_body<TH, F>(d, red, alpha, beta, un);
   copy_halo_ring(d, d.u, un);
 }
 
-// The Chebyshev residual step shared by tea_leaf_cheby_solve_init_p and
-// tea_leaf_cheby_solve_calc_p (tea_leaf_cheby_cl.cl:4-64, :78-145):
-// w = A u, r = u0 - w, then p from M^-1 r.  mode 0: p = M^-1 r / theta;
-// mode 1: p = alpha p + beta M^-1 r.
+// The same iteration without a preconditioner or with the diagonal one:
+// p = alpha p + beta r or alpha p + (beta Mi) r, u + p to the second u buffer.
+// One pass in place of calc_p and calc_u; 7 FP64 instructions per cell with the
+// products on the integer pipes (bit-identical), 10 with all of them on the
+// FP64 pipe.
+template <int F>
+__global__ void __launch_bounds__(kBlock, 3)
+    k_cheby_calc_pu_point(Dev d, Red red, double alpha, double beta, double* un_) {
+  tile_driver<4, 0>(d, red, [&](int x, int y0, bool xin, double* acc) {
+    if (!xin) return;
+    const double* __restrict__ u = d.u;
+    double* __restrict__ un = un_;
+    double* __restrict__ p = d.p;
+    double* __restrict__ r = d.r;
+    double* __restrict__ w = d.w;
+    const bool dia = d.prec == PREC_JAC_DIAG;
+    const long long S = d.S;
+    const long long c0 = cidx(d, x, y0);
+    const int rows = min(4, d.y_max - y0);
+    double uv[6], kyv[5], wl[4], rl[4], pl[4], mv[4];
+#pragma unroll
+    for (int i = 0; i < 6; i++) uv[i] = u[c0 + min(i - 1, rows) * S];
+#pragma unroll
+    for (int i = 0; i < 5; i++) kyv[i] = __ldg(d.Ky + c0 + min(i, rows) * S);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const long long c = c0 + min(j, rows - 1) * S;
+      wl[j] = smvp_v<F>(__ldg(d.diag + c), kyv[j + 1], kyv[j], __ldg(d.Kx + c + 1),
+                        __ldg(d.Kx + c), uv[j + 1], uv[j + 2], uv[j], u[c + 1], u[c - 1]);
+      rl[j] = __ldg(d.u0 + c) - wl[j];
+      pl[j] = p[c];
+      mv[j] = dia ? __ldg(d.Mi + c) : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (j < rows) {
+        const long long c = c0 + j * S;
+        const double b = emu_dmul(dia ? emu_dmul(beta, mv[j]) : beta, rl[j]);
+        const double pn = F ? __fma_rn(alpha, pl[j], b) : alpha * pl[j] + b;
+        w[c] = wl[j];
+        r[c] = rl[j];
+        p[c] = pn;
+        un[c] = uv[j + 1] + pn;
+      }
+  });
+  copy_halo_ring(d, d.u, un_);
+}
+
+// tea_leaf_cheby_solve_init_p (tea_leaf_cheby_cl.cl:4-64): w = A u,
+// r = u0 - w, p = M^-1 r / theta
 template <int TH, int F>
-__global__ void __launch_bounds__(kBlock)
-    k_cheby_p(Dev d, Red red, int mode, DivConst theta, double alpha,
-              double beta) {
+__global__ void __launch_bounds__(kBlock) k_cheby_init_p(Dev d, Red red, DivConst theta) {
   tile_driver<TH, 0>(d, red, [&](int x, int y0, bool xin, double* acc) {
     if (!xin) return;
-    if (d.prec == PREC_JAC_BLOCK) {
 #pragma unroll 1
-      for (int ys = y0; ys < y0 + TH && ys < d.y_max; ys += 4) {
-        double zl[4], rl[4] = {0.0, 0.0, 0.0, 0.0}, wl[4], pl[4];
-        const long long c0 = cidx(d, x, ys);
+    for (int g = y0; g < y0 + TH && g < d.y_max; g += 4) {
+      double zl[4], rl[4] = {0.0, 0.0, 0.0, 0.0}, wl[4];
+      const long long c0 = cidx(d, x, g);
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-          if (ys + i < d.y_max) {
-            const long long c = c0 + i * d.S;
-            wl[i] = smvp<F, false, false>(d, d.u, c);
-            rl[i] = d.u0[c] - wl[i];
-            if (mode != 0) pl[i] = d.p[c];
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          if (ys + i < d.y_max) {
-            d.w[c0 + i * d.S] = wl[i];
-            d.r[c0 + i * d.S] = rl[i];
-          }
-        }
-        strip_solve<F>(d, c0, strip_rows(d, ys), rl, zl);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          if (ys + i < d.y_max) {
-            const long long c = c0 + i * d.S;
-            if (mode == 0)
-              d.p[c] = emu_ddiv(zl[i], theta);
-            else
-              d.p[c] = cheby_update<F>(alpha, pl[i], beta, zl[i]);
-          }
+      for (int i = 0; i < 4; i++) {
+        if (g + i < d.y_max) {
+          const long long c = c0 + i * d.S;
+          wl[i] = smvp<F, false, false>(d, d.u, c);
+          rl[i] = d.u0[c] - wl[i];
+          zl[i] = d.prec == PREC_JAC_DIAG ? d.Mi[c] * rl[i] : rl[i];
         }
       }
-    } else {
-#pragma unroll 1
-      for (int g = y0; g < y0 + TH; g += 4) {
-        const long long c0 = cidx(d, x, g);
-        double wl[4], rl[4], pl[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          if (g + j < d.y_max) {
-            const long long c = c0 + j * d.S;
-            const double wv = smvp<F, false, false>(d, d.u, c);
-            const double rv = d.u0[c] - wv;
-            wl[j] = wv;
-            rl[j] = rv;
-            if (mode == 0) {
-              if (d.prec == PREC_JAC_DIAG)
-                pl[j] = emu_ddiv(d.Mi[c] * rv, theta);
-              else
-                pl[j] = emu_ddiv(rv, theta);
-            } else {
-              if (d.prec == PREC_JAC_DIAG)
-                pl[j] = cheby_update<F>(alpha, d.p[c], beta * d.Mi[c], rv);
-              else
-                pl[j] = cheby_update<F>(alpha, d.p[c], beta, rv);
-            }
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          if (g + j < d.y_max) {
-            const long long c = c0 + j * d.S;
-            d.w[c] = wl[j];
-            d.r[c] = rl[j];
-            d.p[c] = pl[j];
-          }
+      for (int i = 0; i < 4; i++) {
+        if (g + i < d.y_max) {
+          d.w[c0 + i * d.S] = wl[i];
+          d.r[c0 + i * d.S] = rl[i];
         }
       }
+      if (d.prec == PREC_JAC_BLOCK) strip_solve<F>(d, c0, strip_rows(d, g), rl, zl);
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (g + i < d.y_max) d.p[c0 + i * d.S] = emu_ddiv(zl[i], theta);
     }
   });
 }
@@ -909,6 +908,54 @@ __global__ void __launch_bounds__(kBlock, 3)
   });
 }
 
+// The same inner step without a preconditioner or with the diagonal one
+// (tea_leaf_ppcg_cl.cl:62-155): u += sd, r -= A sd, sd' = alpha sd + beta r or
+// alpha sd + (beta r) Mi, the new sd to the second buffer.  One pass of 80 (88)
+// algorithmic bytes and 7 FP64 instructions per cell in place of update_r and
+// calc_sd; the products run on the integer pipes (bit-identical).  Rows past
+// the interior are clamped to the halo row, so every load is issued before the
+// first use; the values of such rows are not stored.
+template <int F>
+__global__ void __launch_bounds__(kBlock, 3)
+    k_ppcg_step_point(Dev d, Red red, double alpha, double beta, const ResState* st,
+                      const double* sdi_, double* sdo_) {
+  if (st && *(volatile const int*)&st->stop) return;
+  tile_driver<4, 0>(d, red, [&](int x, int y0, bool xin, double* acc) {
+    if (!xin) return;
+    const double* __restrict__ sdi = sdi_;
+    double* __restrict__ sdo = sdo_;
+    double* __restrict__ u = d.u;
+    double* __restrict__ r = d.r;
+    const bool dia = d.prec == PREC_JAC_DIAG;
+    const long long S = d.S;
+    const long long c0 = cidx(d, x, y0);
+    const int rows = min(4, d.y_max - y0);
+    double sv[6], kyv[5], rv[4], uv[4], mv[4];
+#pragma unroll
+    for (int i = 0; i < 6; i++) sv[i] = sdi[c0 + min(i - 1, rows) * S];
+#pragma unroll
+    for (int i = 0; i < 5; i++) kyv[i] = __ldg(d.Ky + c0 + min(i, rows) * S);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const long long c = c0 + min(j, rows - 1) * S;
+      uv[j] = u[c] + sv[j + 1];
+      rv[j] = bms_v<F>(r[c], __ldg(d.diag + c), kyv[j + 1], kyv[j], __ldg(d.Kx + c + 1),
+                       __ldg(d.Kx + c), sv[j + 1], sv[j + 2], sv[j], sdi[c + 1], sdi[c - 1]);
+      mv[j] = dia ? __ldg(d.Mi + c) : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (j < rows) {
+        const long long c = c0 + j * S;
+        double b = emu_dmul(beta, rv[j]);
+        if (dia) b = emu_dmul(b, mv[j]);
+        u[c] = uv[j];
+        r[c] = rv[j];
+        sdo[c] = F ? __fma_rn(alpha, sv[j + 1], b) : alpha * sv[j + 1] + b;
+      }
+  });
+}
+
 // tea_leaf_ppcg_solve_update_r, tea_leaf_ppcg_cl.cl:62-88
 template <int TH, int F>
 __global__ void __launch_bounds__(kBlock, 1)
@@ -1154,17 +1201,22 @@ void launch_cg_calc_p(Chunk& c, double beta) {
 }
 
 void launch_cheby_init_p(Chunk& c, double theta) {
-  TH_DISPATCH(c, "tea_leaf_cheby_solve_init_p", k_cheby_p, c.dev(), c.red(), 0,
-              div_const(theta), 0.0, 0.0);
-}
-
-// calc_p alone (block Jacobi takes k_cheby_calc_pu_block, with calc_u)
-void launch_cheby_calc_p(Chunk& c, double alpha, double beta) {
-  TH_DISPATCH(c, "tea_leaf_cheby_solve_calc_p", k_cheby_p, c.dev(), c.red(), 1,
-              div_const(1.0), alpha, beta);
+  TH_DISPATCH(c, "tea_leaf_cheby_solve_init_p", k_cheby_init_p, c.dev(), c.red(),
+              div_const(theta));
 }
 
 void launch_cheby_calc_pu(Chunk& c, double alpha, double beta, double* un) {
+  if (c.prec != PREC_JAC_BLOCK) {
+    const Dev d4 = dev4(c);
+    const char* name = "tea_leaf_cheby_solve_calc_p_u";
+    if (c.arith == 2)
+      launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<2>, d4, c.red(), alpha, beta, un);
+    else if (c.arith == 1)
+      launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<1>, d4, c.red(), alpha, beta, un);
+    else
+      launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<0>, d4, c.red(), alpha, beta, un);
+    return;
+  }
   TH_DISPATCH(c, "tea_leaf_cheby_solve_calc_p_u", k_cheby_calc_pu_block, c.dev(), c.red(),
               alpha, beta, un);
 }
@@ -1182,6 +1234,15 @@ void launch_ppcg_step(Chunk& c, double alpha, double beta, const double* sdi, do
   const Dev d4 = dev4(c);
   const char* name = "tea_leaf_ppcg_solve_inner_step";
   const ResState* st = nullptr;
+  if (c.prec != PREC_JAC_BLOCK) {
+    if (c.arith == 2)
+      launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<2>, d4, c.red(), alpha, beta, st, sdi, sdo);
+    else if (c.arith == 1)
+      launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<1>, d4, c.red(), alpha, beta, st, sdi, sdo);
+    else
+      launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<0>, d4, c.red(), alpha, beta, st, sdi, sdo);
+    return;
+  }
   if (c.arith == 2)
     launch_tile_ns(c, name, d4.ns, k_ppcg_step<2>, d4, c.red(), alpha, beta, st, sdi, sdo);
   else if (c.arith == 1)
@@ -1444,10 +1505,11 @@ static void enqueue_ppcg_iterations_t(Chunk& c, int iters) {
   const bool blk = c.prec == PREC_JAC_BLOCK;
   const int gs = blk ? tile_grid(c, k_ppcg_calc_sd_block<F>, sd_blocks(d4))
                      : tile_grid(c, k_ppcg_sd<4, F>, d4.ns);
-  const int gst = tile_grid(c, k_ppcg_step<F>, d4.ns);
-  // block Jacobi: inner steps two at a time through k_ppcg_step, the first
-  // writing sd to the second buffer and the second back, so each outer
-  // iteration ends with sd where it began
+  auto* const step = blk ? k_ppcg_step<F> : k_ppcg_step_point<F>;
+  const int gst = tile_grid(c, step, d4.ns);
+  // inner steps two at a time in one pass each, the first writing sd to the
+  // second buffer and the second back, so each outer iteration ends with sd
+  // where it began
   double* const sd_a = d4.sd;
   double* const sd_b = c.sd2.f;
   const int gz = tile_grid(c, k_ppcg_rz_step<TH, F>);
@@ -1456,11 +1518,11 @@ static void enqueue_ppcg_iterations_t(Chunk& c, int iters) {
     k_cg_calc_w<TH, F><<<gw, kBlock, 0, c.stream>>>(d, red, st);
     k_ppcg_ur_sd<TH, F><<<gu, kBlock, 0, c.stream>>>(d, red, st, theta);
     for (int k = 0; k < c.n_ppcg; k++) {
-      if (blk && sd_b && k + 1 < c.n_ppcg) {
-        k_ppcg_step<F><<<gst, kBlock, 0, c.stream>>>(d4, red, c.ppcg_alpha_h[k],
-                                                     c.ppcg_beta_h[k], st, sd_a, sd_b);
-        k_ppcg_step<F><<<gst, kBlock, 0, c.stream>>>(d4, red, c.ppcg_alpha_h[k + 1],
-                                                     c.ppcg_beta_h[k + 1], st, sd_b, sd_a);
+      if (k + 1 < c.n_ppcg) {
+        step<<<gst, kBlock, 0, c.stream>>>(d4, red, c.ppcg_alpha_h[k], c.ppcg_beta_h[k], st,
+                                           sd_a, sd_b);
+        step<<<gst, kBlock, 0, c.stream>>>(d4, red, c.ppcg_alpha_h[k + 1], c.ppcg_beta_h[k + 1],
+                                           st, sd_b, sd_a);
         k++;
         continue;
       }
@@ -1681,8 +1743,8 @@ int resident_ppcg_iterations(int n_begin, int loop_max, double rro_in,
   flush_pending_inner(c);
   const bool pairs = resident_pairs(c);
   if (pairs && (!ensure_alt_fields(c) || !tb_prepare(c))) return -1;
-  // the one-pass inner steps (k_ppcg_step) write sd to the second buffer
-  if (c.prec == PREC_JAC_BLOCK && !ensure_alt_fields(c)) return -1;
+  // the one-pass inner steps write sd to the second buffer
+  if (!ensure_alt_fields(c)) return -1;
   std::vector<double> key = {c.ppcg_theta, (double)c.arith, (double)c.n_ppcg,
                              (double)c.field_epoch, pairs ? 1.0 : 0.0};
   key.insert(key.end(), c.ppcg_alpha_h, c.ppcg_alpha_h + c.n_ppcg);
@@ -1715,8 +1777,7 @@ int resident_ppcg_iterations(int n_begin, int loop_max, double rro_in,
     c.res_ppcg_key = key;
   }
   const int per_iter = pairs ? 4 + c.n_ppcg / 2 + 2 * (c.n_ppcg % 2)
-                       : c.prec == PREC_JAC_BLOCK ? 4 + c.n_ppcg + c.n_ppcg % 2
-                                                  : 4 + 2 * c.n_ppcg;
+                       : 4 + c.n_ppcg + c.n_ppcg % 2;
   const long long max_batches = (long long)(loop_max - n_begin) / batch + 3;
   for (long long nb = 0;; nb++) {
     if (nb >= max_batches) {

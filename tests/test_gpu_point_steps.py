@@ -1,0 +1,26 @@
+"""PPCG inner steps and Chebyshev iterations without a preconditioner or with
+the diagonal one, each in one pass, against the CPU oracle bit for bit: tile
+edges (two cells, 31 to 33 and 255 to 257 columns, 1 to 5 rows past a strip),
+odd inner step counts, halo depths, reflective faces and the three arithmetic
+forms."""
+import pytest
+
+from oracle import oracle
+from tealeaf_opencl_gb300 import lib
+from tests import scenarios
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("solver", ["ppcg", "chebyshev"])
+@pytest.mark.parametrize("prec", ["none", "jac_diag"])
+@pytest.mark.parametrize("x,y,halo,form,reflective", [
+    (2, 1, 1, 1, False), (31, 5, 2, 2, False), (33, 6, 1, 0, True), (255, 7, 1, 1, True),
+    (257, 13, 3, 2, True), (300, 67, 1, 1, False),
+])
+def test_one_pass_steps_match_oracle(solver, prec, x, y, halo, form, reflective):
+    args = (x, y, halo, lib.SOLVER[solver], lib.PREC[prec])
+    recs = [scenarios.run(mod.Chunk(*args), x, y, solver, prec, halo=halo, inner=5,
+                          cg_iters=4 if x * y > 8 else 0, lognormal_seed=3, fused=form,
+                          reflective=reflective) for mod in (lib, oracle)]
+    assert scenarios.compare(*recs) == []
