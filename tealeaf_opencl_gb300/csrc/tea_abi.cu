@@ -921,9 +921,12 @@ extern "C" void tea_leaf_jacobi_solve_kernel_ocl_(double* error) {
   *error = NAN;
   if (!need_chunk("tea_leaf_jacobi_solve_kernel_ocl_")) return;
   Chunk& c = chunk();
-  launch_jacobi_copy_u(c);
+  // the new u goes to the second buffer, which then becomes u
+  if (!ensure_u_alt(c)) return;
   arm_host_result(c);
-  launch_jacobi_solve(c);
+  launch_jacobi_sweep(c, c.u2.f);
+  std::swap(c.u, c.u2);
+  c.field_epoch++;
   fetch(1, error);
 }
 

@@ -136,7 +136,7 @@ struct Chunk {
   // allocated on first use, with the halos of the live pair
   Field r2, sd2;
   // second u buffer of the Chebyshev iteration with calc_u folded into
-  // calc_p, which writes the new u, halo included, to the
+  // calc_p and of the Jacobi sweep, which write the new u, halo included, to the
   // buffer it does not read; the two then trade places
   Field u2;
   Field p2;  // second p buffer of the resident CG loop (tea_cg_loop.cu)
@@ -213,8 +213,8 @@ void launch_ppcg_update_r(Chunk& c);
 // update_r and calc_sd of one inner step in one pass, sd read from sdi and the new sd written to sdo
 void launch_ppcg_step(Chunk& c, double alpha, double beta, const double* sdi, double* sdo);
 void launch_ppcg_calc_sd(Chunk& c, double alpha, double beta);
-void launch_jacobi_copy_u(Chunk& c);
-void launch_jacobi_solve(Chunk& c);
+// one Jacobi sweep, the new u into unew
+void launch_jacobi_sweep(Chunk& c, double* unew);
 void launch_finalise(Chunk& c);
 void launch_field_summary(Chunk& c);
 void launch_update_halo(Chunk& c, int mask, int depth);

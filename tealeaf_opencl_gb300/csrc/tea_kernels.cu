@@ -984,56 +984,60 @@ __global__ void __launch_bounds__(kBlock, 1)
   });
 }
 
-// tea_leaf_jacobi_copy_u, tea_leaf_jacobi_cl.cl:3-13 (un is vector_Mi, as
-// in the reference, ocl_kernels.cpp:576-585)
+// tea_leaf_jacobi_copy_u and tea_leaf_jacobi_solve in one pass
+// (tea_leaf_jacobi_cl.cl:3-42; un is vector_Mi, as in the reference,
+// ocl_kernels.cpp:576-585): un = u over the interior, one sweep from un, the sum
+// of |u - un|.  The sweep reads the old u where un would hold its copy, and
+// un's own halo; the new u goes to unew with u's halo ring, and un gets the old
+// u, so the fields end as the two kernels leave them.  48 bytes per cell in
+// place of 56 and one launch in place of two.  The sums of each cell stay in
+// the reference's association (its denominator differs from the stored
+// diagonal); two of the four products run on the integer pipes beside the
+// division (bit-identical).
 template <int TH, int F>
-__global__ void __launch_bounds__(kBlock) k_jacobi_copy_u(Dev d, Red red) {
-  tile_driver<TH, 0>(d, red, [&](int x, int y0, bool xin, double* acc) {
-    if (!xin) return;
-#pragma unroll 1
-    for (int g = y0; g < y0 + TH; g += 4) {
-      const long long c0 = cidx(d, x, g);
-      double uv[4];
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (g + j < d.y_max) uv[j] = d.u[c0 + j * d.S];
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (g + j < d.y_max) d.un[c0 + j * d.S] = uv[j];
-    }
-  });
-}
-
-// tea_leaf_jacobi_solve, tea_leaf_jacobi_cl.cl:15-42 (the same arithmetic in
-// both forms; its denominator associates differently from the diagonal)
-template <int TH, int F>
-__global__ void __launch_bounds__(kBlock) k_jacobi_solve(Dev d, Red red) {
+__global__ void __launch_bounds__(kBlock) k_jacobi_sweep(Dev d, Red red, double* unew_) {
   tile_driver<TH, 1>(d, red, [&](int x, int y0, bool xin, double* acc) {
+    const double* __restrict__ u = d.u;
+    const double* __restrict__ hal = d.un;  // read only outside the interior
+    double* __restrict__ un = d.un;         // written only inside it
+    double* __restrict__ unew = unew_;
     const long long S = d.S;
+    if (!xin) return;
+    const double* west = x > 0 ? u : hal;
+    const double* east = x + 1 < d.x_max ? u : hal;
+    const int rows = min(TH, d.y_max - y0);
 #pragma unroll 1
-    for (int g = y0; g < y0 + TH; g += 4) {
-      const long long c0 = cidx(d, x, g);
-      double uv[4], v[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int g = 0; g < rows; g += 4) {
+      const long long c0 = cidx(d, x, y0 + g);
+      const int last = rows - 1 - g;  // last interior row of the group, or more
+      double uc[6], kyv[5], nw[4], v[4];
+#pragma unroll
+      for (int i = 0; i < 6; i++) {
+        const int j = min(i - 1, last + 1), y = y0 + g + j;
+        uc[i] = (y < 0 || y >= d.y_max ? hal : u)[c0 + j * S];
+      }
+#pragma unroll
+      for (int i = 0; i < 5; i++) kyv[i] = __ldg(d.Ky + c0 + min(i, last + 1) * S);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const long long c = c0 + min(j, last) * S;
+        const double kxc = __ldg(d.Kx + c), kxe = __ldg(d.Kx + c + 1);
+        const double s = __ldg(d.u0 + c) + emu_dmul(kxe, east[c + 1]) + kxc * west[c - 1] +
+                         emu_dmul(kyv[j + 1], uc[j + 2]) + kyv[j] * uc[j];
+        nw[j] = emu_ddiv_var(s, 1.0 + (kxc + kxe) + (kyv[j] + kyv[j + 1]));
+        v[j] = j <= last ? fabs(nw[j] - uc[j + 1]) : 0.0;
+      }
 #pragma unroll
       for (int j = 0; j < 4; j++)
-        if (xin && g + j < d.y_max) {
-          const long long c = c0 + j * S;
-          const double* un = d.un;
-          const double kxc = d.Kx[c], kxe = d.Kx[c + 1];
-          const double kyc = d.Ky[c], kyn = d.Ky[c + S];
-          const double u1 = emu_ddiv_var(d.u0[c] + kxe * un[c + 1] + kxc * un[c - 1] +
-                                             kyn * un[c + S] + kyc * un[c - S],
-                                         1.0 + (kxc + kxe) + (kyc + kyn));
-          uv[j] = u1;
-          v[j] = fabs(u1 - un[c]);
+        if (j <= last) {
+          unew[c0 + j * S] = nw[j];
+          un[c0 + j * S] = uc[j + 1];
         }
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (xin && g + j < d.y_max) d.u[c0 + j * S] = uv[j];
 #pragma unroll
       for (int j = 0; j < 4; j++) acc[0] = acc[0] + v[j];
     }
   });
+  copy_halo_ring(d, d.u, unew_);
 }
 
 // tea_leaf_finalise, tea_leaf_common_cl.cl:4-15
@@ -1276,12 +1280,8 @@ void launch_ppcg_calc_sd(Chunk& c, double alpha, double beta) {
               div_const(1.0), alpha, beta, (const ResState*)nullptr);
 }
 
-void launch_jacobi_copy_u(Chunk& c) {
-  TH4_DISPATCH(c, "tea_leaf_jacobi_copy_u", k_jacobi_copy_u, dev4(c), c.red());
-}
-
-void launch_jacobi_solve(Chunk& c) {
-  TH_DISPATCH(c, "tea_leaf_jacobi_solve", k_jacobi_solve, c.dev(), c.red());
+void launch_jacobi_sweep(Chunk& c, double* unew) {
+  TH_DISPATCH(c, "tea_leaf_jacobi_solve", k_jacobi_sweep, c.dev(), c.red(), unew);
 }
 
 void launch_finalise(Chunk& c) {
