@@ -4,18 +4,20 @@
 // Every problem keeps its own padded fields (one arena for the batch), its
 // own reduction partials, completion counter and CG scalar state
 // (ResState) in device memory.  One CG iteration of every still-active
-// problem is three persistent grid-stride kernels over a flat work list of
-// (problem, supertile) items, largest problems first:
-//   k_b_calc_w   w = A p, p.w           (tea_leaf_cg_cl.cl:45-69)
-//   k_b_calc_ur  u, r, z updates, r.z   (tea_leaf_cg_cl.cl:73-137)
-//   k_b_calc_p   p = z + beta p         (tea_leaf_cg_cl.cl:141-160)
-// The block that completes a problem's last supertile of a phase finishes
-// that problem's sum in the fixed order of tea_device.cuh and, after
-// calc_ur, takes its CG scalar step and exit test on the device
-// (cg_scalar_step).  Items of problems that have stopped are skipped.  The
-// phase boundaries are kernel boundaries, so no block ever waits for
-// another.  Batches of iterations are replayed from a captured CUDA graph
-// until no problem is active.
+// problem is the two passes of the single-chunk loop (tea_cg_loop.cu) over a
+// flat work list of (problem, supertile) items, largest problems first:
+//   pass w  p' = z + beta p, u += alpha p, w = A p', p'.w
+//   pass r  r -= alpha w, z = M^-1 r, r.z
+// (tea_leaf_cg_cl.cl:45-160).  A block takes one contiguous run of the list,
+// so it looks a problem up, loads its field set and counts itself done once
+// per problem, not once per item.  The block that completes a problem's last
+// item of a pass finishes that problem's sum in the fixed order of
+// tea_device.cuh and takes its scalar steps (alpha after pass w; beta and the
+// exit test, cg_scalar_step, after pass r).  Items of problems that have
+// stopped are skipped.  The pass boundaries are kernel boundaries, so no block
+// ever waits for another.  Batches of iterations are replayed from a captured
+// CUDA graph until no problem is active; a last kernel of each batch finishes
+// u of the problems that stopped in it.
 //
 // Each problem's arithmetic, summation order and exit test are those of a
 // single-chunk run of that problem, so its iteration counts and field
@@ -47,11 +49,6 @@ struct WorkList {
   int G;
 };
 
-// Minimum resident blocks per SM of the iteration kernels (a register cap).
-// Measured on configuration 4: 2.59e10 cell-iterations/s without the bound,
-// 2.70e10 / 2.63e10 / 2.56e10 with 4 / 6 / 8.
-constexpr int kBatchMinBlocks = 4;
-
 __device__ __forceinline__ int units_of(int ns, int G) { return (ns + G - 1) / G; }
 
 // Position in the active list of the problem that owns unit u (every
@@ -68,71 +65,60 @@ __device__ __forceinline__ int find_problem(const WorkList& wl, int np, int u) {
   return lo;
 }
 
-// Runs body(x, y0, xin, acc) for this warp's tile of supertile s of a
-// problem and butterflies the NV sums (the inner part of tile_driver).
-template <int NV, class Body>
-__device__ __forceinline__ void run_supertile(const Dev& d, int s, double* acc,
-                                              Body body) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int sy = s / d.nsx, sx = s - sy * d.nsx;
-  const int tx = sx * kTilesPerSuper + warp;
-#pragma unroll
-  for (int v = 0; v < (NV > 0 ? NV : 1); v++) acc[v] = 0.0;
-  if (tx < d.ntx) {
-    const int x = tx * kTileW + lane;
-    body(x, sy * d.th, x < d.x_max, acc);
-    if (NV > 0) {
-#pragma unroll
-      for (int v = 0; v < NV; v++) acc[v] = bfly(acc[v]);
-    }
-  }
-}
+constexpr int kRounds = 4;  // supertiles whose tile sums share a sweep
 
-// The supertile partial sums of supertiles s0..s1-1 of a problem (one
-// value), four supertiles at a time with the shared butterflies of
-// tea_device.cuh (bfly4, supertile_partials4): the same sums as one
-// run_supertile and supertile_partial per supertile.  sh holds 32 doubles.
+struct BatchShared {
+  double lanes[kRounds * kBlock];
+  double tiles[32];  // tile sums of up to 4 supertiles, scratch of the final sum
+  Dev d;             // field set and reduction of the run's problem: read from
+  long long red[sizeof(Red) / 8];  // here they cost no registers over a pass
+  unsigned int last;
+};
+
+// Runs body(x, y0) -> lane sum over supertiles s0..s1-1 of a problem, one
+// tile per warp, and stores the supertile partials: four supertiles' lane sums
+// go through shared memory and whole warps sum four tiles (bfly4) and four
+// supertiles (supertile_partials4) each.
 template <class Body>
-__device__ __forceinline__ void unit_partials(const Dev& d, const Red& red, int s0,
-                                              int s1, double* sh, Body body) {
+__device__ __forceinline__ void run_partials(const Dev& d, const Red& red, int s0, int s1,
+                                             BatchShared& sh, Body body) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int g = s0; g < s1; g += 4) {
-    double tiles[4];
-    int s_k[4];
+  for (int g = s0; g < s1; g += kRounds) {
+    const int nr = min(kRounds, s1 - g);
 #pragma unroll 1
-    for (int k = 0; k < 4; k++) {
-      double acc[1] = {0.0};
-      const int s = g + k;
-      if (s < s1) {
-        const int sy = s / d.nsx, sx = s - sy * d.nsx;
-        const int tx = sx * kTilesPerSuper + warp;
-        if (tx < d.ntx) {
-          const int x = tx * kTileW + lane;
-          body(x, sy * d.th, x < d.x_max, acc);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 4; q++)
-        if (q == k) {
-          tiles[q] = acc[0];
-          s_k[q] = s < s1 ? s : d.ns;
-        }
+    for (int k = 0; k < nr; k++) {
+      const int s = g + k, sy = s / d.nsx, sx = s - sy * d.nsx;
+      const int tx = sx * kTilesPerSuper + warp;
+      double acc = 0.0;
+      if (tx < d.ntx) acc = body(tx * kTileW + lane, sy * d.th);
+      sh.lanes[k * kBlock + threadIdx.x] = acc;
     }
-    const double t = bfly4(tiles[0], tiles[1], tiles[2], tiles[3]);
-    if ((lane & 7) == 0) sh[bfly4_slot(lane) * 8 + warp] = t;
-    supertile_partials4<1>(red, s_k, d.ns, sh);
+    __syncthreads();
+    if (warp < 2 * nr) {
+      const double* a = sh.lanes + warp * 128 + lane;
+      const double t = bfly4(a[0], a[32], a[64], a[96]);
+      if ((lane & 7) == 0) sh.tiles[warp * 4 + bfly4_slot(lane)] = t;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      double t = sh.tiles[lane];
+      t = t + 0.0;
+#pragma unroll
+      for (int off = 4; off >= 1; off >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, off);
+      if ((lane & 7) == 0 && (lane >> 3) < nr) red.partials[g + (lane >> 3)] = t;
+    }
   }
 }
 
-// Counts one finished unit of a problem; true in the block that finished
-// the problem's last one, which also resets the counter.
-__device__ __forceinline__ bool unit_done(unsigned int* counter, int units,
-                                          unsigned int* is_last) {
+// Counts `mine` of a problem's `units` units done; true in the block that
+// finished the last one, which also resets the counter.
+__device__ __forceinline__ bool units_done(unsigned int* counter, int mine, int units,
+                                           unsigned int* is_last) {
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
-    const unsigned int t = atomicAdd(counter, 1u);
-    *is_last = (t == (unsigned int)units - 1u) ? 1u : 0u;
+    const unsigned int t = atomicAdd(counter, (unsigned int)mine);
+    *is_last = (t + (unsigned int)mine == (unsigned int)units) ? 1u : 0u;
     if (*is_last) *counter = 0u;
   }
   __syncthreads();
@@ -140,181 +126,157 @@ __device__ __forceinline__ bool unit_done(unsigned int* counter, int units,
   return *is_last != 0u;
 }
 
-// A double of the loop state written by another block of the same
-// (persistent) launch is read through L2 (CG); plain otherwise.
-template <bool CG>
-__device__ __forceinline__ double st_load(const double* p) {
-  return CG ? __ldcg(p) : *p;
+// The block's run of the work list, problem by problem:
+// f(problem, its Dev, its Red, first and last+1 supertile, units of the run).
+template <class F>
+__device__ __forceinline__ void for_each_run(const Dev* __restrict__ devs,
+                                             const Red* __restrict__ reds, const WorkList& wl,
+                                             int U, int np, BatchShared& sh, F f) {
+  const int nb = gridDim.x, b = blockIdx.x;
+  int u = (int)((long long)b * U / nb);
+  const int end = (int)((long long)(b + 1) * U / nb);
+  if (u >= end) return;
+  for (int j = find_problem(wl, np, u); u < end; j++) {
+    const int i = wl.plist[j], first = wl.ustart[j];
+    const int stop = min(end, wl.ustart[j + 1]);
+    __syncthreads();  // the run before has been worked off
+    for (int k = threadIdx.x; k < (int)(sizeof(Dev) / 4); k += kBlock)
+      ((int*)&sh.d)[k] = ((const int*)(devs + i))[k];
+    for (int k = threadIdx.x; k < (int)(sizeof(Red) / 4); k += kBlock)
+      ((int*)sh.red)[k] = ((const int*)(reds + i))[k];
+    __syncthreads();
+    f(i, sh.d, *(const Red*)sh.red, (u - first) * wl.G, min((stop - first) * wl.G, sh.d.ns), stop - u);
+    u = stop;
+  }
 }
 
-// The three phases of one CG iteration over the block's work units.  The
-// separate kernels below run one phase each; k_b_iterations runs them in
-// turn with grid barriers between them (CG = true: fields and loop state
-// written by other blocks in an earlier phase are read through L2).
-
-// w = A p and p.w of every active problem (tea_leaf_cg_cl.cl:45-69); the
-// finishing block stores pw and alpha = rro/pw in the problem's loop state.
-template <int F, bool CG>
+// Pass w of every active problem.  p alternates between d.p and the second
+// buffer with the iteration number, the first
+// iteration copying it.  The loop state is read through L2: in the persistent
+// launch other blocks write it.
+template <int F>
 __device__ __forceinline__ void phase_w(const Dev* __restrict__ devs,
-                                        const Red* __restrict__ reds, ResState* st,
-                                        const WorkList& wl, int U, int np, double* sh,
-                                        unsigned int* is_last) {
-  for (int u = blockIdx.x; u < U; u += gridDim.x) {
-    const int j = find_problem(wl, np, u);
-    const int i = wl.plist[j];
-    if (*(volatile int*)&st[i].stop) continue;
-    const Dev d = devs[i];
-    const Red red = reds[i];
-    const int s0 = (u - wl.ustart[j]) * wl.G, s1 = min(s0 + wl.G, d.ns);
-    unit_partials(d, red, s0, s1, sh, [&](int x, int y0, bool xin, double* a) {
-      // the three-kernel mode takes the restrict-qualified bodies; the
-      // persistent mode reads other blocks' writes through L2 (CG)
-      if constexpr (CG) {
-        if (d.th == 16)
-          cg_w_tile<16, F, CG>(d, x, y0, xin, a);
-        else
-          cg_w_tile<4, F, CG>(d, x, y0, xin, a);
-      } else {
-        if (d.th == 16)
-          cg_w_tile_r<16, F>(d, x, y0, xin, a);
-        else
-          cg_w_tile_r<4, F>(d, x, y0, xin, a);
-      }
+                                        const Red* __restrict__ reds,
+                                        double* const* __restrict__ p2s, ResState* st,
+                                        const WorkList& wl, int U, int np, BatchShared& sh) {
+  for_each_run(devs, reds, wl, U, np, sh,
+               [&](int i, const Dev& d, const Red& red, int s0, int s1, int mine) {
+    if (*(volatile int*)&st[i].stop) return;
+    const int n = *(volatile int*)&st[i].n;
+    const double alpha = __ldcg(&st[i].alpha), beta = __ldcg(&st[i].beta);
+    double* const p2 = p2s[i];
+    const double* pin = (n & 1) ? d.p : p2;
+    double* pout = (n & 1) ? p2 : d.p;
+    const double* z = d.prec != PREC_NONE ? d.z : d.r;
+    run_partials(d, red, s0, s1, sh, [&](int x, int y0) {
+      return d.th == 16 ? loop_w_tile<16, F, true>(d, pin, pout, z, x, y0, alpha, beta, n == 1)
+                        : loop_w_tile<4, F, true>(d, pin, pout, z, x, y0, alpha, beta, n == 1);
     });
-    if (unit_done(red.counter, units_of(d.ns, wl.G), is_last)) {
-      block_final_sum<1>(red.partials, red.stride, d.ns, red.result, sh);
+    if (units_done(red.counter, mine, units_of(d.ns, wl.G), &sh.last)) {
+      block_final_sum<1>(red.partials, red.stride, d.ns, red.result, sh.tiles);
       if (threadIdx.x == 0) {
-        // alpha once per problem: a division in every thread of phase_ur
-        // costs each unit there about 10 FP64 instructions per warp
         st[i].pw = red.result[0];
-        st[i].alpha = st_load<CG>(&st[i].rro) / red.result[0];
+        st[i].alpha = __ldcg(&st[i].rro) / red.result[0];
         __threadfence();
       }
       __syncthreads();
     }
-  }
+  });
 }
 
-// u, r, z updates and r.z (tea_leaf_cg_cl.cl:73-137);
-// the finishing block takes the problem's scalar step and exit test.
-template <int F, bool CG>
-__device__ __forceinline__ void phase_ur(const Dev* __restrict__ devs,
-                                         const Red* __restrict__ reds, ResState* st,
-                                         const WorkList& wl, int U, int np, double* sh,
-                                         unsigned int* is_last) {
-  for (int u = blockIdx.x; u < U; u += gridDim.x) {
-    const int j = find_problem(wl, np, u);
-    const int i = wl.plist[j];
-    if (*(volatile int*)&st[i].stop) continue;
-    const Dev d = devs[i];
-    const Red red = reds[i];
-    const double alpha = st_load<CG>(&st[i].alpha);
-    const int s0 = (u - wl.ustart[j]) * wl.G, s1 = min(s0 + wl.G, d.ns);
-    unit_partials(d, red, s0, s1, sh, [&](int x, int y0, bool xin, double* a) {
-      if constexpr (CG) {
-        if (d.th == 16)
-          cg_ur_tile<16, F, 1, CG>(d, x, y0, xin, a, alpha);
-        else
-          cg_ur_tile<4, F, 1, CG>(d, x, y0, xin, a, alpha);
-      } else {
-        if (d.th == 16)
-          cg_ur_tile_r<16, F, 1>(d, x, y0, xin, a, alpha);
-        else
-          cg_ur_tile_r<4, F, 1>(d, x, y0, xin, a, alpha);
-      }
+// Pass r; the finishing block takes the problem's scalar step and exit test.
+template <int F>
+__device__ __forceinline__ void phase_r(const Dev* __restrict__ devs,
+                                        const Red* __restrict__ reds, ResState* st,
+                                        const WorkList& wl, int U, int np, BatchShared& sh) {
+  for_each_run(devs, reds, wl, U, np, sh,
+               [&](int i, const Dev& d, const Red& red, int s0, int s1, int mine) {
+    if (*(volatile int*)&st[i].stop) return;
+    const double alpha = __ldcg(&st[i].alpha);
+    run_partials(d, red, s0, s1, sh, [&](int x, int y0) {
+      double acc[1] = {0.0};
+      if (d.th == 16)
+        loop_r_tile<16, F>(d, x, y0, alpha, acc);
+      else
+        loop_r_tile<4, F>(d, x, y0, alpha, acc);
+      return acc[0];
     });
-    if (unit_done(red.counter, units_of(d.ns, wl.G), is_last)) {
-      block_final_sum<1>(red.partials, red.stride, d.ns, red.result, sh);
+    if (units_done(red.counter, mine, units_of(d.ns, wl.G), &sh.last)) {
+      block_final_sum<1>(red.partials, red.stride, d.ns, red.result, sh.tiles);
       if (threadIdx.x == 0) {
         cg_scalar_step<1>(&st[i], alpha, red.result);
         __threadfence();
       }
       __syncthreads();
     }
-  }
+  });
 }
 
-// p = z + beta p (tea_leaf_cg_cl.cl:141-160) for every problem whose
-// calc_ur has just run, including the iteration on which it stopped.
-template <int F, bool CG>
-__device__ __forceinline__ void phase_p(const Dev* __restrict__ devs,
-                                        const Red* __restrict__ reds, ResState* st,
-                                        const WorkList& wl, int U, int np,
-                                        unsigned int* is_last) {
-  for (int u = blockIdx.x; u < U; u += gridDim.x) {
-    const int j = find_problem(wl, np, u);
-    const int i = wl.plist[j];
-    if (!*(volatile int*)&st[i].p_pending) continue;
-    const Dev d = devs[i];
-    const Red red = reds[i];
-    const double beta = st_load<CG>(&st[i].beta);
-    const int s0 = (u - wl.ustart[j]) * wl.G, s1 = min(s0 + wl.G, d.ns);
+// Pass w takes 128 registers (two blocks per SM; at three or four the
+// single-chunk kernel of the same body is slower by a fifth and more), pass r
+// 64.
+template <int F>
+__global__ void __launch_bounds__(kBlock, 2)
+    k_b_pass_w(const Dev* __restrict__ devs, const Red* __restrict__ reds,
+               double* const* __restrict__ p2s, ResState* st, WorkList wl) {
+  __shared__ BatchShared sh;
+  phase_w<F>(devs, reds, p2s, st, wl, wl.counts[0], wl.counts[1], sh);
+}
+
+template <int F>
+__global__ void __launch_bounds__(kBlock, 4)
+    k_b_pass_r(const Dev* __restrict__ devs, const Red* __restrict__ reds, ResState* st,
+               WorkList wl) {
+  __shared__ BatchShared sh;
+  phase_r<F>(devs, reds, st, wl, wl.counts[0], wl.counts[1], sh);
+}
+
+// u += alpha p of the problems that stopped in this batch of iterations (they
+// leave the active list after it).
+template <int F>
+__global__ void __launch_bounds__(kBlock)
+    k_b_pass_end(const Dev* __restrict__ devs, const Red* __restrict__ reds,
+                 double* const* __restrict__ p2s, const ResState* st, WorkList wl) {
+  __shared__ BatchShared sh;
+  for_each_run(devs, reds, wl, wl.counts[0], wl.counts[1], sh,
+               [&](int i, const Dev& d, const Red&, int s0, int s1, int) {
+    if (!st[i].stop) return;
+    const double* p = (st[i].n & 1) ? p2s[i] : d.p;
+    const double alpha = st[i].alpha;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int s = s0; s < s1; s++) {
-      double acc[1];
-      run_supertile<0>(d, s, acc, [&](int x, int y0, bool xin, double* a) {
-        if (d.th == 16)
-          cg_p_tile<16, F, CG>(d, x, y0, xin, beta);
-        else
-          cg_p_tile<4, F, CG>(d, x, y0, xin, beta);
-      });
-    }
-    if (unit_done(red.counter, units_of(d.ns, wl.G), is_last)) {
-      if (threadIdx.x == 0) {
-        st[i].p_pending = 0;
-        __threadfence();
+      const int sy = s / d.nsx, sx = s - sy * d.nsx;
+      const int x = (sx * kTilesPerSuper + warp) * kTileW + lane;
+      if (x >= d.x_max) continue;
+      const int y1 = min((sy + 1) * d.th, d.y_max);
+      for (int y = sy * d.th; y < y1; y++) {
+        const long long c = cidx(d, x, y);
+        d.u[c] = F ? __fma_rn(alpha, p[c], d.u[c]) : d.u[c] + alpha * p[c];
       }
-      __syncthreads();
     }
-  }
-}
-
-template <int F>
-__global__ void __launch_bounds__(kBlock, kBatchMinBlocks)
-    k_b_calc_w(const Dev* __restrict__ devs, const Red* __restrict__ reds,
-               ResState* st, WorkList wl) {
-  __shared__ double sh[32];
-  __shared__ unsigned int is_last;
-  phase_w<F, false>(devs, reds, st, wl, wl.counts[0], wl.counts[1], sh, &is_last);
-}
-
-template <int F>
-__global__ void __launch_bounds__(kBlock, kBatchMinBlocks)
-    k_b_calc_ur(const Dev* __restrict__ devs, const Red* __restrict__ reds,
-                ResState* st, WorkList wl) {
-  __shared__ double sh[32];
-  __shared__ unsigned int is_last;
-  phase_ur<F, false>(devs, reds, st, wl, wl.counts[0], wl.counts[1], sh, &is_last);
-}
-
-template <int F>
-__global__ void __launch_bounds__(kBlock, kBatchMinBlocks)
-    k_b_calc_p(const Dev* __restrict__ devs, const Red* __restrict__ reds,
-               ResState* st, WorkList wl) {
-  __shared__ unsigned int is_last;
-  phase_p<F, false>(devs, reds, st, wl, wl.counts[0], wl.counts[1], &is_last);
+  });
 }
 
 // `iters` CG iterations of every active problem in one cooperative launch:
-// the three phases above with grid barriers between them (all blocks are
+// the two passes above with grid barriers between them (all blocks are
 // resident).  The active list is fixed for the launch (problems that stop
-// are skipped, as in the separate kernels); bar[0..1] is the barrier,
-// bar[2] its error flag, set if a barrier times out, after which every
-// block returns.  Results are those of the separate kernels.
+// are skipped, as in the separate kernels), and so is each block's run of it,
+// so a lane reads back the u, r and w that it wrote; p and z of neighbours
+// come through L2.  bar[0..1] is the barrier, bar[2] its error flag, set if a
+// barrier times out, after which every block returns.  Results are those of
+// the separate kernels.
 template <int F>
-__global__ void __launch_bounds__(kBlock, kBatchMinBlocks)
+__global__ void __launch_bounds__(kBlock, 2)
     k_b_iterations(const Dev* __restrict__ devs, const Red* __restrict__ reds,
-                   ResState* st, WorkList wl, int iters, unsigned int* bar,
-                   long long spin_limit) {
-  __shared__ double sh[32];
-  __shared__ unsigned int is_last;
+                   double* const* __restrict__ p2s, ResState* st, WorkList wl, int iters,
+                   unsigned int* bar, long long spin_limit) {
+  __shared__ BatchShared sh;
   int* err = (int*)(bar + 2);
   const int U = wl.counts[0], np = wl.counts[1];
   for (int it = 0; it < iters; it++) {
-    phase_w<F, true>(devs, reds, st, wl, U, np, sh, &is_last);
+    phase_w<F>(devs, reds, p2s, st, wl, U, np, sh);
     if (!grid_barrier(bar, err, spin_limit)) return;
-    phase_ur<F, true>(devs, reds, st, wl, U, np, sh, &is_last);
-    if (!grid_barrier(bar, err, spin_limit)) return;
-    phase_p<F, true>(devs, reds, st, wl, U, np, &is_last);
+    phase_r<F>(devs, reds, st, wl, U, np, sh);
     if (!grid_barrier(bar, err, spin_limit)) return;
   }
 }
@@ -459,6 +421,7 @@ struct Batch {
   double* results_h = nullptr;  // pinned, n * kResults
   Dev* devs_d = nullptr;
   Red* reds_d = nullptr;
+  double** p2s_d = nullptr;     // every problem's second p buffer
   ResState* st_d = nullptr;
   int* order_d = nullptr;       // problems, largest first
   int* ustart_all_d = nullptr;  // unit prefix sums over order (n + 1)
@@ -479,7 +442,7 @@ struct Batch {
   tea_gb300_batch_launch launch{0, 16, 1, 0};
   int ustart_G = 0;             // G that ustart_all_d was built for
   int max_bps = 1;
-  int occ[3][3] = {};  // [arithmetic form][w, ur, p]
+  int occ[3][3] = {};  // [arithmetic form][pass w, pass r, end]
   int occ_persistent[3] = {};  // [arithmetic form] k_b_iterations
   cudaGraphExec_t iter_graph = nullptr;
   int graph_bps = 0, graph_iters = 0, graph_G = 0, graph_persistent = 0;
@@ -505,6 +468,7 @@ void release_batch() {
   cudaFree(b.results);
   cudaFree(b.devs_d);
   cudaFree(b.reds_d);
+  cudaFree(b.p2s_d);
   cudaFree(b.st_d);
   cudaFree(b.order_d);
   cudaFree(b.ustart_all_d);
@@ -542,18 +506,18 @@ int occupancy(const void* k) {
   return std::max(v, 1);
 }
 
-// Occupancy of the iteration kernels ([arithmetic form][w, ur, p]) and the
-// largest of them (the upper end of blocks_per_sm).
+// Occupancy of the iteration kernels ([arithmetic form][pass w, pass r, end])
+// and the largest of them (the upper end of blocks_per_sm).
 int set_occupancy(Batch& b) {
-  b.occ[0][0] = occupancy((const void*)k_b_calc_w<0>);
-  b.occ[0][1] = occupancy((const void*)k_b_calc_ur<0>);
-  b.occ[0][2] = occupancy((const void*)k_b_calc_p<0>);
-  b.occ[1][0] = occupancy((const void*)k_b_calc_w<1>);
-  b.occ[1][1] = occupancy((const void*)k_b_calc_ur<1>);
-  b.occ[1][2] = occupancy((const void*)k_b_calc_p<1>);
-  b.occ[2][0] = occupancy((const void*)k_b_calc_w<2>);
-  b.occ[2][1] = occupancy((const void*)k_b_calc_ur<2>);
-  b.occ[2][2] = occupancy((const void*)k_b_calc_p<2>);
+  b.occ[0][0] = occupancy((const void*)k_b_pass_w<0>);
+  b.occ[0][1] = occupancy((const void*)k_b_pass_r<0>);
+  b.occ[0][2] = occupancy((const void*)k_b_pass_end<0>);
+  b.occ[1][0] = occupancy((const void*)k_b_pass_w<1>);
+  b.occ[1][1] = occupancy((const void*)k_b_pass_r<1>);
+  b.occ[1][2] = occupancy((const void*)k_b_pass_end<1>);
+  b.occ[2][0] = occupancy((const void*)k_b_pass_w<2>);
+  b.occ[2][1] = occupancy((const void*)k_b_pass_r<2>);
+  b.occ[2][2] = occupancy((const void*)k_b_pass_end<2>);
   b.occ_persistent[0] = occupancy((const void*)k_b_iterations<0>);
   b.occ_persistent[1] = occupancy((const void*)k_b_iterations<1>);
   b.occ_persistent[2] = occupancy((const void*)k_b_iterations<2>);
@@ -627,7 +591,7 @@ extern "C" int tea_gb300_batch_create(int n, const int* x_cells, const int* y_ce
   cudaEventCreate(&b.s1);
 
   // arena layout: problem after problem, each with its fields in turn
-  const int nf = preconditioner == PREC_JAC_BLOCK ? 15 : 13;
+  const int nf = preconditioner == PREC_JAC_BLOCK ? 16 : 14;
   b.probs.resize(n);
   size_t total = 0, part_total = 0;
   std::vector<size_t> offs(n), part_offs(n);
@@ -672,6 +636,7 @@ extern "C" int tea_gb300_batch_create(int n, const int* x_cells, const int* y_ce
     release_batch();
     return -1;
   }
+  std::vector<double*> p2s(n);
   for (int i = 0; i < n; i++) {
     Problem& p = b.probs[i];
     Dev d;
@@ -698,6 +663,7 @@ extern "C" int tea_gb300_batch_create(int n, const int* x_cells, const int* y_ce
     d.Ky = next();
     d.z = next();
     d.diag = next();
+    p2s[i] = next();
     if (preconditioner == PREC_JAC_BLOCK) {
       d.cp = next();
       d.bfp = next();
@@ -722,6 +688,9 @@ extern "C" int tea_gb300_batch_create(int n, const int* x_cells, const int* y_ce
   }
   if (!check_cuda(cudaMalloc(&b.devs_d, n * sizeof(Dev)), "cudaMalloc devs") ||
       !check_cuda(cudaMalloc(&b.reds_d, n * sizeof(Red)), "cudaMalloc reds") ||
+      !check_cuda(cudaMalloc(&b.p2s_d, n * sizeof(double*)), "cudaMalloc p2s") ||
+      !check_cuda(cudaMemcpyAsync(b.p2s_d, p2s.data(), n * sizeof(double*),
+                                  cudaMemcpyHostToDevice, b.stream), "p2s upload") ||
       !check_cuda(cudaMemcpyAsync(b.order_d, b.order.data(), n * sizeof(int),
                                   cudaMemcpyHostToDevice, b.stream), "order upload") ||
       !check_cuda(cudaMemcpyAsync(b.devs_d, devs.data(), n * sizeof(Dev),
@@ -914,9 +883,14 @@ template <int F>
 void enqueue_iteration(Batch& b, const WorkList& wl, int bps) {
   const int* occ = b.occ[F];
   auto grid = [&](int k) { return std::max(1, b.num_sms * std::min(bps, occ[k])); };
-  k_b_calc_w<F><<<grid(0), kBlock, 0, b.stream>>>(b.devs_d, b.reds_d, b.st_d, wl);
-  k_b_calc_ur<F><<<grid(1), kBlock, 0, b.stream>>>(b.devs_d, b.reds_d, b.st_d, wl);
-  k_b_calc_p<F><<<grid(2), kBlock, 0, b.stream>>>(b.devs_d, b.reds_d, b.st_d, wl);
+  k_b_pass_w<F><<<grid(0), kBlock, 0, b.stream>>>(b.devs_d, b.reds_d, b.p2s_d, b.st_d, wl);
+  k_b_pass_r<F><<<grid(1), kBlock, 0, b.stream>>>(b.devs_d, b.reds_d, b.st_d, wl);
+}
+
+template <int F>
+void enqueue_end(Batch& b, const WorkList& wl) {
+  k_b_pass_end<F><<<b.num_sms * b.occ[F][2], kBlock, 0, b.stream>>>(b.devs_d, b.reds_d, b.p2s_d,
+                                                                    b.st_d, wl);
 }
 
 // All `iters` iterations as one cooperative launch of k_b_iterations: as
@@ -937,7 +911,7 @@ void enqueue_persistent(Batch& b, const WorkList& wl, int iters, int bps) {
   cfg.numAttrs = 1;
   const long long spin_limit = 1LL << 26;
   check_cuda(cudaLaunchKernelEx(&cfg, k_b_iterations<F>, (const Dev*)b.devs_d,
-                                (const Red*)b.reds_d, b.st_d, wl, iters, b.bar_d, spin_limit),
+                                (const Red*)b.reds_d, (double* const*)b.p2s_d, b.st_d, wl, iters, b.bar_d, spin_limit),
              "batch persistent launch");
 }
 
@@ -961,9 +935,16 @@ int enqueue_iterations(Batch& b, int iters, int bps, bool compact) {
       else
         enqueue_iteration<0>(b, wl, bps);
     }
-    launched = 3 * iters;
+    launched = 2 * iters;
   }
   if (compact) {
+    if (b.arith == 2)
+      enqueue_end<2>(b, wl);
+    else if (b.arith == 1)
+      enqueue_end<1>(b, wl);
+    else
+      enqueue_end<0>(b, wl);
+    launched++;
     k_b_compact<<<1, 1024, 0, b.stream>>>(b.devs_d, b.st_d, b.plist_d, b.ustart_d,
                                           b.counts_d, wl.G);
     cudaMemcpyAsync(b.counts_h, b.counts_d, 2 * sizeof(int), cudaMemcpyDeviceToHost,
@@ -1033,7 +1014,7 @@ extern "C" int tea_gb300_batch_run(int steps, double dt, double eps, int max_ite
     b.graph_G = b.launch.supertiles_per_unit;
     b.graph_persistent = b.launch.persistent;
   }
-  per_replay = b.launch.persistent ? 2 : 3 * gi + 1;
+  per_replay = b.launch.persistent ? 3 : 2 * gi + 2;
   b.counts_h[2] = 0;
   long long n0 = tea_gb300_kernel_launches();
   cudaGraphExec_t pro = capture(b, [&]() { enqueue_prologue(b, dt, eps, max_iters); });
@@ -1200,7 +1181,7 @@ extern "C" int tea_gb300_batch_autotune(tea_gb300_batch_launch* best) {
       return -1;
     }
     enqueue_prologue(b, 0.004, 0.0, 1 << 30);
-    // three kernels per iteration, or one persistent launch per replay
+    // two kernels per iteration, or one persistent launch per replay
     for (int persistent = 0; persistent < 2; persistent++) {
       b.launch.persistent = persistent;
       const int top = persistent ? std::min(b.max_bps, b.occ_persistent[b.arith]) : b.max_bps;
@@ -1217,10 +1198,10 @@ extern "C" int tea_gb300_batch_autotune(tea_gb300_batch_launch* best) {
             b.launch = keep;
             return -1;
           }
-          count_launches(persistent ? 1 : 3 * timed);
+          count_launches(persistent ? 1 : 2 * timed);
           if (rep == 0 || ms < ms_min) ms_min = ms;
         }
-        count_launches(persistent ? 1 : 3);
+        count_launches(persistent ? 1 : 2);
         if (persistent) {
           // a launch whose barrier timed out returned early: never a candidate
           unsigned int flag = 0;

@@ -14,33 +14,8 @@ namespace tea {
 // first keeps 4 rows of loads in flight instead of one.  The arithmetic and
 // the order of the per-lane sums are those of the row-by-row form.
 
-// w = A p and the lane's share of p.w (tea_leaf_cg_cl.cl:45-69)
-template <int TH, int F, bool CG = false>
-__device__ __forceinline__ void cg_w_tile(const Dev& d, int x, int y0, bool xin,
-                                          double* acc) {
-#pragma unroll 1
-  for (int g = y0; g < y0 + TH; g += 4) {
-    const long long c0 = cidx(d, x, g);
-    double pv[4], wv[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      pv[j] = 0.0;
-      wv[j] = 0.0;
-      if (xin && g + j < d.y_max) {
-        wv[j] = smvp<F, CG>(d, d.p, c0 + j * d.S);
-        pv[j] = ldv<CG>(d.p + c0 + j * d.S);
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-      if (xin && g + j < d.y_max) d.w[c0 + j * d.S] = wv[j];
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[0] = accum<F>(acc[0], pv[j], wv[j]);
-  }
-}
-
-// cg_w_tile for the single-chunk calc_w kernel, with the fields reached
-// through restrict-qualified pointers: p and the coefficients are only
+// w = A p and the lane's share of p.w (tea_leaf_cg_cl.cl:45-69), with the fields
+// reached through restrict-qualified pointers: p and the coefficients are only
 // read and w only written, so the compiler may issue a group's loads before
 // the previous group's stores and keep more loads in flight.  Same
 // arithmetic and per-lane summation order; with 4 blocks per SM (64
@@ -90,67 +65,11 @@ __device__ __forceinline__ void ur_values(double alpha, double& u, double p,
   }
 }
 
-// u += alpha p, r -= alpha w, z = M^-1 r and the lane's share of r.z (and
-// of r.r when NV == 2; no sum when NV == 0), tea_leaf_cg_cl.cl:73-137.
-// With SD it also starts PPCG's inner steps, sd = M^-1 r / theta
-// (tea_leaf_ppcg_cl.cl:4-60), from the z it has just formed: the same
-// values tea_leaf_ppcg_solve_init_sd computes from the stored r.
-template <int TH, int F, int NV, bool CG = false, bool SD = false>
-__device__ __forceinline__ void cg_ur_tile(const Dev& d, int x, int y0, bool xin,
-                                           double* acc, double alpha,
-                                           const DivConst& theta = DivConst{}) {
-#pragma unroll 1
-  for (int g = y0; g < y0 + TH; g += 4) {
-    const long long c0 = cidx(d, x, g);
-    bool in[4];
-    double uv[4], pv[4], rv[4], wv[4], mv[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      in[j] = xin && g + j < d.y_max;
-      uv[j] = pv[j] = rv[j] = wv[j] = mv[j] = 0.0;
-      if (in[j]) {
-        const long long c = c0 + j * d.S;
-        uv[j] = ldv<CG>(d.u + c);
-        pv[j] = ldv<CG>(d.p + c);
-        rv[j] = ldv<CG>(d.r + c);
-        wv[j] = ldv<CG>(d.w + c);
-        if (d.prec == PREC_JAC_DIAG) mv[j] = d.Mi[c];
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      if (in[j]) {
-        ur_values<F>(alpha, uv[j], pv[j], rv[j], wv[j]);
-        d.u[c0 + j * d.S] = uv[j];
-        d.r[c0 + j * d.S] = rv[j];
-      }
-    }
-    double zv[4] = {0.0, 0.0, 0.0, 0.0};
-    if (d.prec == PREC_JAC_BLOCK) {
-      // one 4-row strip of the block-Jacobi solve (strips start at rows
-      // that are multiples of 4)
-      if (in[0]) strip_solve<F>(d, c0, strip_rows(d, g), rv, zv);
-    } else if (d.prec == PREC_JAC_DIAG) {
-#pragma unroll
-      for (int j = 0; j < 4; j++) zv[j] = rv[j] * mv[j];
-    }
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      double av = 0.0, bv = 0.0;
-      if (in[j]) {
-        if (d.prec != PREC_NONE) d.z[c0 + j * d.S] = zv[j];
-        if (SD) d.sd[c0 + j * d.S] = emu_ddiv(d.prec != PREC_NONE ? zv[j] : rv[j], theta);
-        av = rv[j];
-        bv = d.prec != PREC_NONE ? zv[j] : rv[j];
-      }
-      if (NV > 0) acc[0] = accum<F>(acc[0], av, bv);
-      if (NV > 1) acc[NV - 1] = accum<F>(acc[NV - 1], av, av);
-    }
-  }
-}
-
-// cg_ur_tile for the single-chunk kernels (CG calc_ur, PPCG's calc_ur +
-// init_sd), with the fields reached through restrict-qualified pointers and
+// u += alpha p, r -= alpha w, z = M^-1 r and the lane's share of r.z (no sum
+// when NV == 0), tea_leaf_cg_cl.cl:73-137.  With SD it also starts PPCG's inner
+// steps, sd = M^-1 r / theta (tea_leaf_ppcg_cl.cl:4-60), from the z it has just
+// formed: the same values tea_leaf_ppcg_solve_init_sd computes from the stored
+// r.  The fields are reached through restrict-qualified pointers and
 // the strip coefficients loaded with u, p, r and w, before the stores of u
 // and r, so that more loads are in flight.  The strip solve reads exactly
 // the rows strip_solve reads (a strip may end in the halo row).  Same
@@ -181,7 +100,6 @@ __device__ __forceinline__ void cg_ur_tile_r(const Dev& d, int x, int y0, bool x
         bv = prec ? zv[j] : rv[j];
       }
       if (NV > 0) acc[0] = accum<F>(acc[0], av, bv);
-      if (NV > 1) acc[NV - 1] = accum<F>(acc[NV - 1], av, av);
     }
   };
   if (d.prec == PREC_JAC_BLOCK) {
@@ -257,7 +175,7 @@ __device__ __forceinline__ void cg_ur_tile_r(const Dev& d, int x, int y0, bool x
 
 // p = z + beta p, or r + beta p without a preconditioner
 // (tea_leaf_cg_cl.cl:141-160)
-template <int TH, int F, bool CG = false>
+template <int TH, int F>
 __device__ __forceinline__ void cg_p_tile(const Dev& d, int x, int y0, bool xin,
                                           double beta) {
   if (!xin) return;
@@ -270,14 +188,189 @@ __device__ __forceinline__ void cg_p_tile(const Dev& d, int x, int y0, bool xin,
     for (int j = 0; j < 4; j++) {
       sv[j] = pv[j] = 0.0;
       if (g + j < d.y_max) {
-        sv[j] = ldv<CG>(src + c0 + j * d.S);
-        pv[j] = ldv<CG>(d.p + c0 + j * d.S);
+        sv[j] = src[c0 + j * d.S];
+        pv[j] = d.p[c0 + j * d.S];
       }
     }
 #pragma unroll
     for (int j = 0; j < 4; j++)
       if (g + j < d.y_max)
         d.p[c0 + j * d.S] = F ? __fma_rn(beta, pv[j], sv[j]) : sv[j] + beta * pv[j];
+  }
+}
+
+// ---- the two-pass CG iteration (tea_cg_loop.cu, tea_batch.cu) ----
+
+template <int F>
+__device__ __forceinline__ double p_next(double beta, double p, double z) {
+  return F ? __fma_rn(beta, p, z) : z + beta * p;
+}
+
+// Pass A on one tile: lane column x, rows y0 .. y0+TH-1.  p' of the rows
+// above and below and of the columns either side is formed here too (the
+// two columns by lanes 0-7, one multiply-add for four rows), so no pass and
+// no grid barrier separates p' from w.  Halo cells keep the p they were given
+// (they are read from d.p whichever buffer is current).  On the first
+// iteration of a launch p is current already (it stays in pin, or with COPY
+// goes to pout as it is) and u has nothing pending.
+// p and z are written by other SMs during the launch: they are read through
+// L2.  All loads of four rows are issued before anything waits for one; rows
+// past the interior are clamped to the halo row above it and lanes past the
+// last column read the row's padding, and neither is used.
+template <int TH, int F, bool COPY = false>
+__device__ __forceinline__ double loop_w_tile(const Dev& d, const double* __restrict__ pin,
+                                              double* __restrict__ pout,
+                                              const double* __restrict__ zsrc, int x, int y0,
+                                              double alpha, double beta, bool first) {
+  const int lane = threadIdx.x & 31;
+  const double* __restrict__ hal = d.p;
+  const double* __restrict__ kx = d.Kx;
+  const double* __restrict__ ky = d.Ky;
+  const double* __restrict__ dg = d.diag;
+  double* __restrict__ u = d.u;
+  double* __restrict__ w = d.w;
+  const long long S = d.S;
+  const long long c0 = cidx(d, x, y0);
+  const bool xin = x < d.x_max;
+  const int rows = min(TH, d.y_max - y0);
+  const bool top = y0 + rows == d.y_max;  // row `rows` is halo
+  const double* __restrict__ pcol = xin ? pin : hal;
+  // p' from the old p and z; halo cells keep p
+  auto fresh = [&](double po, double zv, bool in) {
+    return first || !in ? po : p_next<F>(beta, po, zv);
+  };
+  double acc = 0.0;
+  double pm = 0.0, pc = 0.0, pco = 0.0;  // p' of rows g-1 and g, old p of row g
+#pragma unroll 1
+  for (int g = 0; g < rows; g += 4) {
+    const bool bottom = TH == 4 || g == 0;
+    double po[6], zv[6], uv[4], kyv[5], kxc[4], kxe[4], dv[4];
+    const int er = min(g + (lane >> 1), rows - 1);
+    const int xe = (lane & 1) ? x - lane + 32 : x - lane - 1;
+    const bool ein = xe >= 0 && xe < d.x_max;
+    double ep = 0.0, ez = 0.0;
+#pragma unroll
+    for (int j = 0; j < 6; j++) {
+      po[j] = zv[j] = 0.0;
+      if (j < 2 && !bottom) continue;  // carried from the group below
+      const int row = min(g + j - 1, rows);
+      const bool rin = (row >= 0 || y0 > 0) && !(row == rows && top);
+      const long long c = c0 + row * S;
+      po[j] = __ldcg((rin ? pcol : hal) + c);
+      zv[j] = __ldcg(zsrc + c);
+    }
+    if (lane < 8) {
+      const long long c = cidx(d, xe, y0 + er);
+      ep = __ldcg((ein ? pin : hal) + c);
+      ez = __ldcg(zsrc + c);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const long long c = c0 + min(g + j, rows - 1) * S;
+      uv[j] = u[c];
+      kyv[j] = __ldg(ky + c);
+      kxc[j] = __ldg(kx + c);
+      kxe[j] = __ldg(kx + c + 1);
+      dv[j] = __ldg(dg + c);
+    }
+    kyv[4] = __ldg(ky + c0 + min(g + 4, rows) * S);
+    double pv[6];
+    pv[0] = pm;
+    pv[1] = pc;
+    if (!bottom) po[1] = pco;
+#pragma unroll
+    for (int j = 0; j < 6; j++) {
+      if (j < 2 && !bottom) continue;
+      const int row = min(g + j - 1, rows);
+      const bool rin = (row >= 0 || y0 > 0) && !(row == rows && top);
+      pv[j] = fresh(po[j], zv[j], rin && xin);
+    }
+    const double ev = fresh(ep, ez, ein);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const long long c = c0 + (g + j) * S;
+      const bool own = xin && g + j < rows;
+      if (own && !first)
+        u[c] = F ? __fma_rn(alpha, po[j + 1], uv[j]) : uv[j] + alpha * po[j + 1];
+      double pe = __shfl_down_sync(0xffffffffu, pv[j + 1], 1);
+      double pw = __shfl_up_sync(0xffffffffu, pv[j + 1], 1);
+      const double e = __shfl_sync(0xffffffffu, ev, 2 * j + 1);
+      const double wst = __shfl_sync(0xffffffffu, ev, 2 * j);
+      if (lane == 31) pe = e;
+      if (lane == 0) pw = wst;
+      const double kyn = j < 3 && g + j + 1 < rows ? kyv[j + 1] : kyv[4];
+      const double wv = smvp_v<F>(dv[j], kyn, kyv[j], kxe[j], kxc[j], pv[j + 1], pv[j + 2], pv[j],
+                                  pe, pw);
+      if (own) {
+        w[c] = wv;
+        if (COPY || !first) pout[c] = pv[j + 1];
+      }
+      acc = accum<F>(acc, own ? pv[j + 1] : 0.0, own ? wv : 0.0);
+    }
+    pm = pv[4];
+    pc = pv[5];
+    pco = po[5];
+  }
+  return acc;
+}
+
+// Pass B on one tile: r -= alpha w, z = M^-1 r and the lane's share of r.z
+// (cg_ur_tile_r without u, which pass A updates).  A lane reads back only
+// the r and w that it wrote itself.
+template <int TH, int F, int NV = 1>
+__device__ __forceinline__ void loop_r_tile(const Dev& d, int x, int y0, double alpha,
+                                            double* acc) {
+  double* __restrict__ r = d.r;
+  const double* __restrict__ w = d.w;
+  double* __restrict__ z = d.z;
+  const long long S = d.S;
+  if (x >= d.x_max) return;
+  const int rows = min(TH, d.y_max - y0);
+#pragma unroll 1
+  for (int g = 0; g < rows; g += 4) {
+    const long long c0 = cidx(d, x, y0 + g);
+    double rv[4], wv[4], mv[4], zv[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const long long c = c0 + min(j, rows - 1 - g) * S;
+      wv[j] = w[c];
+      rv[j] = r[c];
+      mv[j] = d.prec == PREC_JAC_DIAG ? __ldg(d.Mi + c) : 0.0;
+    }
+    if (d.prec == PREC_JAC_BLOCK) {
+      const int upper = strip_rows(d, y0 + g);
+      double bl[4], kl[4], cl[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const long long c = c0 + min(j, upper - 1) * S;
+        bl[j] = __ldg(d.bfp + c);
+        kl[j] = __ldg(d.Ky + c);
+        cl[j] = __ldg(d.cp + c);
+      }
+      const double d0 = F ? 0.0 : __ldg(d.diag + c0);
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        rv[j] = g + j >= rows ? 0.0 : F ? __fma_rn(-alpha, wv[j], rv[j]) : rv[j] - alpha * wv[j];
+      if (upper == 4)
+        strip_solve_v<F, false, true>(4, rv, bl, kl, cl, d0, zv);
+      else
+        strip_solve_v<F, false>(upper, rv, bl, kl, cl, d0, zv);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        rv[j] = F ? __fma_rn(-alpha, wv[j], rv[j]) : rv[j] - alpha * wv[j];
+        zv[j] = d.prec == PREC_JAC_DIAG ? mul_e<true>(rv[j], mv[j]) : rv[j];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (g + j < rows) {
+        r[c0 + j * S] = rv[j];
+        if (d.prec != PREC_NONE) z[c0 + j * S] = zv[j];
+        acc[0] = accum<F>(acc[0], rv[j], zv[j]);
+        if (NV > 1) acc[NV - 1] = accum<F>(acc[NV - 1], rv[j], rv[j]);
+      }
+    }
   }
 }
 

@@ -57,179 +57,6 @@ __device__ __forceinline__ double square_limit(double t) {
   return sqrt(x) >= t && sqrt(__longlong_as_double(__double_as_longlong(x) - 1)) < t ? x : -1.0;
 }
 
-template <int F>
-__device__ __forceinline__ double p_next(double beta, double p, double z) {
-  return F ? __fma_rn(beta, p, z) : z + beta * p;
-}
-
-// Pass A on one tile: lane column x, rows y0 .. y0+TH-1.  p' of the rows
-// above and below and of the columns either side is formed here too (the
-// two columns by lanes 0-7, one multiply-add for four rows), so no pass and
-// no grid barrier separates p' from w.  Halo cells keep the p they were given
-// (they are read from d.p whichever buffer is current).  On the first
-// iteration of a launch p is current already (it stays in pin, or with COPY
-// goes to pout as it is) and u has nothing pending.
-// p and z are written by other SMs during the launch: they are read through
-// L2.  All loads of four rows are issued before anything waits for one; rows
-// past the interior are clamped to the halo row above it and lanes past the
-// last column read the row's padding, and neither is used.
-template <int TH, int F, bool COPY = false>
-__device__ __forceinline__ double loop_w_tile(const Dev& d, const double* __restrict__ pin,
-                                              double* __restrict__ pout,
-                                              const double* __restrict__ zsrc, int x, int y0,
-                                              double alpha, double beta, bool first) {
-  const int lane = threadIdx.x & 31;
-  const double* __restrict__ hal = d.p;
-  const double* __restrict__ kx = d.Kx;
-  const double* __restrict__ ky = d.Ky;
-  const double* __restrict__ dg = d.diag;
-  double* __restrict__ u = d.u;
-  double* __restrict__ w = d.w;
-  const long long S = d.S;
-  const long long c0 = cidx(d, x, y0);
-  const bool xin = x < d.x_max;
-  const int rows = min(TH, d.y_max - y0);
-  const bool top = y0 + rows == d.y_max;  // row `rows` is halo
-  const double* __restrict__ pcol = xin ? pin : hal;
-  // p' from the old p and z; halo cells keep p
-  auto fresh = [&](double po, double zv, bool in) {
-    return first || !in ? po : p_next<F>(beta, po, zv);
-  };
-  double acc = 0.0;
-  double pm = 0.0, pc = 0.0, pco = 0.0;  // p' of rows g-1 and g, old p of row g
-#pragma unroll 1
-  for (int g = 0; g < rows; g += 4) {
-    const bool bottom = TH == 4 || g == 0;
-    double po[6], zv[6], uv[4], kyv[5], kxc[4], kxe[4], dv[4];
-    const int er = min(g + (lane >> 1), rows - 1);
-    const int xe = (lane & 1) ? x - lane + 32 : x - lane - 1;
-    const bool ein = xe >= 0 && xe < d.x_max;
-    double ep = 0.0, ez = 0.0;
-#pragma unroll
-    for (int j = 0; j < 6; j++) {
-      po[j] = zv[j] = 0.0;
-      if (j < 2 && !bottom) continue;  // carried from the group below
-      const int row = min(g + j - 1, rows);
-      const bool rin = (row >= 0 || y0 > 0) && !(row == rows && top);
-      const long long c = c0 + row * S;
-      po[j] = __ldcg((rin ? pcol : hal) + c);
-      zv[j] = __ldcg(zsrc + c);
-    }
-    if (lane < 8) {
-      const long long c = cidx(d, xe, y0 + er);
-      ep = __ldcg((ein ? pin : hal) + c);
-      ez = __ldcg(zsrc + c);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const long long c = c0 + min(g + j, rows - 1) * S;
-      uv[j] = u[c];
-      kyv[j] = __ldg(ky + c);
-      kxc[j] = __ldg(kx + c);
-      kxe[j] = __ldg(kx + c + 1);
-      dv[j] = __ldg(dg + c);
-    }
-    kyv[4] = __ldg(ky + c0 + min(g + 4, rows) * S);
-    double pv[6];
-    pv[0] = pm;
-    pv[1] = pc;
-    if (!bottom) po[1] = pco;
-#pragma unroll
-    for (int j = 0; j < 6; j++) {
-      if (j < 2 && !bottom) continue;
-      const int row = min(g + j - 1, rows);
-      const bool rin = (row >= 0 || y0 > 0) && !(row == rows && top);
-      pv[j] = fresh(po[j], zv[j], rin && xin);
-    }
-    const double ev = fresh(ep, ez, ein);
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const long long c = c0 + (g + j) * S;
-      const bool own = xin && g + j < rows;
-      if (own && !first)
-        u[c] = F ? __fma_rn(alpha, po[j + 1], uv[j]) : uv[j] + alpha * po[j + 1];
-      double pe = __shfl_down_sync(0xffffffffu, pv[j + 1], 1);
-      double pw = __shfl_up_sync(0xffffffffu, pv[j + 1], 1);
-      const double e = __shfl_sync(0xffffffffu, ev, 2 * j + 1);
-      const double wst = __shfl_sync(0xffffffffu, ev, 2 * j);
-      if (lane == 31) pe = e;
-      if (lane == 0) pw = wst;
-      const double kyn = j < 3 && g + j + 1 < rows ? kyv[j + 1] : kyv[4];
-      const double wv = smvp_v<F>(dv[j], kyn, kyv[j], kxe[j], kxc[j], pv[j + 1], pv[j + 2], pv[j],
-                                  pe, pw);
-      if (own) {
-        w[c] = wv;
-        if (COPY || !first) pout[c] = pv[j + 1];
-      }
-      acc = accum<F>(acc, own ? pv[j + 1] : 0.0, own ? wv : 0.0);
-    }
-    pm = pv[4];
-    pc = pv[5];
-    pco = po[5];
-  }
-  return acc;
-}
-
-// Pass B on one tile: r -= alpha w, z = M^-1 r and the lane's share of r.z
-// (cg_ur_tile_r without u, which pass A updates).  A lane reads back only
-// the r and w that it wrote itself.
-template <int TH, int F, int NV = 1>
-__device__ __forceinline__ void loop_r_tile(const Dev& d, int x, int y0, double alpha,
-                                            double* acc) {
-  double* __restrict__ r = d.r;
-  const double* __restrict__ w = d.w;
-  double* __restrict__ z = d.z;
-  const long long S = d.S;
-  if (x >= d.x_max) return;
-  const int rows = min(TH, d.y_max - y0);
-#pragma unroll 1
-  for (int g = 0; g < rows; g += 4) {
-    const long long c0 = cidx(d, x, y0 + g);
-    double rv[4], wv[4], mv[4], zv[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const long long c = c0 + min(j, rows - 1 - g) * S;
-      wv[j] = w[c];
-      rv[j] = r[c];
-      mv[j] = d.prec == PREC_JAC_DIAG ? __ldg(d.Mi + c) : 0.0;
-    }
-    if (d.prec == PREC_JAC_BLOCK) {
-      const int upper = strip_rows(d, y0 + g);
-      double bl[4], kl[4], cl[4];
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const long long c = c0 + min(j, upper - 1) * S;
-        bl[j] = __ldg(d.bfp + c);
-        kl[j] = __ldg(d.Ky + c);
-        cl[j] = __ldg(d.cp + c);
-      }
-      const double d0 = F ? 0.0 : __ldg(d.diag + c0);
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        rv[j] = g + j >= rows ? 0.0 : F ? __fma_rn(-alpha, wv[j], rv[j]) : rv[j] - alpha * wv[j];
-      if (upper == 4)
-        strip_solve_v<F, false, true>(4, rv, bl, kl, cl, d0, zv);
-      else
-        strip_solve_v<F, false>(upper, rv, bl, kl, cl, d0, zv);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        rv[j] = F ? __fma_rn(-alpha, wv[j], rv[j]) : rv[j] - alpha * wv[j];
-        zv[j] = d.prec == PREC_JAC_DIAG ? mul_e<true>(rv[j], mv[j]) : rv[j];
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      if (g + j < rows) {
-        r[c0 + j * S] = rv[j];
-        if (d.prec != PREC_NONE) z[c0 + j * S] = zv[j];
-        acc[0] = accum<F>(acc[0], rv[j], zv[j]);
-        if (NV > 1) acc[NV - 1] = accum<F>(acc[NV - 1], rv[j], rv[j]);
-      }
-    }
-  }
-}
-
 // Runs body(x, y0) -> lane sum over the block's supertiles and stores the
 // supertile partials.  A warp writes its lane sums to shared memory and
 // whole warps then sum four tiles each (bfly4) and four supertiles each
