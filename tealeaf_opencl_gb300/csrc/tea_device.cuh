@@ -302,41 +302,30 @@ __device__ __forceinline__ void block_final_sum(const double* partials,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll 1
   for (int v = 0; v < NV; v++) {
+    const double* p = partials + v * stride;
     double a = 0.0;
-    for (int k = threadIdx.x; k < ns; k += kBlock)
-      a = a + __ldcg(partials + v * stride + k);
+    int k = threadIdx.x;
+    for (; k + 3 * kBlock < ns; k += 4 * kBlock) {  // four loads in flight
+      const double b0 = __ldcg(p + k), b1 = __ldcg(p + k + kBlock);
+      const double b2 = __ldcg(p + k + 2 * kBlock), b3 = __ldcg(p + k + 3 * kBlock);
+      a = a + b0;
+      a = a + b1;
+      a = a + b2;
+      a = a + b3;
+    }
+    for (; k < ns; k += kBlock) a = a + __ldcg(p + k);
     a = bfly(a);
     if (lane == 0) sh[warp] = a;
     __syncthreads();
     if (warp == 0) {
       double t = lane < 8 ? sh[lane] : 0.0;
-      t = bfly(t);
+      t = t + 0.0;  // the stages that add the zeros of lanes 8-31
+#pragma unroll
+      for (int off = 4; off >= 1; off >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, off);
       if (lane == 0) result[v] = t;
     }
     __syncthreads();
   }
-}
-
-// The same sum as block_final_sum for one value, handed to every thread of
-// the block instead of stored (used by persistent kernels, in which every
-// block forms the reduced value itself).  sh holds at least 9 doubles.
-__device__ __forceinline__ double block_final_value(const double* partials, int ns,
-                                                    double* sh) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double a = 0.0;
-  for (int k = threadIdx.x; k < ns; k += kBlock) a = a + __ldcg(partials + k);
-  a = bfly(a);
-  if (lane == 0) sh[warp] = a;
-  __syncthreads();
-  if (warp == 0) {
-    double t = lane < 8 ? sh[lane] : 0.0;
-    t = bfly(t);
-    if (lane == 0) sh[8] = t;
-  }
-  __syncthreads();
-  const double v = sh[8];
-  __syncthreads();
-  return v;
 }
 
 // Barrier across every block of a cooperative launch (all blocks resident).
@@ -387,9 +376,10 @@ template <int NV>
 __device__ __forceinline__ bool finish_reduction(const Red& red, int ns,
                                                  double* sh) {
   __shared__ unsigned int is_last;
-  __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
+    // the barrier above orders the block's partials before this fence
+    __threadfence();
     const unsigned int t = atomicAdd(red.counter, 1u);
     is_last = (t == gridDim.x - 1) ? 1u : 0u;
   }
@@ -466,7 +456,7 @@ __device__ __forceinline__ void supertile_partials4(const Red& red, const int* s
 // Walks the block's supertiles (s = blockIdx.x + j*gridDim.x);
 // body(x, y0, xin, acc) processes the TH rows of one lane's column x
 // starting at interior row y0 and adds its contributions row by row into
-// acc[0..NV).  With P = 4 the sums of four supertiles share their
+// acc[0..NV).  With P = 4 the sums of up to four supertiles share their
 // butterflies (bfly4, supertile_partials4); with P = 1 every supertile is
 // summed on its own, which needs fewer registers (the FP32 kernels of the
 // mixed solve, held to 32 registers for full occupancy, are faster so).
@@ -507,6 +497,46 @@ __device__ __forceinline__ bool tile_driver(const Dev& d, const Red& red,
     }
     return false;
   }
+  if constexpr (TH == 4) {
+  // 4-row tiles, of which a block often has fewer than four: lane sums go
+  // through shared memory and whole warps sum four tiles each, 12 FP64 warp
+  // instructions per supertile where each warp summing its own four takes 48
+  // for the four however few there are (calc_w at 960^2 22.3 -> 20.1 us, at
+  // 512^2 14.0 -> 11.9).
+  __shared__ double lanes[NVV * 4 * kBlock];
+  for (int s0 = blockIdx.x; s0 < d.ns; s0 += 4 * gridDim.x) {
+    const int nr = min(4, (d.ns - 1 - s0) / (int)gridDim.x + 1);
+#pragma unroll 1
+    for (int k = 0; k < nr; k++) {
+      double acc[NVV];
+#pragma unroll
+      for (int v = 0; v < NVV; v++) acc[v] = 0.0;
+      const int s = s0 + k * gridDim.x;
+      const int sy = s / d.nsx, sx = s - sy * d.nsx;
+      const int tx = sx * kTilesPerSuper + warp;
+      if (tx < d.ntx) {
+        const int x = tx * kTileW + lane;
+        body(x, sy * TH, x < d.x_max, acc);
+      }
+#pragma unroll
+      for (int v = 0; v < NVV; v++) lanes[(v * 4 + k) * kBlock + threadIdx.x] = acc[v];
+    }
+    __syncthreads();
+    for (int job = warp; job < NVV * 2 * nr; job += kBlock / 32) {
+      const int v = job / (2 * nr), w = job - v * 2 * nr;  // tiles 4w .. 4w+3 of value v
+      const double* a = lanes + v * 4 * kBlock + w * 128 + lane;
+      const double t = bfly4(a[0], a[32], a[64], a[96]);
+      if ((lane & 7) == 0) sh[v * 32 + w * 4 + bfly4_slot(lane)] = t;
+    }
+    int s_k[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) s_k[k] = s0 + k * gridDim.x;
+    supertile_partials4<NVV>(red, s_k, d.ns, sh);
+  }
+  return finish_reduction<NVV>(red, d.ns, sh);
+  }
+  // 16-row tiles: each warp keeps the lane sums of its four in registers
+  // (through shared memory calc_ur at 4096^2 took 226 us against 217)
   for (int s0 = blockIdx.x; s0 < d.ns; s0 += 4 * gridDim.x) {
     double tiles[4][NVV];
     int s_k[4];
