@@ -294,11 +294,13 @@ __device__ __forceinline__ void supertile_partial(const Red& red, int s,
 }
 
 // Step 4 of the summation order, by one whole block: the ns partials of
-// each of the NV sums (NV arrays, `stride` apart) reduced into result[v].
+// each of the NV sums (NV arrays, `stride` apart) reduced into result[v], and
+// its bit pattern into host[v] if there is one.
 template <int NV>
 __device__ __forceinline__ void block_final_sum(const double* partials,
                                                 long long stride, int ns,
-                                                double* result, double* sh) {
+                                                double* result, double* sh,
+                                                unsigned long long* host = nullptr) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll 1
   for (int v = 0; v < NV; v++) {
@@ -322,7 +324,11 @@ __device__ __forceinline__ void block_final_sum(const double* partials,
       t = t + 0.0;  // the stages that add the zeros of lanes 8-31
 #pragma unroll
       for (int off = 4; off >= 1; off >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, off);
-      if (lane == 0) result[v] = t;
+      if (lane == 0) {
+        result[v] = t;
+        if (host)
+          *(volatile unsigned long long*)(host + v) = (unsigned long long)__double_as_longlong(t);
+      }
     }
     __syncthreads();
   }
@@ -386,18 +392,8 @@ __device__ __forceinline__ bool finish_reduction(const Red& red, int ns,
   __syncthreads();
   if (!is_last) return false;
   __threadfence();
-  block_final_sum<NV>(red.partials, red.stride, ns, red.result, sh);
-  if (threadIdx.x == 0) {
-    *red.counter = 0u;
-    if (red.host) {
-      // thread 0 wrote red.result itself (block_final_sum)
-#pragma unroll
-      for (int v = 0; v < NV; v++)
-        red.host[v] = (unsigned long long)__double_as_longlong(red.result[v]);
-      __threadfence_system();
-      *(volatile unsigned long long*)(red.host + 8) = 1ull;
-    }
-  }
+  if (threadIdx.x == 0) *red.counter = 0u;
+  block_final_sum<NV>(red.partials, red.stride, ns, red.result, sh, red.host);
   return true;
 }
 

@@ -52,8 +52,8 @@ struct Red {
   double* result;       // [nvals]
   // Optional copy of the result in mapped pinned host memory for a caller
   // waiting on the host: the bit patterns of the result values at
-  // host[0..nvals), then a nonzero word at host[8] once they are visible
-  // (see tea_abi.cu, fetch).
+  // host[0..nvals), each written by one 8-byte store over a pattern that no
+  // sum has (see tea_abi.cu, fetch).
   unsigned long long* host = nullptr;
 };
 
@@ -108,7 +108,7 @@ struct Chunk {
   unsigned int* red_counter = nullptr;
   double* red_result = nullptr;
   double* host_result = nullptr;  // pinned, 8 doubles
-  unsigned long long* host_map = nullptr;      // mapped pinned: 8 results, ready word
+  unsigned long long* host_map = nullptr;      // mapped pinned: 8 results
   unsigned long long* host_map_dev = nullptr;  // its device address
   bool red_to_host = false;        // next c.red() copies its result to host_map
   // coefficients kept on the host (passed to kernels by value) and on device
