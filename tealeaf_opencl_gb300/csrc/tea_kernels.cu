@@ -57,6 +57,13 @@ Dev rows4_tiling(Dev d) {
 
 static Dev dev4(const Chunk& c) { return rows4_tiling(c.dev()); }
 
+// Blocks per SM (the register budget) of the one-pass point-preconditioner
+// steps.  Four blocks of 64 registers keep more loads in flight where the
+// passes stream (3000x2500: PPCG step 117.5 -> 112.8 us, Chebyshev 138.9 ->
+// 129.8); three of 80 are quicker over few tiles (500^2: 10.9 against 11.7,
+// 11.3 against 12.0).  At 1111x901, 7.4 supertiles per SM, they are level.
+static bool point_blocks4(const Chunk& c) { return dev4(c).ns > 8 * c.num_sms; }
+
 
 
 template <class... KArgs, class... Args>
@@ -563,8 +570,8 @@ __global__ void __launch_bounds__(kBlock, 3)
 // One pass in place of calc_p and calc_u; 7 FP64 instructions per cell with the
 // products on the integer pipes (bit-identical), 10 with all of them on the
 // FP64 pipe.
-template <int F>
-__global__ void __launch_bounds__(kBlock, 3)
+template <int F, int MB>
+__global__ void __launch_bounds__(kBlock, MB)
     k_cheby_calc_pu_point(Dev d, Red red, double alpha, double beta, double* un_) {
   tile_driver<4, 0>(d, red, [&](int x, int y0, bool xin, double* acc) {
     if (!xin) return;
@@ -915,8 +922,8 @@ __global__ void __launch_bounds__(kBlock, 3)
 // calc_sd; the products run on the integer pipes (bit-identical).  Rows past
 // the interior are clamped to the halo row, so every load is issued before the
 // first use; the values of such rows are not stored.
-template <int F>
-__global__ void __launch_bounds__(kBlock, 3)
+template <int F, int MB>
+__global__ void __launch_bounds__(kBlock, MB)
     k_ppcg_step_point(Dev d, Red red, double alpha, double beta, const ResState* st,
                       const double* sdi_, double* sdo_) {
   if (st && *(volatile const int*)&st->stop) return;
@@ -1214,11 +1221,14 @@ void launch_cheby_calc_pu(Chunk& c, double alpha, double beta, double* un) {
     const Dev d4 = dev4(c);
     const char* name = "tea_leaf_cheby_solve_calc_p_u";
     if (c.arith == 2)
-      launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<2>, d4, c.red(), alpha, beta, un);
+      point_blocks4(c) ? launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<2, 4>, d4, c.red(), alpha, beta, un)
+                       : launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<2, 3>, d4, c.red(), alpha, beta, un);
     else if (c.arith == 1)
-      launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<1>, d4, c.red(), alpha, beta, un);
+      point_blocks4(c) ? launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<1, 4>, d4, c.red(), alpha, beta, un)
+                       : launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<1, 3>, d4, c.red(), alpha, beta, un);
     else
-      launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<0>, d4, c.red(), alpha, beta, un);
+      point_blocks4(c) ? launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<0, 4>, d4, c.red(), alpha, beta, un)
+                       : launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<0, 3>, d4, c.red(), alpha, beta, un);
     return;
   }
   TH_DISPATCH(c, "tea_leaf_cheby_solve_calc_p_u", k_cheby_calc_pu_block, c.dev(), c.red(),
@@ -1240,11 +1250,20 @@ void launch_ppcg_step(Chunk& c, double alpha, double beta, const double* sdi, do
   const ResState* st = nullptr;
   if (c.prec != PREC_JAC_BLOCK) {
     if (c.arith == 2)
-      launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<2>, d4, c.red(), alpha, beta, st, sdi, sdo);
+      point_blocks4(c) ? launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<2, 4>, d4, c.red(), alpha, beta, st,
+                                        sdi, sdo)
+                       : launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<2, 3>, d4, c.red(), alpha, beta, st,
+                                        sdi, sdo);
     else if (c.arith == 1)
-      launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<1>, d4, c.red(), alpha, beta, st, sdi, sdo);
+      point_blocks4(c) ? launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<1, 4>, d4, c.red(), alpha, beta, st,
+                                        sdi, sdo)
+                       : launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<1, 3>, d4, c.red(), alpha, beta, st,
+                                        sdi, sdo);
     else
-      launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<0>, d4, c.red(), alpha, beta, st, sdi, sdo);
+      point_blocks4(c) ? launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<0, 4>, d4, c.red(), alpha, beta, st,
+                                        sdi, sdo)
+                       : launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<0, 3>, d4, c.red(), alpha, beta, st,
+                                        sdi, sdo);
     return;
   }
   if (c.arith == 2)
@@ -1505,7 +1524,9 @@ static void enqueue_ppcg_iterations_t(Chunk& c, int iters) {
   const bool blk = c.prec == PREC_JAC_BLOCK;
   const int gs = blk ? tile_grid(c, k_ppcg_calc_sd_block<F>, sd_blocks(d4))
                      : tile_grid(c, k_ppcg_sd<4, F>, d4.ns);
-  auto* const step = blk ? k_ppcg_step<F> : k_ppcg_step_point<F>;
+  auto* const step = blk              ? k_ppcg_step<F>
+                     : point_blocks4(c) ? k_ppcg_step_point<F, 4>
+                                        : k_ppcg_step_point<F, 3>;
   const int gst = tile_grid(c, step, d4.ns);
   // inner steps two at a time in one pass each, the first writing sd to the
   // second buffer and the second back, so each outer iteration ends with sd
