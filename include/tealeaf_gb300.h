@@ -538,6 +538,10 @@ int tea_gb300_adjoint_forward(const double* density, const double* energy0,
                               const tea_gb300_adjoint_config* config,
                               double* loss, double* u_final,
                               tea_gb300_adjoint_stats* stats);
+/* A number of the forward pass that tea_gb300_adjoint_backward would use, new
+ * for every kept pass of the process; 0 if there is none (no forward call with
+ * u_obs since the object was made or since the last backward call). */
+long long tea_gb300_adjoint_pass(void);
 /* d loss / d log(density) of the last forward pass into grad_log_density. */
 int tea_gb300_adjoint_backward(double* grad_log_density,
                                tea_gb300_adjoint_stats* stats);

@@ -21,7 +21,7 @@ class TimeSteppedLoss(torch.autograd.Function):
         u_obs = u_obs.contiguous()
         torch.cuda.synchronize()
         loss, _ = adj.forward(density, energy0, u_obs, cfg=cfg)
-        ctx.adj, ctx.cfg = adj, cfg
+        ctx.adj, ctx.cfg, ctx.kept = adj, cfg, adj.kept_pass()
         ctx.save_for_backward(density, energy0, u_obs)
         return torch.tensor(loss, dtype=torch.float64, device=log_density.device)
 
@@ -29,9 +29,14 @@ class TimeSteppedLoss(torch.autograd.Function):
     def backward(ctx, grad_loss):
         density, energy0, u_obs = ctx.saved_tensors
         adj, cfg = ctx.adj, ctx.cfg
-        # another forward call may have replaced the kept pass: run it again
-        adj.forward(density, energy0, u_obs, cfg=cfg)
+        # the library keeps one pass: if another forward call has replaced it,
+        # or a backward call consumed it, run it again
+        if ctx.kept == 0 or adj.kept_pass() != ctx.kept:
+            torch.cuda.synchronize()
+            adj.forward(density, energy0, u_obs, cfg=cfg)
         grad = torch.empty_like(density)
+        # the library writes grad on its own stream
+        torch.cuda.current_stream(density.device).synchronize()
         adj.backward(grad)
         return grad * grad_loss, None, None, None, None
 

@@ -133,6 +133,7 @@ struct Adjoint {
   cudaGraphExec_t graph = nullptr;
   // the last forward pass
   bool have_pass = false;
+  long long pass_id = 0;  // of that pass; never used twice
   tea_gb300_adjoint_config cfg{};
   double rx = 0, ry = 0;
   long long fwd_iters = 0;
@@ -141,6 +142,7 @@ struct Adjoint {
 };
 
 Adjoint g_adj;
+long long g_passes = 0;  // forward passes kept since load
 
 void release_adjoint() {
   Adjoint& a = g_adj;
@@ -448,12 +450,17 @@ extern "C" int tea_gb300_adjoint_forward(const double* density, const double* en
   a.fwd_ms = ms;
   a.checkpoints = nseg;
   a.have_pass = u_obs != nullptr && error_count() == errors;
+  if (a.have_pass) a.pass_id = ++g_passes;
   if (stats) {
     stats->forward_iterations = iters;
     stats->checkpoints = nseg;
     stats->forward_ms = ms;
   }
   return error_count() == errors ? 0 : -1;
+}
+
+extern "C" long long tea_gb300_adjoint_pass(void) {
+  return g_adj.ready && g_adj.have_pass ? g_adj.pass_id : 0;
 }
 
 extern "C" int tea_gb300_adjoint_backward(double* grad_log_density,

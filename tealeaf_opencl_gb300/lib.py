@@ -53,7 +53,7 @@ EXTRA_SYMBOLS = [
     "tea_gb300_batch_read_field", "tea_gb300_batch_set_launch",
     "tea_gb300_batch_get_launch", "tea_gb300_batch_autotune", "tea_gb300_batch_free",
     "tea_gb300_adjoint_create", "tea_gb300_adjoint_forward", "tea_gb300_adjoint_backward",
-    "tea_gb300_adjoint_free",
+    "tea_gb300_adjoint_pass", "tea_gb300_adjoint_free",
 ]
 
 
@@ -225,6 +225,7 @@ def load(build=True):
                                           C.POINTER(AdjointConfig), PD, C.c_void_p,
                                           C.POINTER(AdjointStats)]),
         "tea_gb300_adjoint_backward": (i, [C.c_void_p, C.POINTER(AdjointStats)]),
+        "tea_gb300_adjoint_pass": (C.c_longlong, []),
         "tea_gb300_adjoint_free": (v, []),
     }
     for name, (res, args) in sig.items():
@@ -619,6 +620,11 @@ class Adjoint:
             check()
             raise TeaError("adjoint_backward failed")
         return st
+
+    @staticmethod
+    def kept_pass():
+        """Number of the forward pass that backward() would use, or 0."""
+        return load().tea_gb300_adjoint_pass()
 
     def free(self):
         load().tea_gb300_adjoint_free()
