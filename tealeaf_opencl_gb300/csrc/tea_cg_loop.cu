@@ -16,6 +16,7 @@
 
 #include "tea_cg.cuh"
 #include "tea_device.cuh"
+#include "tea_loop.cuh"
 
 namespace tea {
 
@@ -36,13 +37,6 @@ struct LoopShared {
   int go;      // barrier passed
   int stop;    // the loop ends after this iteration
 };
-
-// t + 0.0 without the FP64 pipe: only -0 changes (a signalling NaN, which no
-// arithmetic makes, would be quieted)
-__device__ __forceinline__ double plus_zero(double t) {
-  const long long b = __double_as_longlong(t);
-  return __longlong_as_double(b == (long long)0x8000000000000000ull ? 0 : b);
-}
 
 // The least non-negative x with sqrt(x) >= t, so that sqrt(x) < t can be
 // tested without the square root (monotonic), or -1 where t^2 leaves the
@@ -101,59 +95,6 @@ __device__ __forceinline__ void loop_pass(const Dev& d, double* partials, LoopSh
   }
 }
 
-// Grid barrier on a counter that only grows during the launch.  Bounded: a
-// block that polls spin_limit times, or sees another's error flag, sets the
-// flag and returns false, and the kernel must return.
-__device__ __forceinline__ bool loop_barrier(unsigned int* bar, int* err, int* timed_out,
-                                             unsigned int target, long long spin_limit,
-                                             LoopShared& sh) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-    for (long long spins = 0;;) {
-      unsigned int v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-      if ((int)(v - target) >= 0) break;
-      if (++spins > spin_limit || ((spins & 255) == 0 && *(volatile int*)err)) {
-        atomicExch(err, 1);
-        *timed_out = 1;
-        ok = 0;
-        break;
-      }
-    }
-    sh.go = ok;
-  }
-  __syncthreads();
-  return sh.go != 0;
-}
-
-// The reduced value (step 4 of the summation order) in lane 0 of warps 0 and
-// 1 of every block.
-__device__ __forceinline__ double loop_total(const double* partials, int ns, LoopShared& sh) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x < kBlock) {
-    double a = 0.0;
-#pragma unroll 4
-    for (int k = threadIdx.x; k < ns; k += kBlock) a = a + __ldcg(partials + k);
-    sh.lanes[threadIdx.x] = a;
-  }
-  __syncthreads();
-  if (warp < 2) {
-    const double* a = sh.lanes + warp * 128 + lane;
-    const double t = bfly4(a[0], a[32], a[64], a[96]);
-    if ((lane & 7) == 0) sh.tiles[warp * 4 + bfly4_slot(lane)] = t;
-  }
-  __syncthreads();
-  double t = 0.0;
-  if (warp < 2) {
-    t = lane < 8 ? plus_zero(sh.tiles[lane]) : 0.0;
-#pragma unroll
-    for (int off = 4; off >= 1; off >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, off);
-  }
-  return t;
-}
-
 template <int TH, int F>
 __global__ void __launch_bounds__(kLoopThreads, 1)
     k_cg_loop(Dev d, double* p2, Red red, ResState* st, unsigned int* bar, int* err,
@@ -183,8 +124,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
       return loop_w_tile<TH, F>(d, pin, pout, zsrc, x, y0, alpha, beta, first);
     });
     target += arrivals;
-    if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, sh)) return;
-    const double pw = loop_total(pw_parts, d.ns, sh);
+    if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, &sh.go)) return;
+    const double pw = loop_total(pw_parts, d.ns, sh.lanes, sh.tiles);
     if (threadIdx.x == 0) sh.alpha = rro / pw;
     __syncthreads();
     alpha = sh.alpha;
@@ -194,8 +135,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
       return acc[0];
     });
     target += arrivals;
-    if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, sh)) return;
-    const double rrn = loop_total(rz_parts, d.ns, sh);
+    if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, &sh.go)) return;
+    const double rrn = loop_total(rz_parts, d.ns, sh.lanes, sh.tiles);
     // the host steps of the iteration (cg_scalar_step): beta by thread 0, the
     // exit test beside it by thread 32
     if (threadIdx.x == 0) {

@@ -12,8 +12,8 @@
 // On GB300 the FP64 pipe bounds the FP64 stencils while FP32 stencils run at
 // HBM speed with half the bytes, so each inner iteration costs a fraction
 // of an FP64 CG iteration; the few FP64 residual passes keep the answer an
-// FP64 one.  The inner loop keeps its scalars on the device and runs in
-// batches replayed from a CUDA graph, like the FP64 resident CG loop.
+// FP64 one.  The inner loop runs as one cooperative launch per correction
+// (k_mix_loop), its scalars on the device.
 //
 // Every sum uses the fixed tile order of tea_device.cuh.  Within a lane the
 // (at most 16) products of an FP32 dot product are accumulated exactly as
@@ -31,6 +31,7 @@
 
 #include "../../include/tealeaf_gb300.h"
 #include "tea_device.cuh"
+#include "tea_loop.cuh"
 
 namespace tea {
 
@@ -47,7 +48,8 @@ struct MixState {
   double rro, pw, rrn, alpha, beta, rz0;
   double eps2;  // (inner relative tolerance)^2 * rz0
   int n, max_iters, stop, p_pending;
-  int done_iters, pad;
+  int done_iters;
+  int timed_out;   // a grid barrier of the one-launch loop gave up
   double* alphas;  // CG alpha and beta by iteration number (PPCG presteps)
   double* betas;
 };
@@ -62,7 +64,6 @@ struct MixChunk {
   MixState* st_h = nullptr;  // pinned
   unsigned int* counter = nullptr;
   cudaGraphExec_t graph = nullptr;
-  cudaGraphExec_t graph_fused = nullptr;  // CG with calc_p folded into calc_w
   int graph_batch = 0;
   int graph_epoch = 0;  // the chunk's field_epoch at capture
 };
@@ -232,8 +233,30 @@ __global__ void __launch_bounds__(kBlock, kMixMinBlocks)
 __device__ __forceinline__ float4 ld4(const float* p) {
   return *reinterpret_cast<const float4*>(p);
 }
+template <bool CG>
+__device__ __forceinline__ float4 ldf4(const float* p) {
+  return CG ? __ldcg(reinterpret_cast<const float4*>(p)) : ld4(p);
+}
+template <bool CG>
+__device__ __forceinline__ float ldf(const float* p) {
+  return CG ? __ldcg(p) : *p;
+}
 __device__ __forceinline__ float f4(const float4& v, int k) {
   return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w;
+}
+
+// The tile sum from a quad's column sums v[0..3] (q: the quad, 0-7).  Each
+// stage adds the pairs of the butterfly, but a lane carries on with half of its
+// columns after the first two: 6 FP64 instructions in place of 15 (the last
+// two stages add columns within a quad, k with k^2, k^1).
+__device__ __forceinline__ double quad_tile_sum(const double* v, int q) {
+  const bool h4 = q & 4, h2 = q & 2;
+  const double a0 = (h4 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, h4 ? v[0] : v[2], 4);
+  const double a1 = (h4 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, h4 ? v[1] : v[3], 4);
+  double t = (h2 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, h2 ? a0 : a1, 2);
+  t = t + __shfl_xor_sync(0xffffffffu, t, 1);
+  t = t + __shfl_xor_sync(0xffffffffu, t, 4);
+  return t + __shfl_xor_sync(0xffffffffu, t, 2);
 }
 
 // Walks 4 supertiles per block and round; body(x, y0, v) gives v[k], the
@@ -255,16 +278,7 @@ __device__ __forceinline__ bool quad_driver(const Dev& d, const Red& red, Body b
       const int tx = sx * kTilesPerSuper + tile;
       if (tx < d.ntx) body(tx * kTileW + 4 * q, sy * TH, v);
     }
-    // Each stage adds the pairs of the butterfly, but a lane carries on with
-    // half of its columns after the first two: 6 FP64 instructions in place
-    // of 15 (the last two stages add columns within a quad, k with k^2, k^1).
-    const bool h4 = q & 4, h2 = q & 2;
-    const double a0 = (h4 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, h4 ? v[0] : v[2], 4);
-    const double a1 = (h4 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, h4 ? v[1] : v[3], 4);
-    double t = (h2 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, h2 ? a0 : a1, 2);
-    t = t + __shfl_xor_sync(0xffffffffu, t, 1);
-    t = t + __shfl_xor_sync(0xffffffffu, t, 4);
-    t = t + __shfl_xor_sync(0xffffffffu, t, 2);
+    const double t = quad_tile_sum(v, q);
     if (q == 0) sh[grp * 8 + tile] = t;
     int s_k[4];
 #pragma unroll
@@ -337,105 +351,142 @@ __global__ void __launch_bounds__(kBlock, 4)
 // k_mix_calc_w4.  On the first iteration of an inner solve (no calc_p
 // pending) p' is p.  In FP32 the extra multiply-adds are cheap; the pass
 // over p, Mi and r that calc_p made disappears with its launch.
-template <int TH>
-__global__ void __launch_bounds__(kBlock, 4)
-    k_mix_calc_pw4(Dev d, MixDev m, float* pout, Red red, MixState* st) {
-  if (*(volatile int*)&st->stop) return;
-  const bool pend = *(volatile int*)&st->p_pending != 0;
-  const float bf = (float)st->beta;
-  const bool last = quad_driver<TH>(d, red, [&](int x, int y0, double* v) {
-    const long long S = m.S;
-    const float* __restrict__ pin = m.p;
-    const float* __restrict__ mi = m.Mi;
-    const float* __restrict__ rr = m.r;
-    float* __restrict__ w = m.w;
-    float* __restrict__ po = pout;
-    // p' of one interior cell, or the old p elsewhere
-    auto pn1 = [&](long long c, int xx, int y) -> float {
-      const float pv = pin[c];
-      if (!pend || xx < 0 || xx >= d.x_max || y < 0 || y >= d.y_max) return pv;
-      return __fmaf_rn(bf, pv, mi[c] * rr[c]);
+// One lane's 4 columns of a tile.  CG: p and r, which other SMs write during
+// the launch, through L2.
+template <int TH, bool CG>
+__device__ __forceinline__ void mix_pw_body(const Dev& d, const MixDev& m, const float* pin_,
+                                            float* pout_, bool pend, float bf, int x, int y0,
+                                            double* v) {
+  const long long S = m.S;
+  const float* __restrict__ pin = pin_;
+  const float* __restrict__ mi = m.Mi;
+  const float* __restrict__ rr = m.r;
+  float* __restrict__ w = m.w;
+  float* __restrict__ po = pout_;
+  // p' of one interior cell, or the old p elsewhere
+  auto pn1 = [&](long long c, int xx, int y) -> float {
+    const float pv = ldf<CG>(pin + c);
+    if (!pend || xx < 0 || xx >= d.x_max || y < 0 || y >= d.y_max) return pv;
+    return __fmaf_rn(bf, pv, mi[c] * ldf<CG>(rr + c));
+  };
+  float hi[4] = {0.0f, 0.0f, 0.0f, 0.0f}, lo[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  if (x + 4 <= d.x_max) {
+    // p' of the 4 columns at row y (a halo row keeps the old p)
+    auto pn4 = [&](long long c, int y) -> float4 {
+      const float4 pv = ldf4<CG>(pin + c);
+      if (!pend || y < 0 || y >= d.y_max) return pv;
+      const float4 m4 = ld4(mi + c), r4 = ldf4<CG>(rr + c);
+      return make_float4(__fmaf_rn(bf, pv.x, m4.x * r4.x), __fmaf_rn(bf, pv.y, m4.y * r4.y),
+                         __fmaf_rn(bf, pv.z, m4.z * r4.z), __fmaf_rn(bf, pv.w, m4.w * r4.w));
     };
-    float hi[4] = {0.0f, 0.0f, 0.0f, 0.0f}, lo[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (x + 4 <= d.x_max) {
-      // p' of the 4 columns at row y (a halo row keeps the old p)
-      auto pn4 = [&](long long c, int y) -> float4 {
-        const float4 pv = ld4(pin + c);
-        if (!pend || y < 0 || y >= d.y_max) return pv;
-        const float4 m4 = ld4(mi + c), r4 = ld4(rr + c);
-        return make_float4(__fmaf_rn(bf, pv.x, m4.x * r4.x), __fmaf_rn(bf, pv.y, m4.y * r4.y),
-                           __fmaf_rn(bf, pv.z, m4.z * r4.z), __fmaf_rn(bf, pv.w, m4.w * r4.w));
-      };
-      const long long cb = cidx32(d, m, x, y0);
-      float4 ps = pn4(cb - S, y0 - 1), pc = pn4(cb, y0);
+    const long long cb = cidx32(d, m, x, y0);
+    float4 ps = pn4(cb - S, y0 - 1), pc = pn4(cb, y0);
 #pragma unroll 1
-      for (int j = 0; j < TH; j++) {
-        const int y = y0 + j;
-        float pv[4] = {0.0f, 0.0f, 0.0f, 0.0f}, wv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (y < d.y_max) {
-          const long long c = cb + j * S;
-          const float4 pnr = pn4(c + S, y + 1);
-          const float4 kx = ld4(m.Kx + c), kyc = ld4(m.Ky + c), kyn = ld4(m.Ky + c + S);
-          const float4 D = ld4(m.D + c);
-          const float pwst = pn1(c - 1, x - 1, y), peas = pn1(c + 4, x + 4, y);
-          const float kx4 = m.Kx[c + 4];
+    for (int j = 0; j < TH; j++) {
+      const int y = y0 + j;
+      float pv[4] = {0.0f, 0.0f, 0.0f, 0.0f}, wv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      if (y < d.y_max) {
+        const long long c = cb + j * S;
+        const float4 pnr = pn4(c + S, y + 1);
+        const float4 kx = ld4(m.Kx + c), kyc = ld4(m.Ky + c), kyn = ld4(m.Ky + c + S);
+        const float4 D = ld4(m.D + c);
+        const float pwst = pn1(c - 1, x - 1, y), peas = pn1(c + 4, x + 4, y);
+        const float kx4 = m.Kx[c + 4];
 #pragma unroll
-          for (int k = 0; k < 4; k++) {
-            const float xw = k == 0 ? pwst : f4(pc, k - 1);
-            const float xe = k == 3 ? peas : f4(pc, k + 1);
-            const float ke = k == 3 ? kx4 : f4(kx, k + 1);
-            const float t1 = __fmaf_rn(f4(kyc, k), f4(ps, k), f4(kyn, k) * f4(pnr, k));
-            const float t2 = __fmaf_rn(f4(kx, k), xw, ke * xe);
-            wv[k] = __fmaf_rn(f4(D, k), f4(pc, k), -t1) - t2;
-            pv[k] = f4(pc, k);
-          }
-          *reinterpret_cast<float4*>(w + c) = make_float4(wv[0], wv[1], wv[2], wv[3]);
-          *reinterpret_cast<float4*>(po + c) = pc;
-          ps = pc;
-          pc = pnr;
+        for (int k = 0; k < 4; k++) {
+          const float xw = k == 0 ? pwst : f4(pc, k - 1);
+          const float xe = k == 3 ? peas : f4(pc, k + 1);
+          const float ke = k == 3 ? kx4 : f4(kx, k + 1);
+          const float t1 = __fmaf_rn(f4(kyc, k), f4(ps, k), f4(kyn, k) * f4(pnr, k));
+          const float t2 = __fmaf_rn(f4(kx, k), xw, ke * xe);
+          wv[k] = __fmaf_rn(f4(D, k), f4(pc, k), -t1) - t2;
+          pv[k] = f4(pc, k);
         }
-#pragma unroll
-        for (int k = 0; k < 4; k++) acc_pair(hi[k], lo[k], pv[k], wv[k]);
+        *reinterpret_cast<float4*>(w + c) = make_float4(wv[0], wv[1], wv[2], wv[3]);
+        *reinterpret_cast<float4*>(po + c) = pc;
+        ps = pc;
+        pc = pnr;
       }
-    } else {
-#pragma unroll 1
-      for (int j = 0; j < TH; j++) {
-        const int y = y0 + j;
-        float pv[4] = {0.0f, 0.0f, 0.0f, 0.0f}, wv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (y < d.y_max) {
-          const long long c = cidx32(d, m, x, y);
 #pragma unroll
-          for (int k = 0; k < 4; k++)
-            if (x + k < d.x_max) {
-              const long long ck = c + k;
-              const float pc = pn1(ck, x + k, y);
-              const float t1 = __fmaf_rn(__ldg(m.Ky + ck), pn1(ck - S, x + k, y - 1),
-                                         __ldg(m.Ky + ck + S) * pn1(ck + S, x + k, y + 1));
-              const float t2 = __fmaf_rn(__ldg(m.Kx + ck), pn1(ck - 1, x + k - 1, y),
-                                         __ldg(m.Kx + ck + 1) * pn1(ck + 1, x + k + 1, y));
-              wv[k] = __fmaf_rn(__ldg(m.D + ck), pc, -t1) - t2;
-              pv[k] = pc;
-              w[ck] = wv[k];
-              po[ck] = pc;
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 4; k++) acc_pair(hi[k], lo[k], pv[k], wv[k]);
-      }
+      for (int k = 0; k < 4; k++) acc_pair(hi[k], lo[k], pv[k], wv[k]);
     }
+  } else {
+#pragma unroll 1
+    for (int j = 0; j < TH; j++) {
+      const int y = y0 + j;
+      float pv[4] = {0.0f, 0.0f, 0.0f, 0.0f}, wv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      if (y < d.y_max) {
+        const long long c = cidx32(d, m, x, y);
 #pragma unroll
-    for (int k = 0; k < 4; k++) v[k] = pair_value(hi[k], lo[k]);
-  });
-  if (last && threadIdx.x == 0) {
-    st->pw = red.result[0];
-    st->alpha = st->rro / red.result[0];
-    st->p_pending = 0;
-    __threadfence();
+        for (int k = 0; k < 4; k++)
+          if (x + k < d.x_max) {
+            const long long ck = c + k;
+            const float pc = pn1(ck, x + k, y);
+            const float t1 = __fmaf_rn(__ldg(m.Ky + ck), pn1(ck - S, x + k, y - 1),
+                                       __ldg(m.Ky + ck + S) * pn1(ck + S, x + k, y + 1));
+            const float t2 = __fmaf_rn(__ldg(m.Kx + ck), pn1(ck - 1, x + k - 1, y),
+                                       __ldg(m.Kx + ck + 1) * pn1(ck + 1, x + k + 1, y));
+            wv[k] = __fmaf_rn(__ldg(m.D + ck), pc, -t1) - t2;
+            pv[k] = pc;
+            w[ck] = wv[k];
+            po[ck] = pc;
+          }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) acc_pair(hi[k], lo[k], pv[k], wv[k]);
+    }
   }
+#pragma unroll
+  for (int k = 0; k < 4; k++) v[k] = pair_value(hi[k], lo[k]);
 }
 
 // d += alpha p; r -= alpha w; z = Mi r; r.z and the inner loop's scalar
 // step (k_mix_calc_ur's values), 4 columns per thread
+// One lane's 4 columns of a tile; a lane reads back the d, r, w and p that it
+// wrote itself.
+template <int TH>
+__device__ __forceinline__ void mix_ur_body(const Dev& d, const MixDev& m, const float* p,
+                                            float af, int x, int y0, double* v) {
+  float hi[4] = {0.0f, 0.0f, 0.0f, 0.0f}, lo[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  const bool full = x + 4 <= d.x_max;
+#pragma unroll 1
+  for (int j = 0; j < TH; j++) {
+    const int y = y0 + j;
+    float rv[4] = {0.0f, 0.0f, 0.0f, 0.0f}, zv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (y < d.y_max) {
+      const long long c = cidx32(d, m, x, y);
+      if (full) {
+        const float4 p4 = ld4(p + c), d4 = ld4(m.d + c), w4 = ld4(m.w + c);
+        const float4 r4 = ld4(m.r + c), mi4 = ld4(m.Mi + c);
+        float dv[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          dv[k] = __fmaf_rn(af, f4(p4, k), f4(d4, k));
+          rv[k] = __fmaf_rn(-af, f4(w4, k), f4(r4, k));
+          zv[k] = f4(mi4, k) * rv[k];
+        }
+        *reinterpret_cast<float4*>(m.d + c) = make_float4(dv[0], dv[1], dv[2], dv[3]);
+        *reinterpret_cast<float4*>(m.r + c) = make_float4(rv[0], rv[1], rv[2], rv[3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (x + k < d.x_max) {
+            const long long ck = c + k;
+            const float dk = __fmaf_rn(af, p[ck], m.d[ck]);
+            rv[k] = __fmaf_rn(-af, m.w[ck], m.r[ck]);
+            zv[k] = m.Mi[ck] * rv[k];
+            m.d[ck] = dk;
+            m.r[ck] = rv[k];
+          }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) acc_pair(hi[k], lo[k], rv[k], zv[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) v[k] = pair_value(hi[k], lo[k]);
+}
+
 template <int TH>
 __global__ void __launch_bounds__(kBlock, 4)
     k_mix_calc_ur4(Dev d, MixDev m, Red red, MixState* st) {
@@ -443,44 +494,7 @@ __global__ void __launch_bounds__(kBlock, 4)
   const double alpha = st->alpha;
   const float af = (float)alpha;
   const bool last = quad_driver<TH>(d, red, [&](int x, int y0, double* v) {
-    float hi[4] = {0.0f, 0.0f, 0.0f, 0.0f}, lo[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    const bool full = x + 4 <= d.x_max;
-#pragma unroll 1
-    for (int j = 0; j < TH; j++) {
-      const int y = y0 + j;
-      float rv[4] = {0.0f, 0.0f, 0.0f, 0.0f}, zv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      if (y < d.y_max) {
-        const long long c = cidx32(d, m, x, y);
-        if (full) {
-          const float4 p4 = ld4(m.p + c), d4 = ld4(m.d + c), w4 = ld4(m.w + c);
-          const float4 r4 = ld4(m.r + c), mi4 = ld4(m.Mi + c);
-          float dv[4];
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            dv[k] = __fmaf_rn(af, f4(p4, k), f4(d4, k));
-            rv[k] = __fmaf_rn(-af, f4(w4, k), f4(r4, k));
-            zv[k] = f4(mi4, k) * rv[k];
-          }
-          *reinterpret_cast<float4*>(m.d + c) = make_float4(dv[0], dv[1], dv[2], dv[3]);
-          *reinterpret_cast<float4*>(m.r + c) = make_float4(rv[0], rv[1], rv[2], rv[3]);
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; k++)
-            if (x + k < d.x_max) {
-              const long long ck = c + k;
-              const float dk = __fmaf_rn(af, m.p[ck], m.d[ck]);
-              rv[k] = __fmaf_rn(-af, m.w[ck], m.r[ck]);
-              zv[k] = m.Mi[ck] * rv[k];
-              m.d[ck] = dk;
-              m.r[ck] = rv[k];
-            }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 4; k++) acc_pair(hi[k], lo[k], rv[k], zv[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++) v[k] = pair_value(hi[k], lo[k]);
+    mix_ur_body<TH>(d, m, m.p, af, x, y0, v);
   });
   if (last && threadIdx.x == 0) {
     const double rrn = red.result[0];
@@ -498,6 +512,121 @@ __global__ void __launch_bounds__(kBlock, 4)
     else
       st->n = st->n + 1;
     __threadfence();
+  }
+}
+
+// ---- the whole CG inner loop as one cooperative launch ----
+
+constexpr int kMixThreads = 1024;                  // one block per SM
+constexpr int kMixSlots = kMixThreads / 64;        // supertiles in flight
+
+struct MixShared {
+  double tiles[2 * kMixSlots * kTilesPerSuper];    // two rounds' tile sums
+  double lanes[kBlock];
+  double alpha, beta;
+  int go, stop;
+};
+
+// Runs body(x, y0, v) over the block's supertiles (b, b + gridDim.x, ...), a
+// quad of columns per thread as in quad_driver, and stores the supertile
+// partials.  Two sets of tile sums, so that a round needs one barrier.
+template <int TH, class Body>
+__device__ __forceinline__ void mix_pass(const Dev& d, double* partials, MixShared& sh,
+                                         Body body) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int slot = warp >> 1, tile = 4 * (warp & 1) + (lane >> 3), q = lane & 7;
+  const int nb = gridDim.x, b = blockIdx.x;
+  const int mine = b < d.ns ? (d.ns - 1 - b) / nb + 1 : 0;
+  for (int r = 0; r * kMixSlots < mine; r++) {
+    const long long s = b + (long long)nb * (r * kMixSlots + slot);
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    if (s < d.ns) {
+      const int sy = (int)s / d.nsx, sx = (int)s - sy * d.nsx;
+      const int tx = sx * kTilesPerSuper + tile;
+      if (tx < d.ntx) body(tx * kTileW + 4 * q, sy * TH, v);
+    }
+    __syncwarp();
+    const double t = quad_tile_sum(v, q);
+    double* tiles = sh.tiles + (r & 1) * kMixSlots * kTilesPerSuper;
+    if (q == 0) tiles[slot * kTilesPerSuper + tile] = t;
+    __syncthreads();
+    if (warp < kMixSlots / 4) {
+      double u = plus_zero(tiles[warp * 32 + lane]);
+#pragma unroll
+      for (int off = 4; off >= 1; off >>= 1) u = u + __shfl_xor_sync(0xffffffffu, u, off);
+      const int k = warp * 4 + (lane >> 3);
+      const long long sk = b + (long long)nb * (r * kMixSlots + k);
+      if ((lane & 7) == 0 && sk < d.ns) __stcg(partials + sk, u);
+    }
+  }
+  __syncthreads();
+}
+
+// CG iterations until the inner solve stops, at most `iters` (even): the passes
+// mix_pw_body and mix_ur_body with a grid barrier and the sum in every block
+// after each.  p alternates between m.p and m.p2.  The passes stream (DRAM or
+// L2 latency is half of their stalls) and hold 64 registers either way, so one
+// block of 32 warps per SM runs them as their own kernels did, without the 8 us
+// of launch, drain and last-block sum: per inner iteration, against two kernels
+// replayed from a graph, 512^2 19.2 -> 14.4 us, 1024^2 23.9 -> 19.0, 2048^2
+// 62.4 -> 58.0, 4096^2 179.7 -> 178.2 (HBM floor 148 us for 60 B per cell).
+template <int TH>
+__global__ void __launch_bounds__(kMixThreads, 1)
+    k_mix_loop(Dev d, MixDev m, Red red, MixState* st, unsigned int* bar, int* err,
+               long long spin_limit, int iters) {
+  __shared__ MixShared sh;
+  double* const pw_parts = red.partials;
+  double* const rz_parts = red.partials + red.stride;
+  unsigned int target = 0;
+  double rro = st->rro;  // kept up to date by thread 0
+  const double eps2 = st->eps2;
+  const int max_iters = st->max_iters;
+  int n = st->n, it = 0, stop = 0;
+  bool pend = st->p_pending != 0;
+  float bf = (float)st->beta;
+  for (;; it++, n++) {
+    const float* pin = (it & 1) ? m.p2 : m.p;
+    float* pout = (it & 1) ? m.p : m.p2;
+    mix_pass<TH>(d, pw_parts, sh, [&](int x, int y0, double* v) {
+      mix_pw_body<TH, true>(d, m, pin, pout, pend, bf, x, y0, v);
+    });
+    target += gridDim.x;
+    if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, &sh.go)) return;
+    const double pw = loop_total(pw_parts, d.ns, sh.lanes, sh.tiles);
+    if (threadIdx.x == 0) sh.alpha = rro / pw;
+    __syncthreads();
+    const double alpha = sh.alpha;
+    const float af = (float)alpha;
+    mix_pass<TH>(d, rz_parts, sh, [&](int x, int y0, double* v) {
+      mix_ur_body<TH>(d, m, pout, af, x, y0, v);
+    });
+    target += gridDim.x;
+    if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, &sh.go)) return;
+    const double rrn = loop_total(rz_parts, d.ns, sh.lanes, sh.tiles);
+    if (threadIdx.x == 0) {
+      sh.beta = rrn / rro;
+      sh.stop = rrn <= eps2 || n >= max_iters ? 1 : it + 1 >= iters ? 2 : 0;
+      rro = rrn;
+    }
+    __syncthreads();
+    bf = (float)sh.beta;
+    pend = true;
+    stop = sh.stop;
+    if (stop) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st->pw = pw;
+        st->alpha = alpha;
+        st->beta = sh.beta;
+        st->rro = st->rrn = rrn;
+      }
+      break;
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->done_iters = n;
+    st->n = stop == 1 ? n : n + 1;
+    st->stop = stop == 1;
+    st->p_pending = 1;
   }
 }
 
@@ -728,29 +857,9 @@ static void enqueue_inner(Chunk& c, int iters) {
   }
 }
 
-// The CG inner loop with calc_p folded into calc_w: iteration i reads p
-// from one buffer and writes p' to the other, so an even count ends where
-// it began.
-template <int TH>
-static void enqueue_inner_fused(Chunk& c, int iters) {
-  const Dev d = c.dev();
-  const Red red = c.red();
-  MixDev m[2] = {g_mix.dev, g_mix.dev};
-  m[1].p = g_mix.dev.p2;
-  const int nblk4 = (d.ns + 3) / 4;
-  const int gw = mix_grid(c, k_mix_calc_pw4<TH>, nblk4);
-  const int gu = mix_grid(c, k_mix_calc_ur4<TH>, nblk4);
-  for (int i = 0; i < iters; i++) {
-    const int a = i & 1, b = a ^ 1;
-    k_mix_calc_pw4<TH><<<gw, kBlock, 0, c.stream>>>(d, m[a], m[b].p, red, g_mix.st);
-    k_mix_calc_ur4<TH><<<gu, kBlock, 0, c.stream>>>(d, m[b], red, g_mix.st);
-  }
-}
-
 void mixed_release() {
   MixChunk& g = g_mix;
   if (g.graph) cudaGraphExecDestroy(g.graph);
-  if (g.graph_fused) cudaGraphExecDestroy(g.graph_fused);
   for (float*& b : g.base) {
     cudaFree(b);
     b = nullptr;
@@ -782,7 +891,7 @@ static bool mixed_alloc(Chunk& c) {
   g.dev.S = g.S;
   if (!check_cuda(cudaMalloc(&g.st, sizeof(MixState)), "cudaMalloc mixed state") ||
       !check_cuda(cudaMallocHost(&g.st_h, sizeof(MixState)), "cudaMallocHost") ||
-      !check_cuda(cudaMalloc(&g.counter, sizeof(unsigned int)), "cudaMalloc counter"))
+      !check_cuda(cudaMalloc(&g.counter, 3 * sizeof(unsigned int)), "cudaMalloc counter"))
     return false;
   cudaMemsetAsync(g.counter, 0, sizeof(unsigned int), c.stream);
   g.ready = true;
@@ -835,7 +944,7 @@ static cudaGraphExec_t mix_capture(Chunk& c, F enqueue) {
 // Uploads h, replays `graph` (iters_per_replay iterations, `kernels`
 // kernels each) until the inner loop has stopped, and reads h back.
 static bool run_inner(Chunk& c, cudaGraphExec_t graph, int iters_per_replay, int kernels,
-                      MixState& h, bool stop_only = false) {
+                      MixState& h) {
   MixChunk& g = g_mix;
   if (!check_cuda(cudaMemcpyAsync(g.st, &h, sizeof(MixState), cudaMemcpyHostToDevice,
                                   c.stream),
@@ -854,9 +963,49 @@ static bool run_inner(Chunk& c, cudaGraphExec_t graph, int iters_per_replay, int
                     "mixed state read") ||
         !check_cuda(cudaStreamSynchronize(c.stream), "mixed sync"))
       return false;
-    // the loop with calc_p folded into calc_w leaves the last p' unformed:
-    // a CG correction starts again from p = z
-    if (h.stop && (stop_only || !h.p_pending)) return true;
+    if (h.stop && !h.p_pending) return true;
+  }
+}
+
+// The same inner solve through k_mix_loop.
+template <int TH>
+static bool run_inner_loop(Chunk& c, MixState& h) {
+  MixChunk& g = g_mix;
+  if (!check_cuda(cudaMemcpyAsync(g.st, &h, sizeof(MixState), cudaMemcpyHostToDevice, c.stream),
+                  "mixed state upload"))
+    return false;
+  Dev d = c.dev();
+  MixDev m = g.dev;
+  Red red = c.red();
+  unsigned int* bar = g.counter + 1;
+  int* err = (int*)(g.counter + 2);
+  long long spins = c.barrier_spin_limit;
+  int iters = kLoopLaunchIters;
+  const int grid = std::max(1, std::min(d.ns, c.num_sms));
+  void* args[] = {&d, &m, &red, &g.st, &bar, &err, &spins, &iters};
+  const long long launches = (long long)(h.max_iters - h.n) / iters + 2;
+  for (long long k = 0;; k++) {
+    if (!check_cuda(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned int), c.stream),
+                    "mixed barrier reset") ||
+        !check_cuda(cudaLaunchCooperativeKernel((const void*)k_mix_loop<TH>, dim3(grid),
+                                                dim3(kMixThreads), args, 0, c.stream),
+                    "mixed loop launch"))
+      return false;
+    count_launches(1);
+    if (!check_cuda(cudaMemcpyAsync(&h, g.st, sizeof(MixState), cudaMemcpyDeviceToHost,
+                                    c.stream),
+                    "mixed state read") ||
+        !check_cuda(cudaStreamSynchronize(c.stream), "mixed sync"))
+      return false;
+    if (h.timed_out) {
+      fail(25, "mixed inner loop: a grid barrier timed out");
+      return false;
+    }
+    if (h.stop) return true;
+    if (k >= launches) {
+      fail(40, "mixed inner loop did not stop after %lld launches", k + 1);
+      return false;
+    }
   }
 }
 
@@ -876,18 +1025,12 @@ static bool mixed_solve_t(Chunk& c, double tol, double inner_tol, int max_outer,
   if (g.graph && g.graph_epoch != c.field_epoch) {
     cudaGraphExecDestroy(g.graph);  // the chunk's r/sd buffers have traded places
     g.graph = nullptr;
-    if (g.graph_fused) cudaGraphExecDestroy(g.graph_fused);
-    g.graph_fused = nullptr;
   }
-  if (!g.graph) {
+  if (solver == SOLVER_PPCG && !g.graph) {  // its CG presteps
     g.graph = mix_capture(c, [&]() { enqueue_inner<TH>(c, batch); });
     if (!g.graph) return false;
     g.graph_batch = batch;
     g.graph_epoch = c.field_epoch;
-  }
-  if (!g.graph_fused) {
-    g.graph_fused = mix_capture(c, [&]() { enqueue_inner_fused<TH>(c, batch); });
-    if (!g.graph_fused) return false;
   }
   double res[2];
   auto outer_residual = [&](double* out) -> bool {
@@ -993,7 +1136,7 @@ static bool mixed_solve_t(Chunk& c, double tol, double inner_tol, int max_outer,
         if (!run_inner(c, ppcg_graph, ppcg_batch, ppcg_batch * (5 + 2 * inner_steps), h))
           return cleanup(false);
         cheby_total += (long long)h.done_iters * inner_steps;
-      } else if (!run_inner(c, g.graph_fused, batch, 2 * batch, h, true)) {
+      } else if (!run_inner_loop<TH>(c, h)) {
         return cleanup(false);
       }
       inner_total += h.done_iters;
