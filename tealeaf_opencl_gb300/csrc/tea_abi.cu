@@ -525,30 +525,39 @@ constexpr size_t kStage = 8u << 20;
 static std::mutex g_stage_mutex;
 static char* g_stage = nullptr;
 static cudaEvent_t g_stage_ev[2] = {nullptr, nullptr};
+static int g_stage_device = -1;  // the events' device
+
+static void release_stage_events() {
+  for (cudaEvent_t& e : g_stage_ev) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
+  }
+  g_stage_device = -1;
+}
 
 static void release_stage() {
   std::lock_guard<std::mutex> lock(g_stage_mutex);
   cudaFreeHost(g_stage);
   g_stage = nullptr;
-  for (cudaEvent_t& e : g_stage_ev) {
-    if (e) cudaEventDestroy(e);
-    e = nullptr;
-  }
+  release_stage_events();
 }
 
-static bool ensure_stage() {
-  if (g_stage) return true;
-  if (cudaMallocHost(&g_stage, 2 * kStage) != cudaSuccess) {
+static bool ensure_stage(int device) {
+  if (!g_stage && cudaMallocHost(&g_stage, 2 * kStage) != cudaSuccess) {
     cudaGetLastError();
     g_stage = nullptr;
     return false;
   }
+  if (g_stage_device == device) return true;
+  release_stage_events();
   for (cudaEvent_t& e : g_stage_ev)
-    if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
       e = nullptr;
+      release_stage_events();
       return false;
     }
+  g_stage_device = device;
   return true;
 }
 
@@ -584,7 +593,7 @@ static bool block_to_host(Chunk& c, double* host, const double* dev, int w, int 
   const bool pageable = !known || at.type == cudaMemoryTypeUnregistered;
   if (bytes >= (1u << 20) && row <= kStage && pageable) {
     std::lock_guard<std::mutex> lock(g_stage_mutex);
-    if (ensure_stage()) {
+    if (ensure_stage(c.device)) {
       const int per = (int)(kStage / row), chunks = (h + per - 1) / per;
       for (int k = 0; k <= chunks; k++) {
         if (k < chunks) {

@@ -374,6 +374,63 @@ __device__ __forceinline__ void loop_r_tile(const Dev& d, int x, int y0, double 
   }
 }
 
+// tea_leaf_jacobi_copy_u and tea_leaf_jacobi_solve in one pass
+// (tea_leaf_jacobi_cl.cl:3-42; un is vector_Mi, as in the reference,
+// ocl_kernels.cpp:576-585): un = u over the interior, one sweep from un, the sum
+// of |u - un|.  The sweep reads the old u where un would hold its copy, and
+// un's own halo; the new u goes to unew with u's halo ring, and un gets the old
+// u, so the fields end as the two kernels leave them.  48 bytes per cell in
+// place of 56 and one launch in place of two.  The sums of each cell stay in
+// the reference's association (its denominator differs from the stored
+// diagonal); two of the four products run on the integer pipes beside the
+// division (bit-identical).  One lane's column of one tile: the lane's share of
+// the sum.  un, where the old u goes, may be null (the resident loop copies it
+// once at its end).  CG: u through L2, where other SMs write it during the
+// launch.
+template <int TH, bool CG>
+__device__ __forceinline__ double jacobi_tile(const Dev& d, const double* __restrict__ u,
+                                              double* __restrict__ unew, double* __restrict__ un,
+                                              int x, int y0) {
+  const double* hal = d.un;  // read only outside the interior
+  const long long S = d.S;
+  const double* west = x > 0 ? u : hal;
+  const double* east = x + 1 < d.x_max ? u : hal;
+  const int rows = min(TH, d.y_max - y0);
+  double acc = 0.0;
+#pragma unroll 1
+  for (int g = 0; g < rows; g += 4) {
+    const long long c0 = cidx(d, x, y0 + g);
+    const int last = rows - 1 - g;  // last interior row of the group, or more
+    double uc[6], kyv[5], nw[4], v[4];
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+      const int j = min(i - 1, last + 1), y = y0 + g + j;
+      uc[i] = ldv<CG>((y < 0 || y >= d.y_max ? hal : u) + c0 + j * S);
+    }
+#pragma unroll
+    for (int i = 0; i < 5; i++) kyv[i] = __ldg(d.Ky + c0 + min(i, last + 1) * S);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const long long c = c0 + min(j, last) * S;
+      const double kxc = __ldg(d.Kx + c), kxe = __ldg(d.Kx + c + 1);
+      const double s = __ldg(d.u0 + c) + emu_dmul(kxe, ldv<CG>(east + c + 1)) +
+                       kxc * ldv<CG>(west + c - 1) + emu_dmul(kyv[j + 1], uc[j + 2]) +
+                       kyv[j] * uc[j];
+      nw[j] = emu_ddiv_var(s, 1.0 + (kxc + kxe) + (kyv[j] + kyv[j + 1]));
+      v[j] = j <= last ? fabs(nw[j] - uc[j + 1]) : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (j <= last) {
+        unew[c0 + j * S] = nw[j];
+        if (un) un[c0 + j * S] = uc[j + 1];
+      }
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc = acc + v[j];
+  }
+  return acc;
+}
+
 // The host steps of one CG iteration (tea_solve.f90:282-330) after calc_ur,
 // on the device: beta = rrn/rro, rro = rrn, error = sqrt(rrn), and the exit
 // test (on sqrt(r.z), or on ||r||_2 when NV == 2).  result[] holds the

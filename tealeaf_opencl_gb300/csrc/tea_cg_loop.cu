@@ -201,6 +201,59 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
   });
 }
 
+// Jacobi sweeps until the exit test ends them, at most `iters` (even): u
+// alternates between d.u and u2 (whose halo ring becomes u's), one grid barrier
+// per sweep, the old u of the last one into un.  A sweep through the per-call
+// path costs a launch and a host round trip, about 20 us on small grids.
+template <int TH>
+__global__ void __launch_bounds__(kLoopThreads, 1)
+    k_jacobi_loop(Dev d, double* u2, Red red, ResState* st, unsigned int* bar, int* err,
+                  long long spin_limit, unsigned int extra, int iters) {
+  __shared__ LoopShared sh;
+  const unsigned int arrivals = gridDim.x + extra;
+  unsigned int target = 0;
+  int n = st->n, it = 0, stop = 0;
+  const int loop_max = st->loop_max;
+  const double eps_target = st->eps_target;
+  const double rr_limit = threadIdx.x == 32 ? square_limit(eps_target) : 0.0;
+  copy_halo_ring(d, d.u, u2);
+  for (;; it++, n++) {
+    const double* cur = (it & 1) ? u2 : d.u;
+    double* nxt = (it & 1) ? d.u : u2;
+    // partials alternate too: a block may still read the last sweep's
+    double* parts = red.partials + (it & 1) * red.stride;
+    loop_pass<TH, true>(d, parts, sh, [&](int x, int y0) {
+      return x < d.x_max ? jacobi_tile<TH, true>(d, cur, nxt, nullptr, x, y0) : 0.0;
+    });
+    target += arrivals;
+    if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, &sh.go)) return;
+    const double sum = loop_total(parts, d.ns, sh.lanes, sh.tiles);
+    if (threadIdx.x == 32) {
+      const bool done = rr_limit > 0.0 ? sum < rr_limit && sum >= 0.0 : sqrt(sum) < eps_target;
+      const int s = done              ? kStopConverged
+                    : n >= loop_max   ? kStopLoopMax
+                    : it + 1 >= iters ? kStopLaunch
+                                      : 0;
+      if (blockIdx.x == 0 && s) st->error = sqrt(sum);
+      sh.stop = s;
+    }
+    __syncthreads();
+    stop = sh.stop;
+    if (stop) break;
+  }
+  const double* old = (it & 1) ? u2 : d.u;
+  loop_pass<TH, false>(d, red.partials, sh, [&](int x, int y0) {
+    if (x < d.x_max)
+      for (int y = y0; y < min(y0 + TH, d.y_max); y++) d.un[cidx(d, x, y)] = old[cidx(d, x, y)];
+    return 0.0;
+  });
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->converged = stop == kStopConverged;
+    st->n = stop == kStopLaunch ? n + 1 : n;
+    st->stop = stop != kStopLaunch;
+  }
+}
+
 // ---- the two passes as separate kernels, for grids whose passes are long
 // beside a launch (replayed from a graph) ----
 
@@ -301,6 +354,23 @@ bool launch_loop_t(const LaunchCtx& l, Dev d, double* p2, Red red, ResState* st,
 }
 
 }  // namespace
+
+bool launch_jacobi_loop(const LaunchCtx& l, const Dev& d_, double* u2, const Red& red_,
+                        ResState* st, unsigned int* bar, long long spin_limit,
+                        unsigned int extra) {
+  Dev d = d_;
+  Red red = red_;
+  int grid = std::max(1, std::min(d.ns, l.num_sms)), iters = kLoopLaunchIters;
+  int* err = (int*)(bar + 1);
+  void* args[] = {&d, &u2, &red, &st, &bar, &err, &spin_limit, &extra, &iters};
+  const void* fn = d.th == 16 ? (const void*)k_jacobi_loop<16> : (const void*)k_jacobi_loop<4>;
+  count_launch("resident_jacobi_loop");
+  return check_cuda(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned int), l.stream),
+                    "Jacobi loop barrier reset") &&
+         check_cuda(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kLoopThreads), args, 0,
+                                                l.stream),
+                    "Jacobi loop launch");
+}
 
 // The line between the two: a launch boundary costs a pass about 10 us (start,
 // drain, the last block's sum), a grid barrier with the sum in every block

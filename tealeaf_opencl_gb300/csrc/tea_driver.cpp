@@ -759,6 +759,22 @@ class Driver {
         tea_leaf_cg_calc_p_kernel_ocl_(&beta);
         error = rrn;
         rro = rrn;
+      } else if (use_jacobi && mode == TEA_DRIVER_RESIDENT && !D.verbose &&
+                 !(checks & TEA_CHECK_BREAKDOWN) &&
+                 tea::cg_loop_fits(tea::chunk().dev(), tea::chunk().num_sms)) {
+        // us per sweep, per call / on the device: 64^2 16.0 / 9.3, 512^2 20.9 /
+        // 14.3, 1024^2 47.8 / 40.1, 2048^2 146 / 153
+        int n_done = 0, conv = 0;
+        if (tea::resident_jacobi_iterations(n, loop_max, D.eps * initial_residual, &error,
+                                            &n_done, &conv) != 0)
+          return -1;
+        n = n_done;
+        if (conv) {
+          exited = true;
+          break;
+        }
+        n++;
+        continue;
       } else if (use_jacobi) {
         tea_leaf_jacobi_solve_kernel_ocl_(&error);
         if (!norm_ok(error, n, "the Jacobi error")) return -1;

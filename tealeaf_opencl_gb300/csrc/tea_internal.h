@@ -251,6 +251,11 @@ constexpr long long kLoopSpins = 1LL << 26;  // polls of a barrier before it giv
 bool cg_loop_fits(const Dev& d, int num_sms);
 bool launch_cg_loop(const LaunchCtx& l, const Dev& d, double* p2, const Red& red, ResState* st,
                     unsigned int* bar, long long spin_limit, unsigned int extra);
+// The same for Jacobi sweeps; u2: the second u buffer.  The result is in u2
+// after an odd number of sweeps.
+bool launch_jacobi_loop(const LaunchCtx& l, const Dev& d, double* u2, const Red& red,
+                        ResState* st, unsigned int* bar, long long spin_limit,
+                        unsigned int extra);
 // `iters` (even) iterations of the same loop as two kernels each, and the
 // kernel that finishes u and p once it has stopped, queued for a graph.
 // counter: one word, zero.
@@ -273,6 +278,8 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
 int resident_ppcg_iterations(int n_begin, int loop_max, double rro_in,
                              double eps_target, double* rro_out, double* error_out,
                              int* n_done, int* converged);
+int resident_jacobi_iterations(int n_begin, int loop_max, double eps_target, double* error_out,
+                               int* n_done, int* converged);
 void resident_release();
 // fused pair of PPCG inner steps (tea_ppcg_tb.cu)
 bool tb_applicable(const Chunk& c);

@@ -991,60 +991,13 @@ __global__ void __launch_bounds__(kBlock, 1)
   });
 }
 
-// tea_leaf_jacobi_copy_u and tea_leaf_jacobi_solve in one pass
-// (tea_leaf_jacobi_cl.cl:3-42; un is vector_Mi, as in the reference,
-// ocl_kernels.cpp:576-585): un = u over the interior, one sweep from un, the sum
-// of |u - un|.  The sweep reads the old u where un would hold its copy, and
-// un's own halo; the new u goes to unew with u's halo ring, and un gets the old
-// u, so the fields end as the two kernels leave them.  48 bytes per cell in
-// place of 56 and one launch in place of two.  The sums of each cell stay in
-// the reference's association (its denominator differs from the stored
-// diagonal); two of the four products run on the integer pipes beside the
-// division (bit-identical).
+// one Jacobi sweep (jacobi_tile)
 template <int TH, int F>
-__global__ void __launch_bounds__(kBlock) k_jacobi_sweep(Dev d, Red red, double* unew_) {
+__global__ void __launch_bounds__(kBlock) k_jacobi_sweep(Dev d, Red red, double* unew) {
   tile_driver<TH, 1>(d, red, [&](int x, int y0, bool xin, double* acc) {
-    const double* __restrict__ u = d.u;
-    const double* __restrict__ hal = d.un;  // read only outside the interior
-    double* __restrict__ un = d.un;         // written only inside it
-    double* __restrict__ unew = unew_;
-    const long long S = d.S;
-    if (!xin) return;
-    const double* west = x > 0 ? u : hal;
-    const double* east = x + 1 < d.x_max ? u : hal;
-    const int rows = min(TH, d.y_max - y0);
-#pragma unroll 1
-    for (int g = 0; g < rows; g += 4) {
-      const long long c0 = cidx(d, x, y0 + g);
-      const int last = rows - 1 - g;  // last interior row of the group, or more
-      double uc[6], kyv[5], nw[4], v[4];
-#pragma unroll
-      for (int i = 0; i < 6; i++) {
-        const int j = min(i - 1, last + 1), y = y0 + g + j;
-        uc[i] = (y < 0 || y >= d.y_max ? hal : u)[c0 + j * S];
-      }
-#pragma unroll
-      for (int i = 0; i < 5; i++) kyv[i] = __ldg(d.Ky + c0 + min(i, last + 1) * S);
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const long long c = c0 + min(j, last) * S;
-        const double kxc = __ldg(d.Kx + c), kxe = __ldg(d.Kx + c + 1);
-        const double s = __ldg(d.u0 + c) + emu_dmul(kxe, east[c + 1]) + kxc * west[c - 1] +
-                         emu_dmul(kyv[j + 1], uc[j + 2]) + kyv[j] * uc[j];
-        nw[j] = emu_ddiv_var(s, 1.0 + (kxc + kxe) + (kyv[j] + kyv[j + 1]));
-        v[j] = j <= last ? fabs(nw[j] - uc[j + 1]) : 0.0;
-      }
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (j <= last) {
-          unew[c0 + j * S] = nw[j];
-          un[c0 + j * S] = uc[j + 1];
-        }
-#pragma unroll
-      for (int j = 0; j < 4; j++) acc[0] = acc[0] + v[j];
-    }
+    if (xin) acc[0] = jacobi_tile<TH, false>(d, d.u, unew, d.un, x, y0);
   });
-  copy_halo_ring(d, d.u, unew_);
+  copy_halo_ring(d, d.u, unew);
 }
 
 // tea_leaf_finalise, tea_leaf_common_cl.cl:4-15
@@ -1605,6 +1558,17 @@ void resident_release() {
 // stopped return at once.  The arithmetic and the exit test are those of the
 // per-call path, so the results are bit-identical to it.  The true-residual
 // exit (r.r beside r.z) and profiling use the kernels.
+static bool ensure_resident_state(Chunk& c) {
+  if (c.res_state) return true;
+  if (!check_cuda(cudaMalloc(&c.res_state, sizeof(ResState)), "cudaMalloc state") ||
+      !check_cuda(cudaMallocHost(&c.res_state_h, sizeof(ResState)), "cudaMallocHost state") ||
+      !check_cuda(cudaMalloc(&c.res_counter, sizeof(unsigned int)), "cudaMalloc counter") ||
+      !check_cuda(cudaMalloc(&c.res_bar, 3 * sizeof(unsigned int)), "cudaMalloc barrier"))
+    return false;
+  cudaMemsetAsync(c.res_counter, 0, sizeof(unsigned int), c.stream);
+  return true;
+}
+
 static bool use_cg_loop(const Chunk& c, bool true_exit) {
   if (true_exit || c.profiler_on || c.resident_mode == 1) return false;
   return c.resident_mode == 2 || cg_loop_fits(c.dev(), c.num_sms);
@@ -1631,17 +1595,7 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
       return -1;
     c.res_coef_n = loop_max + 2;
   }
-  if (!c.res_state) {
-    if (!check_cuda(cudaMalloc(&c.res_state, sizeof(ResState)), "cudaMalloc state") ||
-        !check_cuda(cudaMallocHost(&c.res_state_h, sizeof(ResState)),
-                    "cudaMallocHost state") ||
-        !check_cuda(cudaMalloc(&c.res_counter, sizeof(unsigned int)),
-                    "cudaMalloc counter") ||
-        !check_cuda(cudaMalloc(&c.res_bar, 3 * sizeof(unsigned int)),
-                    "cudaMalloc barrier"))
-      return -1;
-    cudaMemsetAsync(c.res_counter, 0, sizeof(unsigned int), c.stream);
-  }
+  if (!ensure_resident_state(c)) return -1;
   ResState& h = *c.res_state_h;
   memset(&h, 0, sizeof(h));
   h.rro = rro_in;
@@ -1737,6 +1691,51 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
   return 0;
 }
 
+// Jacobi sweeps n_begin..loop_max as the per-call path makes them, on the
+// device until the driver's exit test (sqrt of the summed change) ends them.
+int resident_jacobi_iterations(int n_begin, int loop_max, double eps_target, double* error_out,
+                               int* n_done, int* converged) {
+  Chunk& c = chunk();
+  if (!ensure_resident_state(c) || !ensure_u_alt(c)) return -1;
+  ResState& h = *c.res_state_h;
+  memset(&h, 0, sizeof(h));
+  h.eps_target = eps_target;
+  h.n = h.n_first = n_begin;
+  h.loop_max = loop_max;
+  if (!check_cuda(cudaMemcpyAsync(c.res_state, &h, sizeof(ResState), cudaMemcpyHostToDevice,
+                                  c.stream),
+                  "resident state upload"))
+    return -1;
+  const LaunchCtx l{c.stream, c.num_sms, c.arith};
+  const long long launches = (long long)(loop_max - n_begin) / kLoopLaunchIters + 2;
+  for (long long k = 0;; k++) {
+    if (!launch_jacobi_loop(l, c.dev(), c.u2.f, c.red(), c.res_state, c.res_bar,
+                            c.barrier_spin_limit, (unsigned int)c.barrier_extra) ||
+        !check_cuda(cudaMemcpyAsync(&h, c.res_state, sizeof(ResState), cudaMemcpyDeviceToHost,
+                                    c.stream),
+                    "resident state read") ||
+        !check_cuda(cudaStreamSynchronize(c.stream), "resident Jacobi loop"))
+      return -1;
+    if (h.timed_out) {
+      fail(25, "resident Jacobi loop: a grid barrier timed out");
+      return -1;
+    }
+    if (h.stop) break;
+    if (k >= launches) {
+      fail(24, "resident Jacobi loop ended before its exit test");
+      return -1;
+    }
+  }
+  if ((h.n - n_begin + 1) & 1) {  // the last sweep wrote the second buffer
+    std::swap(c.u, c.u2);
+    c.field_epoch++;
+  }
+  *error_out = h.error;
+  *n_done = h.n;
+  *converged = h.converged;
+  return 0;
+}
+
 // PPCG iterations n_begin..loop_max with all scalars on the device, batches
 // of 4 iterations replayed from a captured graph until the loop stops.  The
 // kernels and the exit test are those of the per-call path (whose
@@ -1750,17 +1749,7 @@ int resident_ppcg_iterations(int n_begin, int loop_max, double rro_in,
     return -1;
   }
   const int batch = 4;
-  if (!c.res_state) {
-    if (!check_cuda(cudaMalloc(&c.res_state, sizeof(ResState)), "cudaMalloc state") ||
-        !check_cuda(cudaMallocHost(&c.res_state_h, sizeof(ResState)),
-                    "cudaMallocHost state") ||
-        !check_cuda(cudaMalloc(&c.res_counter, sizeof(unsigned int)),
-                    "cudaMalloc counter") ||
-        !check_cuda(cudaMalloc(&c.res_bar, 3 * sizeof(unsigned int)),
-                    "cudaMalloc barrier"))
-      return -1;
-    cudaMemsetAsync(c.res_counter, 0, sizeof(unsigned int), c.stream);
-  }
+  if (!ensure_resident_state(c)) return -1;
   flush_pending_inner(c);
   const bool pairs = resident_pairs(c);
   if (pairs && (!ensure_alt_fields(c) || !tb_prepare(c))) return -1;
