@@ -20,7 +20,7 @@ namespace tea {
 // the previous group's stores and keep more loads in flight.  Same
 // arithmetic and per-lane summation order; with 4 blocks per SM (64
 // registers) 192.2 -> 174.4 us at 4096^2 on non-zero fields.
-template <int TH, int F>
+template <int TH, int F, bool EMU = true>
 __device__ __forceinline__ void cg_w_tile_r(const Dev& d, int x, int y0, bool xin,
                                             double* acc) {
   const double* __restrict__ p = d.p;
@@ -40,7 +40,7 @@ __device__ __forceinline__ void cg_w_tile_r(const Dev& d, int x, int y0, bool xi
       if (xin && g + j < d.y_max) {
         const long long c = c0 + j * S;
         pv[j] = p[c];
-        wv[j] = smvp_v<F>(__ldg(dg + c), __ldg(ky + c + S), __ldg(ky + c), __ldg(kx + c + 1),
+        wv[j] = smvp_v<F, EMU>(__ldg(dg + c), __ldg(ky + c + S), __ldg(ky + c), __ldg(kx + c + 1),
                           __ldg(kx + c), pv[j], p[c + S], p[c - S], p[c + 1], p[c - 1]);
       }
     }
@@ -217,7 +217,7 @@ __device__ __forceinline__ double p_next(double beta, double p, double z) {
 // L2.  All loads of four rows are issued before anything waits for one; rows
 // past the interior are clamped to the halo row above it and lanes past the
 // last column read the row's padding, and neither is used.
-template <int TH, int F, bool COPY = false>
+template <int TH, int F, bool COPY = false, bool EMU = true>
 __device__ __forceinline__ double loop_w_tile(const Dev& d, const double* __restrict__ pin,
                                               double* __restrict__ pout,
                                               const double* __restrict__ zsrc, int x, int y0,
@@ -299,7 +299,7 @@ __device__ __forceinline__ double loop_w_tile(const Dev& d, const double* __rest
       if (lane == 31) pe = e;
       if (lane == 0) pw = wst;
       const double kyn = j < 3 && g + j + 1 < rows ? kyv[j + 1] : kyv[4];
-      const double wv = smvp_v<F>(dv[j], kyn, kyv[j], kxe[j], kxc[j], pv[j + 1], pv[j + 2], pv[j],
+      const double wv = smvp_v<F, EMU>(dv[j], kyn, kyv[j], kxe[j], kxc[j], pv[j + 1], pv[j + 2], pv[j],
                                   pe, pw);
       if (own) {
         w[c] = wv;
@@ -317,7 +317,7 @@ __device__ __forceinline__ double loop_w_tile(const Dev& d, const double* __rest
 // Pass B on one tile: r -= alpha w, z = M^-1 r and the lane's share of r.z
 // (cg_ur_tile_r without u, which pass A updates).  A lane reads back only
 // the r and w that it wrote itself.
-template <int TH, int F, int NV = 1>
+template <int TH, int F, int NV = 1, bool EMU = true>
 __device__ __forceinline__ void loop_r_tile(const Dev& d, int x, int y0, double alpha,
                                             double* acc) {
   double* __restrict__ r = d.r;
@@ -359,7 +359,7 @@ __device__ __forceinline__ void loop_r_tile(const Dev& d, int x, int y0, double 
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         rv[j] = F ? __fma_rn(-alpha, wv[j], rv[j]) : rv[j] - alpha * wv[j];
-        zv[j] = d.prec == PREC_JAC_DIAG ? mul_e<true>(rv[j], mv[j]) : rv[j];
+        zv[j] = d.prec == PREC_JAC_DIAG ? mul_e<EMU>(rv[j], mv[j]) : rv[j];
       }
     }
 #pragma unroll

@@ -95,7 +95,7 @@ __device__ __forceinline__ void loop_pass(const Dev& d, double* partials, LoopSh
   }
 }
 
-template <int TH, int F>
+template <int TH, int F, bool EMU>
 __global__ void __launch_bounds__(kLoopThreads, 1)
     k_cg_loop(Dev d, double* p2, Red red, ResState* st, unsigned int* bar, int* err,
               long long spin_limit, unsigned int extra, int iters) {
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
     double* pout = (it & 1) ? p2 : d.p;
     const bool first = it == 0;
     loop_pass<TH, true>(d, pw_parts, sh, [&](int x, int y0) {
-      return loop_w_tile<TH, F>(d, pin, pout, zsrc, x, y0, alpha, beta, first);
+      return loop_w_tile<TH, F, false, EMU>(d, pin, pout, zsrc, x, y0, alpha, beta, first);
     });
     target += arrivals;
     if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, &sh.go)) return;
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
     alpha = sh.alpha;
     loop_pass<TH, true>(d, rz_parts, sh, [&](int x, int y0) {
       double acc[1] = {0.0};
-      loop_r_tile<TH, F>(d, x, y0, alpha, acc);
+      loop_r_tile<TH, F, 1, EMU>(d, x, y0, alpha, acc);
       return acc[0];
     });
     target += arrivals;
@@ -346,10 +346,13 @@ bool launch_loop_t(const LaunchCtx& l, Dev d, double* p2, Red red, ResState* st,
   int grid = std::max(1, std::min(d.ns, l.num_sms));
   int* err = (int*)(bar + 1);
   void* args[] = {&d, &p2, &red, &st, &bar, &err, &spin_limit, &extra, &iters};
+  const void* fn = (const void*)k_cg_loop<TH, F, true>;
+  if constexpr (TH == 4)
+    if (few_supertiles(d, l.num_sms)) fn = (const void*)k_cg_loop<TH, F, false>;
   return check_cuda(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned int), l.stream),
                     "CG loop barrier reset") &&
-         check_cuda(cudaLaunchCooperativeKernel((const void*)k_cg_loop<TH, F>, dim3(grid),
-                                                dim3(kLoopThreads), args, 0, l.stream),
+         check_cuda(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kLoopThreads), args, 0,
+                                                l.stream),
                     "CG loop launch");
 }
 

@@ -247,6 +247,12 @@ void dev_cg_init_p(const LaunchCtx& l, const Dev& d, const Red& r);
 // st->stop is set, or the loop goes on with another launch.
 constexpr int kLoopLaunchIters = 1024;
 constexpr long long kLoopSpins = 1LL << 26;  // polls of a barrier before it gives up
+// At most one supertile per SM: few warps share an SM's FP64 pipe, and a
+// product there (64 cycles) is quicker than on the integer pipes (224, 45
+// instructions).  The CG loop then takes 6.6 us per iteration at 64^2 against
+// 7.3, 8.1 against 9.0 at 128^2, 11.4 against 11.6 at 256^2; with two supertiles
+// on some SMs (380^2) it is 15.0 against 14.4.
+inline bool few_supertiles(const Dev& d, int num_sms) { return d.th == 4 && d.ns <= num_sms; }
 // true where the one launch is the faster form (by size, tea_cg_loop.cu)
 bool cg_loop_fits(const Dev& d, int num_sms);
 bool launch_cg_loop(const LaunchCtx& l, const Dev& d, double* p2, const Red& red, ResState* st,

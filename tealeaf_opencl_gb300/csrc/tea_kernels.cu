@@ -443,12 +443,12 @@ __global__ void __launch_bounds__(kBlock) k_cg_init_p(Dev d, Red red) {
 // (device-resident PPCG loop) it does nothing once the loop has stopped and
 // leaves pw and alpha = rro/pw in st (one division: made by every thread of
 // the kernel that uses alpha it cost that kernel about 2.5 us).
-template <int TH, int F>
+template <int TH, int F, bool EMU = true>
 __global__ void __launch_bounds__(kBlock, 4)
     k_cg_calc_w(Dev d, Red red, ResState* st) {
   if (st && *(volatile int*)&st->stop) return;
   const bool last = tile_driver<TH, 1>(d, red, [&](int x, int y0, bool xin, double* acc) {
-    cg_w_tile_r<TH, F>(d, x, y0, xin, acc);
+    cg_w_tile_r<TH, F, EMU>(d, x, y0, xin, acc);
   });
   if (st && last && threadIdx.x == 0) {
     st->pw = red.result[0];
@@ -1144,6 +1144,17 @@ void launch_cg_init_p(Chunk& c) {
 }
 
 void launch_cg_calc_w(Chunk& c) {
+  if (few_supertiles(c.dev(), c.num_sms)) {
+    const char* name = "tea_leaf_cg_solve_calc_w";
+    ResState* const st = nullptr;
+    if (c.arith == 2)
+      launch_tile(c, name, k_cg_calc_w<4, 2, false>, c.dev(), c.red(), st);
+    else if (c.arith == 1)
+      launch_tile(c, name, k_cg_calc_w<4, 1, false>, c.dev(), c.red(), st);
+    else
+      launch_tile(c, name, k_cg_calc_w<4, 0, false>, c.dev(), c.red(), st);
+    return;
+  }
   TH_DISPATCH(c, "tea_leaf_cg_solve_calc_w", k_cg_calc_w, c.dev(), c.red(),
               (ResState*)nullptr);
 }
