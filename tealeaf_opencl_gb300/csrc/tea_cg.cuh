@@ -387,7 +387,7 @@ __device__ __forceinline__ void loop_r_tile(const Dev& d, int x, int y0, double 
 // the sum.  un, where the old u goes, may be null (the resident loop copies it
 // once at its end).  CG: u through L2, where other SMs write it during the
 // launch.
-template <int TH, bool CG>
+template <int TH, bool CG, bool EMU = true>
 __device__ __forceinline__ double jacobi_tile(const Dev& d, const double* __restrict__ u,
                                               double* __restrict__ unew, double* __restrict__ un,
                                               int x, int y0) {
@@ -413,10 +413,11 @@ __device__ __forceinline__ double jacobi_tile(const Dev& d, const double* __rest
     for (int j = 0; j < 4; j++) {
       const long long c = c0 + min(j, last) * S;
       const double kxc = __ldg(d.Kx + c), kxe = __ldg(d.Kx + c + 1);
-      const double s = __ldg(d.u0 + c) + emu_dmul(kxe, ldv<CG>(east + c + 1)) +
-                       kxc * ldv<CG>(west + c - 1) + emu_dmul(kyv[j + 1], uc[j + 2]) +
+      const double s = __ldg(d.u0 + c) + mul_e<EMU>(kxe, ldv<CG>(east + c + 1)) +
+                       kxc * ldv<CG>(west + c - 1) + mul_e<EMU>(kyv[j + 1], uc[j + 2]) +
                        kyv[j] * uc[j];
-      nw[j] = emu_ddiv_var(s, 1.0 + (kxc + kxe) + (kyv[j] + kyv[j + 1]));
+      const double den = 1.0 + (kxc + kxe) + (kyv[j] + kyv[j + 1]);
+      nw[j] = EMU ? emu_ddiv_var(s, den) : s / den;
       v[j] = j <= last ? fabs(nw[j] - uc[j + 1]) : 0.0;
     }
 #pragma unroll

@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
 // alternates between d.u and u2 (whose halo ring becomes u's), one grid barrier
 // per sweep, the old u of the last one into un.  A sweep through the per-call
 // path costs a launch and a host round trip, about 20 us on small grids.
-template <int TH>
+template <int TH, bool EMU>
 __global__ void __launch_bounds__(kLoopThreads, 1)
     k_jacobi_loop(Dev d, double* u2, Red red, ResState* st, unsigned int* bar, int* err,
                   long long spin_limit, unsigned int extra, int iters) {
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
     // partials alternate too: a block may still read the last sweep's
     double* parts = red.partials + (it & 1) * red.stride;
     loop_pass<TH, true>(d, parts, sh, [&](int x, int y0) {
-      return x < d.x_max ? jacobi_tile<TH, true>(d, cur, nxt, nullptr, x, y0) : 0.0;
+      return x < d.x_max ? jacobi_tile<TH, true, EMU>(d, cur, nxt, nullptr, x, y0) : 0.0;
     });
     target += arrivals;
     if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, &sh.go)) return;
@@ -366,7 +366,9 @@ bool launch_jacobi_loop(const LaunchCtx& l, const Dev& d_, double* u2, const Red
   int grid = std::max(1, std::min(d.ns, l.num_sms)), iters = kLoopLaunchIters;
   int* err = (int*)(bar + 1);
   void* args[] = {&d, &u2, &red, &st, &bar, &err, &spin_limit, &extra, &iters};
-  const void* fn = d.th == 16 ? (const void*)k_jacobi_loop<16> : (const void*)k_jacobi_loop<4>;
+  const void* fn = d.th == 16                    ? (const void*)k_jacobi_loop<16, true>
+                   : few_supertiles(d, l.num_sms) ? (const void*)k_jacobi_loop<4, false>
+                                                  : (const void*)k_jacobi_loop<4, true>;
   count_launch("resident_jacobi_loop");
   return check_cuda(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned int), l.stream),
                     "Jacobi loop barrier reset") &&

@@ -992,10 +992,10 @@ __global__ void __launch_bounds__(kBlock, 1)
 }
 
 // one Jacobi sweep (jacobi_tile)
-template <int TH, int F>
+template <int TH, bool EMU>
 __global__ void __launch_bounds__(kBlock) k_jacobi_sweep(Dev d, Red red, double* unew) {
   tile_driver<TH, 1>(d, red, [&](int x, int y0, bool xin, double* acc) {
-    if (xin) acc[0] = jacobi_tile<TH, false>(d, d.u, unew, d.un, x, y0);
+    if (xin) acc[0] = jacobi_tile<TH, false, EMU>(d, d.u, unew, d.un, x, y0);
   });
   copy_halo_ring(d, d.u, unew);
 }
@@ -1264,7 +1264,13 @@ void launch_ppcg_calc_sd(Chunk& c, double alpha, double beta) {
 }
 
 void launch_jacobi_sweep(Chunk& c, double* unew) {
-  TH_DISPATCH(c, "tea_leaf_jacobi_solve", k_jacobi_sweep, c.dev(), c.red(), unew);
+  const char* name = "tea_leaf_jacobi_solve";  // the same arithmetic in every form
+  if (few_supertiles(c.dev(), c.num_sms))
+    launch_tile(c, name, k_jacobi_sweep<4, false>, c.dev(), c.red(), unew);
+  else if (c.TH == 4)
+    launch_tile(c, name, k_jacobi_sweep<4, true>, c.dev(), c.red(), unew);
+  else
+    launch_tile(c, name, k_jacobi_sweep<16, true>, c.dev(), c.red(), unew);
 }
 
 void launch_finalise(Chunk& c) {
