@@ -108,11 +108,11 @@ __device__ __forceinline__ double smvp_v(double D, double kyn, double kyc, doubl
 // b - A x on values: the reference's "b - smvp" (calc_residual,
 // tea_leaf_common_cl.cl:17-36; ppcg update_r, tea_leaf_ppcg_cl.cl:62-88),
 // or in the chain form the chain of fused multiply-adds started from b.
-template <int F>
+template <int F, bool EMU = true>
 __device__ __forceinline__ double bms_v(double b, double D, double kyn, double kyc,
                                         double kxe, double kxc, double xc, double xn,
                                         double xs, double xe, double xw) {
-  if (F != 2) return b - smvp_v<F>(D, kyn, kyc, kxe, kxc, xc, xn, xs, xe, xw);
+  if (F != 2) return b - smvp_v<F, EMU>(D, kyn, kyc, kxe, kxc, xc, xn, xs, xe, xw);
   double t = __fma_rn(-D, xc, b);
   t = __fma_rn(kyn, xn, t);
   t = __fma_rn(kyc, xs, t);

@@ -63,6 +63,12 @@ static Dev dev4(const Chunk& c) { return rows4_tiling(c.dev()); }
 // 129.8); three of 80 are quicker over few tiles (500^2: 10.9 against 11.7,
 // 11.3 against 12.0).  At 1111x901, 7.4 supertiles per SM, they are level.
 static bool point_blocks4(const Chunk& c) { return dev4(c).ns > 8 * c.num_sms; }
+// The kernel of such a step for form F: by that rule, and with its products on
+// the FP64 pipe over few supertiles.
+#define TEA_POINT(kern, F, c)                                    \
+  (few_supertiles((c).dev(), (c).num_sms) ? kern<F, 3, false>    \
+   : point_blocks4(c)                     ? kern<F, 4, true>     \
+                                          : kern<F, 3, true>)
 
 
 
@@ -570,7 +576,7 @@ __global__ void __launch_bounds__(kBlock, 3)
 // One pass in place of calc_p and calc_u; 7 FP64 instructions per cell with the
 // products on the integer pipes (bit-identical), 10 with all of them on the
 // FP64 pipe.
-template <int F, int MB>
+template <int F, int MB, bool EMU>
 __global__ void __launch_bounds__(kBlock, MB)
     k_cheby_calc_pu_point(Dev d, Red red, double alpha, double beta, double* un_) {
   tile_driver<4, 0>(d, red, [&](int x, int y0, bool xin, double* acc) {
@@ -592,7 +598,7 @@ __global__ void __launch_bounds__(kBlock, MB)
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       const long long c = c0 + min(j, rows - 1) * S;
-      wl[j] = smvp_v<F>(__ldg(d.diag + c), kyv[j + 1], kyv[j], __ldg(d.Kx + c + 1),
+      wl[j] = smvp_v<F, EMU>(__ldg(d.diag + c), kyv[j + 1], kyv[j], __ldg(d.Kx + c + 1),
                         __ldg(d.Kx + c), uv[j + 1], uv[j + 2], uv[j], u[c + 1], u[c - 1]);
       rl[j] = __ldg(d.u0 + c) - wl[j];
       pl[j] = p[c];
@@ -602,7 +608,7 @@ __global__ void __launch_bounds__(kBlock, MB)
     for (int j = 0; j < 4; j++)
       if (j < rows) {
         const long long c = c0 + j * S;
-        const double b = emu_dmul(dia ? emu_dmul(beta, mv[j]) : beta, rl[j]);
+        const double b = mul_e<EMU>(dia ? mul_e<EMU>(beta, mv[j]) : beta, rl[j]);
         const double pn = F ? __fma_rn(alpha, pl[j], b) : alpha * pl[j] + b;
         w[c] = wl[j];
         r[c] = rl[j];
@@ -922,7 +928,7 @@ __global__ void __launch_bounds__(kBlock, 3)
 // calc_sd; the products run on the integer pipes (bit-identical).  Rows past
 // the interior are clamped to the halo row, so every load is issued before the
 // first use; the values of such rows are not stored.
-template <int F, int MB>
+template <int F, int MB, bool EMU>
 __global__ void __launch_bounds__(kBlock, MB)
     k_ppcg_step_point(Dev d, Red red, double alpha, double beta, const ResState* st,
                       const double* sdi_, double* sdo_) {
@@ -946,7 +952,7 @@ __global__ void __launch_bounds__(kBlock, MB)
     for (int j = 0; j < 4; j++) {
       const long long c = c0 + min(j, rows - 1) * S;
       uv[j] = u[c] + sv[j + 1];
-      rv[j] = bms_v<F>(r[c], __ldg(d.diag + c), kyv[j + 1], kyv[j], __ldg(d.Kx + c + 1),
+      rv[j] = bms_v<F, EMU>(r[c], __ldg(d.diag + c), kyv[j + 1], kyv[j], __ldg(d.Kx + c + 1),
                        __ldg(d.Kx + c), sv[j + 1], sv[j + 2], sv[j], sdi[c + 1], sdi[c - 1]);
       mv[j] = dia ? __ldg(d.Mi + c) : 0.0;
     }
@@ -954,8 +960,8 @@ __global__ void __launch_bounds__(kBlock, MB)
     for (int j = 0; j < 4; j++)
       if (j < rows) {
         const long long c = c0 + j * S;
-        double b = emu_dmul(beta, rv[j]);
-        if (dia) b = emu_dmul(b, mv[j]);
+        double b = mul_e<EMU>(beta, rv[j]);
+        if (dia) b = mul_e<EMU>(b, mv[j]);
         u[c] = uv[j];
         r[c] = rv[j];
         sdo[c] = F ? __fma_rn(alpha, sv[j + 1], b) : alpha * sv[j + 1] + b;
@@ -1184,15 +1190,10 @@ void launch_cheby_calc_pu(Chunk& c, double alpha, double beta, double* un) {
   if (c.prec != PREC_JAC_BLOCK) {
     const Dev d4 = dev4(c);
     const char* name = "tea_leaf_cheby_solve_calc_p_u";
-    if (c.arith == 2)
-      point_blocks4(c) ? launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<2, 4>, d4, c.red(), alpha, beta, un)
-                       : launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<2, 3>, d4, c.red(), alpha, beta, un);
-    else if (c.arith == 1)
-      point_blocks4(c) ? launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<1, 4>, d4, c.red(), alpha, beta, un)
-                       : launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<1, 3>, d4, c.red(), alpha, beta, un);
-    else
-      point_blocks4(c) ? launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<0, 4>, d4, c.red(), alpha, beta, un)
-                       : launch_tile_ns(c, name, d4.ns, k_cheby_calc_pu_point<0, 3>, d4, c.red(), alpha, beta, un);
+    auto* const kernel = c.arith == 2   ? TEA_POINT(k_cheby_calc_pu_point, 2, c)
+                         : c.arith == 1 ? TEA_POINT(k_cheby_calc_pu_point, 1, c)
+                                        : TEA_POINT(k_cheby_calc_pu_point, 0, c);
+    launch_tile_ns(c, name, d4.ns, kernel, d4, c.red(), alpha, beta, un);
     return;
   }
   TH_DISPATCH(c, "tea_leaf_cheby_solve_calc_p_u", k_cheby_calc_pu_block, c.dev(), c.red(),
@@ -1213,21 +1214,10 @@ void launch_ppcg_step(Chunk& c, double alpha, double beta, const double* sdi, do
   const char* name = "tea_leaf_ppcg_solve_inner_step";
   const ResState* st = nullptr;
   if (c.prec != PREC_JAC_BLOCK) {
-    if (c.arith == 2)
-      point_blocks4(c) ? launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<2, 4>, d4, c.red(), alpha, beta, st,
-                                        sdi, sdo)
-                       : launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<2, 3>, d4, c.red(), alpha, beta, st,
-                                        sdi, sdo);
-    else if (c.arith == 1)
-      point_blocks4(c) ? launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<1, 4>, d4, c.red(), alpha, beta, st,
-                                        sdi, sdo)
-                       : launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<1, 3>, d4, c.red(), alpha, beta, st,
-                                        sdi, sdo);
-    else
-      point_blocks4(c) ? launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<0, 4>, d4, c.red(), alpha, beta, st,
-                                        sdi, sdo)
-                       : launch_tile_ns(c, name, d4.ns, k_ppcg_step_point<0, 3>, d4, c.red(), alpha, beta, st,
-                                        sdi, sdo);
+    auto* const kernel = c.arith == 2   ? TEA_POINT(k_ppcg_step_point, 2, c)
+                         : c.arith == 1 ? TEA_POINT(k_ppcg_step_point, 1, c)
+                                        : TEA_POINT(k_ppcg_step_point, 0, c);
+    launch_tile_ns(c, name, d4.ns, kernel, d4, c.red(), alpha, beta, st, sdi, sdo);
     return;
   }
   if (c.arith == 2)
@@ -1494,9 +1484,7 @@ static void enqueue_ppcg_iterations_t(Chunk& c, int iters) {
   const bool blk = c.prec == PREC_JAC_BLOCK;
   const int gs = blk ? tile_grid(c, k_ppcg_calc_sd_block<F>, sd_blocks(d4))
                      : tile_grid(c, k_ppcg_sd<4, F>, d4.ns);
-  auto* const step = blk              ? k_ppcg_step<F>
-                     : point_blocks4(c) ? k_ppcg_step_point<F, 4>
-                                        : k_ppcg_step_point<F, 3>;
+  auto* const step = blk ? k_ppcg_step<F> : TEA_POINT(k_ppcg_step_point, F, c);
   const int gst = tile_grid(c, step, d4.ns);
   // inner steps two at a time in one pass each, the first writing sd to the
   // second buffer and the second back, so each outer iteration ends with sd
