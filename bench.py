@@ -427,14 +427,13 @@ KERNEL_BYTES = {
     "tea_leaf_ppcg_solve_calc_sd": {"jac_diag": 32, "jac_block": 56, "none": 24},
     "tea_leaf_cheby_solve_calc_p": {"jac_diag": 80, "jac_block": 96, "none": 72},
     "tea_leaf_cheby_solve_calc_u": 24,
-    # calc_p and calc_u in one pass (block Jacobi): calc_p's fields and u written
+    # calc_p and calc_u in one pass: calc_p's fields and u written
     "tea_leaf_cheby_solve_calc_p_u": {"jac_diag": 88, "jac_block": 104, "none": 80},
     "tea_leaf_calc_residual": 48,         # u0 u Kx Ky (diag), r
     "tea_leaf_cg_solve_init_p": {"jac_diag": 32, "jac_block": 56, "none": 24},
     "tea_leaf_ppcg_solve_init_sd": {"jac_diag": 24, "jac_block": 48, "none": 16},
     "tea_leaf_cheby_solve_init_p": {"jac_diag": 72, "jac_block": 88, "none": 64},
-    "tea_leaf_jacobi_copy_u": 16,         # u, un
-    "tea_leaf_jacobi_solve": 48,          # u0 un Kx Ky, u
+    "tea_leaf_jacobi_solve": 64,          # copy_u and solve in one pass: u, un; u0 un Kx Ky, u
     "tea_leaf_finalise": 24,              # u density, energy1
     "field_summary": 32,                  # volume density energy1 u
     "tea_leaf_init_common": 24,           # density, Kx Ky
