@@ -257,11 +257,16 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
 // ---- the two passes as separate kernels, for grids whose passes are long
 // beside a launch (replayed from a graph) ----
 
+// Blocks per SM by measurement.  Pass A at 128 registers: 391 us per iteration
+// at 4096^2 diagonal, 474 and 504 at three and four blocks; pass B streams at
+// four (392, 412 at three, two).  The exact form's pass B needs more registers
+// (its strip divides): three blocks, 3000^2 block Jacobi 468 -> 458 us.
+
 // Pass A.  An iteration whose predecessor has run (p_pending) forms p' and
 // finishes u; the first one copies p, so that p alternates between the two
 // buffers whatever happens.
 template <int TH, int F>
-__global__ void __launch_bounds__(kBlock, 2)
+__global__ void __launch_bounds__(kBlock, F || TH == 16 ? 2 : 3)
     k_cg_pass_w(Dev d, Red red, ResState* st, const double* pin, double* pout) {
   if (*(volatile int*)&st->stop) return;
   const bool first = !*(volatile int*)&st->p_pending;
@@ -280,7 +285,7 @@ __global__ void __launch_bounds__(kBlock, 2)
 // Pass B and the scalar step; with NV = 2 also r.r for the exit test on the
 // unpreconditioned residual.
 template <int TH, int F, int NV>
-__global__ void __launch_bounds__(kBlock, 4) k_cg_pass_r(Dev d, Red red, ResState* st) {
+__global__ void __launch_bounds__(kBlock, F ? 4 : 3) k_cg_pass_r(Dev d, Red red, ResState* st) {
   if (*(volatile int*)&st->stop) return;
   const double alpha = st->alpha;
   const bool last = tile_driver<TH, NV>(d, red, [&](int x, int y0, bool, double* acc) {
