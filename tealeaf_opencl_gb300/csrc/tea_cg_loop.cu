@@ -22,7 +22,15 @@ namespace tea {
 
 namespace {
 
-constexpr int kLoopThreads = 512;               // one block per SM, 128 registers
+// One block of 512 threads with 128 registers per SM: four rows of a tile's 33
+// loads are in flight at once, and 16 warps keep the FP64 pipe busy while some
+// wait (1024 threads with 64 registers, row by row: 480 us per iteration at
+// 4096^2 against 417, 18.8 against 16.4 at 512^2 in the same state of the
+// kernel).  Small grids are bound by latency: of 31 thousand cycles per
+// iteration at 512^2 pass A takes 14, pass B 6, the two barriers and sums 11.
+// Middle ones by the FP64 pipe, 59 % busy at 1501x1203 block Jacobi (the last
+// round of supertiles is half full, and all loads of a round start together).
+constexpr int kLoopThreads = 512;
 constexpr int kLoopWarps = kLoopThreads / 32;
 constexpr int kLoopSlots = kLoopWarps / kTilesPerSuper;  // supertiles in flight
 constexpr int kLoopBatch = 4;                   // rounds whose tile sums share a sweep

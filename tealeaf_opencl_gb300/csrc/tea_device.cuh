@@ -123,7 +123,7 @@ __device__ __forceinline__ double bms_v(double b, double D, double kyn, double k
 // The same operator at offset c of the padded fields, written out with the
 // loads in place (the kernels' register budgets were tuned on this form);
 // its arithmetic is smvp_v's.
-template <int F, bool CG = false, bool EMU = true>
+template <int F, bool EMU = true>
 __device__ __forceinline__ double smvp(const Dev& d, const double* x,
                                        long long c) {
   const long long S = d.S;
@@ -131,19 +131,19 @@ __device__ __forceinline__ double smvp(const Dev& d, const double* x,
   const double kxe = __ldg(d.Kx + c + 1), kxc = __ldg(d.Kx + c);
   const double D = __ldg(d.diag + c);
   if (!F)
-    return D * ldv<CG>(x + c) -
-           (mul_e<EMU>(kyn, ldv<CG>(x + c + S)) + kyc * ldv<CG>(x + c - S)) -
-           (mul_e<EMU>(kxe, ldv<CG>(x + c + 1)) + kxc * ldv<CG>(x + c - 1));
+    return D * x[c] -
+           (mul_e<EMU>(kyn, x[c + S]) + kyc * x[c - S]) -
+           (mul_e<EMU>(kxe, x[c + 1]) + kxc * x[c - 1]);
   if (F == 2) {
-    double t = mul_e<EMU>(D, ldv<CG>(x + c));
-    t = __fma_rn(-kyn, ldv<CG>(x + c + S), t);
-    t = __fma_rn(-kyc, ldv<CG>(x + c - S), t);
-    t = __fma_rn(-kxe, ldv<CG>(x + c + 1), t);
-    return __fma_rn(-kxc, ldv<CG>(x + c - 1), t);
+    double t = mul_e<EMU>(D, x[c]);
+    t = __fma_rn(-kyn, x[c + S], t);
+    t = __fma_rn(-kyc, x[c - S], t);
+    t = __fma_rn(-kxe, x[c + 1], t);
+    return __fma_rn(-kxc, x[c - 1], t);
   }
-  const double t1 = __fma_rn(kyc, ldv<CG>(x + c - S), mul_e<EMU>(kyn, ldv<CG>(x + c + S)));
-  const double t2 = __fma_rn(kxc, ldv<CG>(x + c - 1), mul_e<EMU>(kxe, ldv<CG>(x + c + 1)));
-  return __fma_rn(D, ldv<CG>(x + c), -t1) - t2;
+  const double t1 = __fma_rn(kyc, x[c - S], mul_e<EMU>(kyn, x[c + S]));
+  const double t2 = __fma_rn(kxc, x[c - 1], mul_e<EMU>(kxe, x[c + 1]));
+  return __fma_rn(D, x[c], -t1) - t2;
 }
 
 // b - A x at offset c (the arithmetic of bms_v)

@@ -538,7 +538,7 @@ __device__ __forceinline__ void cheby_block_body(const Dev& d, const Red& red, d
       for (int i = 0; i < 4; i++) {
         if (ys + i < d.y_max) {
           const long long c = c0 + i * d.S;
-          wl[i] = smvp<F, false, false>(d, d.u, c);
+          wl[i] = smvp<F, false>(d, d.u, c);
           ul[i] = d.u[c];
           rl[i] = d.u0[c] - wl[i];
           pl[i] = d.p[c];
@@ -633,7 +633,7 @@ __global__ void __launch_bounds__(kBlock) k_cheby_init_p(Dev d, Red red, DivCons
       for (int i = 0; i < 4; i++) {
         if (g + i < d.y_max) {
           const long long c = c0 + i * d.S;
-          wl[i] = smvp<F, false, false>(d, d.u, c);
+          wl[i] = smvp<F, false>(d, d.u, c);
           rl[i] = d.u0[c] - wl[i];
           zl[i] = d.prec == PREC_JAC_DIAG ? d.Mi[c] * rl[i] : rl[i];
         }
