@@ -158,7 +158,8 @@ struct Chunk {
   cudaGraphExec_t res_graph = nullptr;
   int res_graph_iters = 0;
   bool res_graph_true_exit = false;
-  int res_graph_epoch = 0;  // field_epoch the CG graph was captured at
+  int res_graph_epoch = 0;  // field_epoch and arithmetic form the CG graph was captured at
+  int res_graph_arith = 0;
   double res_last_rr_true = 0.0;
 
   Dev dev() const;

@@ -1587,7 +1587,8 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
   Chunk& c = chunk();
   flush_pending_inner(c);
   if (c.res_graph &&
-      (c.res_graph_true_exit != true_exit || c.res_graph_epoch != c.field_epoch)) {
+      (c.res_graph_true_exit != true_exit || c.res_graph_epoch != c.field_epoch ||
+       c.res_graph_arith != c.arith)) {
     cudaGraphExecDestroy(c.res_graph);
     c.res_graph = nullptr;
   }
@@ -1652,6 +1653,7 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
     c.res_graph_iters = batch;
     c.res_graph_true_exit = true_exit;
     c.res_graph_epoch = c.field_epoch;
+    c.res_graph_arith = c.arith;
   }
   // every batch runs at least one iteration until the loop stops, so the
   // loop needs at most this many batches; more means the state is corrupt
