@@ -17,6 +17,7 @@
 #include "tea_cg.cuh"
 #include "tea_device.cuh"
 #include "tea_loop.cuh"
+#include "tea_resident_launch.h"
 
 namespace tea {
 
@@ -353,10 +354,16 @@ void enqueue_passes_t(const LaunchCtx& l, const Dev& d, double* p2, const Red& r
   k_cg_pass_end<TH, F><<<ge, kBlock, 0, l.stream>>>(d, red, st, p2, counter);
 }
 
+// A loop kernel on a block per SM, or per supertile where there are fewer.
+cudaError_t launch_loop_blocks(const LaunchCtx& l, const Dev& d, const void* fn, void** args) {
+  return launch_resident(std::max(1, std::min(d.ns, l.num_sms)), [&](int blocks) {
+    return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kLoopThreads), args, 0, l.stream);
+  });
+}
+
 template <int TH, int F>
 bool launch_loop_t(const LaunchCtx& l, Dev d, double* p2, Red red, ResState* st,
                    unsigned int* bar, long long spin_limit, unsigned int extra, int iters) {
-  int grid = std::max(1, std::min(d.ns, l.num_sms));
   int* err = (int*)(bar + 1);
   void* args[] = {&d, &p2, &red, &st, &bar, &err, &spin_limit, &extra, &iters};
   const void* fn = (const void*)k_cg_loop<TH, F, true>;
@@ -364,9 +371,7 @@ bool launch_loop_t(const LaunchCtx& l, Dev d, double* p2, Red red, ResState* st,
     if (few_supertiles(d, l.num_sms)) fn = (const void*)k_cg_loop<TH, F, false>;
   return check_cuda(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned int), l.stream),
                     "CG loop barrier reset") &&
-         check_cuda(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kLoopThreads), args, 0,
-                                                l.stream),
-                    "CG loop launch");
+         check_cuda(launch_loop_blocks(l, d, fn, args), "CG loop launch");
 }
 
 }  // namespace
@@ -376,7 +381,7 @@ bool launch_jacobi_loop(const LaunchCtx& l, const Dev& d_, double* u2, const Red
                         unsigned int extra) {
   Dev d = d_;
   Red red = red_;
-  int grid = std::max(1, std::min(d.ns, l.num_sms)), iters = kLoopLaunchIters;
+  int iters = kLoopLaunchIters;
   int* err = (int*)(bar + 1);
   void* args[] = {&d, &u2, &red, &st, &bar, &err, &spin_limit, &extra, &iters};
   const void* fn = d.th == 16                    ? (const void*)k_jacobi_loop<16, true>
@@ -385,9 +390,7 @@ bool launch_jacobi_loop(const LaunchCtx& l, const Dev& d_, double* u2, const Red
   count_launch("resident_jacobi_loop");
   return check_cuda(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned int), l.stream),
                     "Jacobi loop barrier reset") &&
-         check_cuda(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kLoopThreads), args, 0,
-                                                l.stream),
-                    "Jacobi loop launch");
+         check_cuda(launch_loop_blocks(l, d, fn, args), "Jacobi loop launch");
 }
 
 // The line between the two: a launch boundary costs a pass about 10 us (start,

@@ -32,6 +32,7 @@
 #include "../../include/tealeaf_gb300.h"
 #include "tea_device.cuh"
 #include "tea_loop.cuh"
+#include "tea_resident_launch.h"
 
 namespace tea {
 
@@ -981,14 +982,17 @@ static bool run_inner_loop(Chunk& c, MixState& h) {
   int* err = (int*)(g.counter + 2);
   long long spins = c.barrier_spin_limit;
   int iters = kLoopLaunchIters;
-  const int grid = std::max(1, std::min(d.ns, c.num_sms));
   void* args[] = {&d, &m, &red, &g.st, &bar, &err, &spins, &iters};
   const long long launches = (long long)(h.max_iters - h.n) / iters + 2;
   for (long long k = 0;; k++) {
     if (!check_cuda(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned int), c.stream),
                     "mixed barrier reset") ||
-        !check_cuda(cudaLaunchCooperativeKernel((const void*)k_mix_loop<TH>, dim3(grid),
-                                                dim3(kMixThreads), args, 0, c.stream),
+        !check_cuda(launch_resident(std::max(1, std::min(d.ns, c.num_sms)),
+                                    [&](int blocks) {
+                                      return cudaLaunchCooperativeKernel(
+                                          (const void*)k_mix_loop<TH>, dim3(blocks),
+                                          dim3(kMixThreads), args, 0, c.stream);
+                                    }),
                     "mixed loop launch"))
       return false;
     count_launches(1);
