@@ -226,10 +226,11 @@ int tea_gb300_get_arithmetic(void);
  * Results are identical either way.  Applies to the current chunk and later
  * ones.  Returns 0, or -1 for another value. */
 int tea_gb300_set_inner_pairs(int on);
-/* The grid barrier of the one-launch resident loops (CG, Jacobi and the mixed
- * solve's inner loop): a block polls at most spin_limit times (default 2^26,
- * about 10 s) before it gives up, sets the
- * loop's error flag and returns; the call then fails with error 25.
+/* The grid barrier of the one-launch loops (resident CG and Jacobi, the mixed
+ * solve's inner loop, the adjoint's solves, the batch's persistent mode): a
+ * block polls at most spin_limit times (default 2^26, seconds) before it gives
+ * up, sets the loop's error flag and returns; the call then fails with error
+ * 25, in the adjoint 61, in the batch 57.
  * extra_arrivals = 1 makes the barrier wait for one block more than the
  * grid has, so the wait always runs out: the test of that path uses it with
  * a short limit.  Use 2^26 and 0 for normal runs.  Returns 0 or -1. */

@@ -220,7 +220,9 @@ long long solve(Adjoint& a, double eps, int max_iters) {
       return -1;
     }
     if (loop) {
-      if (!launch_cg_loop(l, a.d, a.p2, a.red, a.st, a.counters + 2, kLoopSpins, 0)) return -1;
+      if (!launch_cg_loop(l, a.d, a.p2, a.red, a.st, a.counters + 2, chunk().barrier_spin_limit,
+                          (unsigned int)chunk().barrier_extra))
+        return -1;
     } else {
       if (!check_cuda(cudaGraphLaunch(a.graph, a.stream), "adjoint replay")) return -1;
       count_launches(2 * kReplayIters + 1);

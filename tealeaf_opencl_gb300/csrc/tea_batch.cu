@@ -269,15 +269,15 @@ template <int F>
 __global__ void __launch_bounds__(kBlock, 2)
     k_b_iterations(const Dev* __restrict__ devs, const Red* __restrict__ reds,
                    double* const* __restrict__ p2s, ResState* st, WorkList wl, int iters,
-                   unsigned int* bar, long long spin_limit) {
+                   unsigned int* bar, long long spin_limit, unsigned int extra) {
   __shared__ BatchShared sh;
   int* err = (int*)(bar + 2);
   const int U = wl.counts[0], np = wl.counts[1];
   for (int it = 0; it < iters; it++) {
     phase_w<F>(devs, reds, p2s, st, wl, U, np, sh);
-    if (!grid_barrier(bar, err, spin_limit)) return;
+    if (!grid_barrier(bar, err, spin_limit, extra)) return;
     phase_r<F>(devs, reds, st, wl, U, np, sh);
-    if (!grid_barrier(bar, err, spin_limit)) return;
+    if (!grid_barrier(bar, err, spin_limit, extra)) return;
   }
 }
 
@@ -446,6 +446,8 @@ struct Batch {
   int occ_persistent[3] = {};  // [arithmetic form] k_b_iterations
   cudaGraphExec_t iter_graph = nullptr;
   int graph_bps = 0, graph_iters = 0, graph_G = 0, graph_persistent = 0;
+  long long graph_spins = 0;  // the barrier limits in it
+  int graph_extra = 0;
 };
 
 Batch g_batch;
@@ -909,9 +911,10 @@ void enqueue_persistent(Batch& b, const WorkList& wl, int iters, int bps) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const long long spin_limit = 1LL << 26;
   check_cuda(cudaLaunchKernelEx(&cfg, k_b_iterations<F>, (const Dev*)b.devs_d,
-                                (const Red*)b.reds_d, (double* const*)b.p2s_d, b.st_d, wl, iters, b.bar_d, spin_limit),
+                                (const Red*)b.reds_d, (double* const*)b.p2s_d, b.st_d, wl, iters,
+                                b.bar_d, chunk().barrier_spin_limit,
+                                (unsigned int)chunk().barrier_extra),
              "batch persistent launch");
 }
 
@@ -1001,7 +1004,9 @@ extern "C" int tea_gb300_batch_run(int steps, double dt, double eps, int max_ite
   const int gi = b.launch.graph_iterations;
   if (b.iter_graph && (b.graph_bps != bps || b.graph_iters != gi ||
                        b.graph_G != b.launch.supertiles_per_unit ||
-                       b.graph_persistent != b.launch.persistent)) {
+                       b.graph_persistent != b.launch.persistent ||
+                       b.graph_spins != chunk().barrier_spin_limit ||
+                       b.graph_extra != chunk().barrier_extra)) {
     cudaGraphExecDestroy(b.iter_graph);
     b.iter_graph = nullptr;
   }
@@ -1013,6 +1018,8 @@ extern "C" int tea_gb300_batch_run(int steps, double dt, double eps, int max_ite
     b.graph_iters = gi;
     b.graph_G = b.launch.supertiles_per_unit;
     b.graph_persistent = b.launch.persistent;
+    b.graph_spins = chunk().barrier_spin_limit;
+    b.graph_extra = chunk().barrier_extra;
   }
   per_replay = b.launch.persistent ? 3 : 2 * gi + 2;
   b.counts_h[2] = 0;

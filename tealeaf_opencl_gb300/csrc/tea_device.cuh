@@ -337,16 +337,13 @@ __device__ __forceinline__ void block_final_sum(const double* partials,
 // Barrier across every block of a cooperative launch (all blocks resident).
 // bar[0] counts arrivals, bar[1] is the generation.  Every thread's earlier
 // global writes are visible to every block after it.  A block waits at most
-// spin_limit polls (kBarrierSpins, about 4 s, unless the caller sets
-// another); on time-out, or when another block has timed out, it sets *err
-// and returns false, and the kernel must return.  The barrier opens when
+// spin_limit polls; on time-out, or when another block has timed out, it sets
+// *err and returns false, and the kernel must return.  The barrier opens when
 // gridDim.x + extra blocks have arrived: extra is 0, except in the test that
 // makes the wait run out (one arrival more than the grid has, so no block
 // opens it).
-constexpr long long kBarrierSpins = 1LL << 26;
 __device__ __forceinline__ bool grid_barrier(unsigned int* bar, int* err,
-                                             long long spin_limit = kBarrierSpins,
-                                             unsigned int extra = 0) {
+                                             long long spin_limit, unsigned int extra) {
   __shared__ int ok;
   __threadfence();
   __syncthreads();

@@ -247,7 +247,6 @@ void dev_cg_init_p(const LaunchCtx& l, const Dev& d, const Red& r);
 // flag (also in st->timed_out); red.partials holds at least two arrays of red.stride.  After it
 // st->stop is set, or the loop goes on with another launch.
 constexpr int kLoopLaunchIters = 1024;
-constexpr long long kLoopSpins = 1LL << 26;  // polls of a barrier before it gives up
 // At most one supertile per SM: few warps share an SM's FP64 pipe, and a
 // product there (64 cycles) is quicker than on the integer pipes (224, 45
 // instructions).  The CG loop then takes 6.6 us per iteration at 64^2 against

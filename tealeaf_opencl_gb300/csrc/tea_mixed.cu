@@ -574,10 +574,11 @@ __device__ __forceinline__ void mix_pass(const Dev& d, double* partials, MixShar
 template <int TH>
 __global__ void __launch_bounds__(kMixThreads, 1)
     k_mix_loop(Dev d, MixDev m, Red red, MixState* st, unsigned int* bar, int* err,
-               long long spin_limit, int iters) {
+               long long spin_limit, unsigned int extra, int iters) {
   __shared__ MixShared sh;
   double* const pw_parts = red.partials;
   double* const rz_parts = red.partials + red.stride;
+  const unsigned int arrivals = gridDim.x + extra;
   unsigned int target = 0;
   double rro = st->rro;  // kept up to date by thread 0
   const double eps2 = st->eps2;
@@ -591,7 +592,7 @@ __global__ void __launch_bounds__(kMixThreads, 1)
     mix_pass<TH>(d, pw_parts, sh, [&](int x, int y0, double* v) {
       mix_pw_body<TH, true>(d, m, pin, pout, pend, bf, x, y0, v);
     });
-    target += gridDim.x;
+    target += arrivals;
     if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, &sh.go)) return;
     const double pw = loop_total(pw_parts, d.ns, sh.lanes, sh.tiles);
     if (threadIdx.x == 0) sh.alpha = rro / pw;
@@ -601,7 +602,7 @@ __global__ void __launch_bounds__(kMixThreads, 1)
     mix_pass<TH>(d, rz_parts, sh, [&](int x, int y0, double* v) {
       mix_ur_body<TH>(d, m, pout, af, x, y0, v);
     });
-    target += gridDim.x;
+    target += arrivals;
     if (!loop_barrier(bar, err, &st->timed_out, target, spin_limit, &sh.go)) return;
     const double rrn = loop_total(rz_parts, d.ns, sh.lanes, sh.tiles);
     if (threadIdx.x == 0) {
@@ -981,8 +982,9 @@ static bool run_inner_loop(Chunk& c, MixState& h) {
   unsigned int* bar = g.counter + 1;
   int* err = (int*)(g.counter + 2);
   long long spins = c.barrier_spin_limit;
+  unsigned int extra = (unsigned int)c.barrier_extra;
   int iters = kLoopLaunchIters;
-  void* args[] = {&d, &m, &red, &g.st, &bar, &err, &spins, &iters};
+  void* args[] = {&d, &m, &red, &g.st, &bar, &err, &spins, &extra, &iters};
   const long long launches = (long long)(h.max_iters - h.n) / iters + 2;
   for (long long k = 0;; k++) {
     if (!check_cuda(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned int), c.stream),
