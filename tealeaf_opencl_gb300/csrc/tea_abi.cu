@@ -98,6 +98,8 @@ static bool timed_match(const char* name) {
   return !g_timed_name.empty() && (g_timed_name == "*" || g_timed_name == name);
 }
 
+bool kernels_timed() { return chunk().profiler_on || !g_timed_name.empty(); }
+
 void profile_begin(const char* name) {
   Chunk& c = chunk();
   if (timed_match(name)) {

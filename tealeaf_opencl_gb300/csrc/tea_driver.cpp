@@ -723,11 +723,13 @@ class Driver {
         }
         cheby_calc_steps++;
       } else if (use_cg || use_cheby || use_ppcg) {
-        if (mode == TEA_DRIVER_RESIDENT && (use_cg || !D.verbose)) {
+        if (mode == TEA_DRIVER_RESIDENT &&
+            (use_cg || (!D.verbose && !tea::kernels_timed()))) {
           // The whole remaining CG loop, or the CG iterations before the
           // switch to Chebyshev or PPCG, on the device; it stops exactly
           // where this loop would (same tests, same arithmetic).  PPCG
           // switches after one iteration once the eigenvalues are known.
+          // While kernels are timed the latter stay the separate kernels.
           int n_done = 0, conv = 0;
           tea::chunk().solver_checks = checks & TEA_CHECK_BREAKDOWN;
           const bool one = use_ppcg && !first;
@@ -760,7 +762,7 @@ class Driver {
         error = rrn;
         rro = rrn;
       } else if (use_jacobi && mode == TEA_DRIVER_RESIDENT && !D.verbose &&
-                 !(checks & TEA_CHECK_BREAKDOWN) &&
+                 !(checks & TEA_CHECK_BREAKDOWN) && !tea::kernels_timed() &&
                  tea::cg_loop_fits(tea::chunk().dev(), tea::chunk().num_sms)) {
         // us per sweep, per call / on the device: 64^2 16.0 / 9.3, 512^2 20.9 /
         // 14.3, 1024^2 47.8 / 40.1, 2048^2 146 / 153

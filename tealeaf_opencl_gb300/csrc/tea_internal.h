@@ -177,6 +177,8 @@ void count_launch(const char* name);
 void count_launches(long long n);  // n kernels run from a graph replay
 void profile_begin(const char* name);
 void profile_end(const char* name);
+// true while the profiler or a kernel timer is on (it sees separate launches only)
+bool kernels_timed();
 
 int reduction_rows(int x_max, int y_max);
 
