@@ -211,7 +211,7 @@ long long solve(Adjoint& a, double eps, int max_iters) {
   dev_cg_init_p(l, a.d, a.red);
   k_adj_begin<<<1, 1, 0, a.stream>>>(a.st, a.red.result, eps, max_iters);
   count_launch("adjoint_begin");
-  const bool loop = cg_loop_fits(a.d, a.num_sms);
+  const bool loop = cg_loop_fits(a.d, a.num_sms, a.arith);
   const int per_launch = loop ? kLoopLaunchIters : kReplayIters;
   const long long max_launches = (long long)max_iters / per_launch + 3;
   for (long long nb = 0;; nb++) {
@@ -345,7 +345,7 @@ extern "C" int tea_gb300_adjoint_create(int x_cells, int y_cells, double xmin,
   a.red.result = a.results;
   // the graph of kReplayIters resident CG iterations on these fields, for
   // grids beyond the one-launch loop
-  if (cg_loop_fits(a.d, a.num_sms)) {
+  if (cg_loop_fits(a.d, a.num_sms, a.arith)) {
     if (!check_cuda(cudaStreamSynchronize(a.stream), "adjoint create")) {
       release_adjoint();
       return -1;

@@ -214,10 +214,11 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
 // alternates between d.u and u2 (whose halo ring becomes u's), one grid barrier
 // per sweep, the old u of the last one into un.  A sweep through the per-call
 // path costs a launch and a host round trip, about 20 us on small grids.
-template <int TH, bool EMU>
+template <bool EMU>
 __global__ void __launch_bounds__(kLoopThreads, 1)
     k_jacobi_loop(Dev d, double* u2, Red red, ResState* st, unsigned int* bar, int* err,
                   long long spin_limit, unsigned int extra, int iters) {
+  constexpr int TH = 4;  // jacobi_loop_fits
   __shared__ LoopShared sh;
   const unsigned int arrivals = gridDim.x + extra;
   unsigned int target = 0;
@@ -384,27 +385,39 @@ bool launch_jacobi_loop(const LaunchCtx& l, const Dev& d_, double* u2, const Red
   int iters = kLoopLaunchIters;
   int* err = (int*)(bar + 1);
   void* args[] = {&d, &u2, &red, &st, &bar, &err, &spin_limit, &extra, &iters};
-  const void* fn = d.th == 16                    ? (const void*)k_jacobi_loop<16, true>
-                   : few_supertiles(d, l.num_sms) ? (const void*)k_jacobi_loop<4, false>
-                                                  : (const void*)k_jacobi_loop<4, true>;
+  const void* fn = few_supertiles(d, l.num_sms) ? (const void*)k_jacobi_loop<false>
+                                                : (const void*)k_jacobi_loop<true>;
   count_launch("resident_jacobi_loop");
   return check_cuda(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned int), l.stream),
                     "Jacobi loop barrier reset") &&
          check_cuda(launch_loop_blocks(l, d, fn, args), "Jacobi loop launch");
 }
 
-// The line between the two: a launch boundary costs a pass about 10 us (start,
-// drain, the last block's sum), a grid barrier with the sum in every block
-// about 3.5 us; but the cooperative kernel's passes share one register budget
-// (16 warps per SM), so pass B of long passes streams at 0.8 of the rate of its
-// own kernel.  us per iteration, cooperative / graph (three kernels per
-// iteration before them): 64^2 7.3 / 9.9 (11.7), 512^2 diagonal 15.3 / 21.6
-// (25.1), 960^2 33.0 / 38.9 (43.5), 1024^2 diagonal 34.7 / 39.7 (47.4),
-// 1501x1203 block 67.4 / 69.8 (71.8), 1700^2 diagonal 103 / 98, 2048^2
-// diagonal 134 / 121 (125), 4096^2 diagonal 419 / 391 (425), block 466 / 440
-// (463).  They cross between 12 and 20 supertiles per SM.
-constexpr int kLoopSupertilesPerSM = 14;
-bool cg_loop_fits(const Dev& d, int num_sms) { return d.ns <= kLoopSupertilesPerSM * num_sms; }
+// The line between the one launch and separate kernels, in supertiles of 4 rows
+// per SM (one of 16 rows is the work of four).  A launch boundary costs a pass
+// 8-10 us (start, drain, the last block's sum), a grid barrier with the sum in
+// every block 2.5 us; but the cooperative kernel's passes share one register
+// budget (16 warps per SM), so long passes run at 0.8-0.95 of the rate of their
+// own kernels.  us per CG iteration, graph / one launch, at 1501 columns:
+//   per SM                  7.9         9.9         10.4        11.9        13.9        14.9
+//   diagonal, fused     43.7 / 40.5 55.2 / 55.2 59.1 / 61.6 64.6 / 65.7 71.6 / 74.3 76.1 / 81.3
+//   block, fused        49.6 / 45.1 61.4 / 60.2 65.2 / 67.3 71.5 / 71.9 79.4 / 81.6 85.2 / 89.1
+//   none, fused         41.7 / 36.6 51.2 / 47.1 55.4 / 52.8 61.6 / 59.1 68.8 / 68.5 72.9 / 75.1
+//   block, exact form   81.1 / 70.2 96.4 / 90.3 98.4 / 99.7  109 / 107   130 / 122   133 / 132
+// (the exact form's strip divides keep both forms on the FP64 pipe).  In 16-row
+// tiles, 32 per SM and more, the graph is ahead throughout: diagonal fused 2176^2
+// 143 / 149, 2500^2 172 / 186, 2800^2 208 / 219.
+static int rows4_supertiles(const Dev& d) { return d.ns * (d.th / 4); }
+bool cg_loop_fits(const Dev& d, int num_sms, int arith) {
+  const int per_sm = arith != 0 && d.prec != PREC_NONE ? 10 : 14;
+  return rows4_supertiles(d) <= per_sm * num_sms;
+}
+
+// Jacobi: one barrier per sweep in place of a launch and a host round trip.  us
+// per sweep, per call / one launch: 64^2 16.0 / 9.3, 512^2 20.9 / 14.3; at 1501
+// columns 9.9 per SM 60.1 / 54.1, 13.9 79.9 / 73.1, 15.9 89.4 / 83.9, 17.9 99.9 /
+// 98.5; 1600^2 (18.4) 94.4 / 100.2, 2048^2 145 / 152, 2500^2 222 / 234.
+bool jacobi_loop_fits(const Dev& d, int num_sms) { return rows4_supertiles(d) <= 18 * num_sms; }
 
 void enqueue_cg_passes(const LaunchCtx& l, const Dev& d, double* p2, const Red& red,
                        ResState* st, unsigned int* counter, int iters, bool true_exit) {

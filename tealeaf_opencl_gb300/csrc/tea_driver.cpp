@@ -763,9 +763,7 @@ class Driver {
         rro = rrn;
       } else if (use_jacobi && mode == TEA_DRIVER_RESIDENT && !D.verbose &&
                  !(checks & TEA_CHECK_BREAKDOWN) && !tea::kernels_timed() &&
-                 tea::cg_loop_fits(tea::chunk().dev(), tea::chunk().num_sms)) {
-        // us per sweep, per call / on the device: 64^2 16.0 / 9.3, 512^2 20.9 /
-        // 14.3, 1024^2 47.8 / 40.1, 2048^2 146 / 153
+                 tea::jacobi_loop_fits(tea::chunk().dev(), tea::chunk().num_sms)) {
         int n_done = 0, conv = 0;
         if (tea::resident_jacobi_iterations(n, loop_max, D.eps * initial_residual, &error,
                                             &n_done, &conv) != 0)

@@ -256,10 +256,11 @@ constexpr int kLoopLaunchIters = 1024;
 // on some SMs (380^2) it is 15.0 against 14.4.
 inline bool few_supertiles(const Dev& d, int num_sms) { return d.th == 4 && d.ns <= num_sms; }
 // true where the one launch is the faster form (by size, tea_cg_loop.cu)
-bool cg_loop_fits(const Dev& d, int num_sms);
+bool cg_loop_fits(const Dev& d, int num_sms, int arith);
+bool jacobi_loop_fits(const Dev& d, int num_sms);
 bool launch_cg_loop(const LaunchCtx& l, const Dev& d, double* p2, const Red& red, ResState* st,
                     unsigned int* bar, long long spin_limit, unsigned int extra);
-// The same for Jacobi sweeps; u2: the second u buffer.  The result is in u2
+// The same for Jacobi sweeps on 4-row tiles; u2: the second u buffer.  The result is in u2
 // after an odd number of sweeps.
 bool launch_jacobi_loop(const LaunchCtx& l, const Dev& d, double* u2, const Red& red,
                         ResState* st, unsigned int* bar, long long spin_limit,

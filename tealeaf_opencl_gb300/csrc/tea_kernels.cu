@@ -1576,7 +1576,7 @@ static bool ensure_resident_state(Chunk& c) {
 
 static bool use_cg_loop(const Chunk& c, bool true_exit) {
   if (true_exit || c.profiler_on || c.resident_mode == 1) return false;
-  return c.resident_mode == 2 || cg_loop_fits(c.dev(), c.num_sms);
+  return c.resident_mode == 2 || cg_loop_fits(c.dev(), c.num_sms, c.arith);
 }
 
 int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
