@@ -155,11 +155,14 @@ struct Chunk {
   long long barrier_spin_limit = 1LL << 26;
   int barrier_extra = 0;
   int res_breakdown = 0, res_breakdown_n = 0;  // what the last one found
-  cudaGraphExec_t res_graph = nullptr;
-  int res_graph_iters = 0;
-  bool res_graph_true_exit = false;
-  int res_graph_epoch = 0;  // field_epoch and arithmetic form the CG graph was captured at
-  int res_graph_arith = 0;
+  // replays of CG passes, with what each was captured from: u has two buffers
+  // that Chebyshev iterations swap, so two are kept
+  struct CgGraph {
+    cudaGraphExec_t exec = nullptr;
+    const double *u = nullptr, *r = nullptr;
+    int arith = 0;
+    bool true_exit = false;
+  } res_graph[2];
   double res_last_rr_true = 0.0;
 
   Dev dev() const;

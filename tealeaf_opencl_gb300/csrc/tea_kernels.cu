@@ -1537,9 +1537,10 @@ static void enqueue_resident_iterations(Chunk& c, int iters, bool true_exit) {
 
 void resident_release() {
   Chunk& c = chunk();
-  if (c.res_graph) cudaGraphExecDestroy(c.res_graph);
-  c.res_graph = nullptr;
-  c.res_graph_iters = 0;
+  for (Chunk::CgGraph& g : c.res_graph) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g = Chunk::CgGraph();
+  }
   cudaFree(c.res_state);
   cudaFree(c.res_coef);
   cudaFree(c.res_counter);
@@ -1556,13 +1557,6 @@ void resident_release() {
   c.res_coef_n = 0;
 }
 
-// CG iterations n_begin..loop_max of tea_solve.f90:147-332 with all scalars
-// on the device (tea_cg_loop.cu): the whole loop as one cooperative launch, or
-// batches of iterations, two kernels each, replayed from a captured graph with
-// one read of the loop state per batch.  Kernels queued after the loop has
-// stopped return at once.  The arithmetic and the exit test are those of the
-// per-call path, so the results are bit-identical to it.  The true-residual
-// exit (r.r beside r.z) and profiling use the kernels.
 static bool ensure_resident_state(Chunk& c) {
   if (c.res_state) return true;
   if (!check_cuda(cudaMalloc(&c.res_state, sizeof(ResState)), "cudaMalloc state") ||
@@ -1574,11 +1568,45 @@ static bool ensure_resident_state(Chunk& c) {
   return true;
 }
 
+constexpr int kGraphIters = 16;  // iterations of one graph replay (even)
+
+// The graph of kGraphIters iterations on the current buffers in the current
+// form, captured unless one of the two kept is that (one per buffer of u).
+static cudaGraphExec_t cg_graph(Chunk& c, bool true_exit) {
+  for (Chunk::CgGraph& g : c.res_graph)
+    if (g.exec && g.u == c.u.f && g.r == c.r.f && g.arith == c.arith && g.true_exit == true_exit)
+      return g.exec;
+  Chunk::CgGraph& g = c.res_graph[c.res_graph[0].exec && c.res_graph[0].u != c.u.f ? 1 : 0];
+  if (g.exec) cudaGraphExecDestroy(g.exec);
+  g = Chunk::CgGraph();
+  cudaGraph_t graph = nullptr;
+  if (!check_cuda(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal),
+                  "graph capture"))
+    return nullptr;
+  enqueue_resident_iterations(c, kGraphIters, true_exit);
+  if (!check_cuda(cudaStreamEndCapture(c.stream, &graph), "graph capture end")) return nullptr;
+  const bool ok = check_cuda(cudaGraphInstantiate(&g.exec, graph, 0), "graph instantiate");
+  cudaGraphDestroy(graph);
+  if (!ok) g.exec = nullptr;
+  g.u = c.u.f;
+  g.r = c.r.f;
+  g.arith = c.arith;
+  g.true_exit = true_exit;
+  return g.exec;
+}
+
 static bool use_cg_loop(const Chunk& c, bool true_exit) {
   if (true_exit || c.profiler_on || c.resident_mode == 1) return false;
   return c.resident_mode == 2 || cg_loop_fits(c.dev(), c.num_sms, c.arith);
 }
 
+// CG iterations n_begin..loop_max of tea_solve.f90:147-332 with all scalars
+// on the device (tea_cg_loop.cu): the whole loop as one cooperative launch, or
+// batches of iterations, two kernels each, replayed from a captured graph with
+// one read of the loop state per batch.  Kernels queued after the loop has
+// stopped return at once.  The arithmetic and the exit test are those of the
+// per-call path, so the results are bit-identical to it.  The true-residual
+// exit (r.r beside r.z) and profiling use the kernels.
 int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
                            double eps_target, double* rro_out,
                            double* error_out, int* n_done, int* converged,
@@ -1586,13 +1614,12 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
                            double switch_eps) {
   Chunk& c = chunk();
   flush_pending_inner(c);
-  if (c.res_graph &&
-      (c.res_graph_true_exit != true_exit || c.res_graph_epoch != c.field_epoch ||
-       c.res_graph_arith != c.arith)) {
-    cudaGraphExecDestroy(c.res_graph);
-    c.res_graph = nullptr;
-  }
-  const int batch = 16;
+  // Fewer iterations than a replay makes (PPCG's single one in the timesteps
+  // after its first) are queued without a graph: the 30 further kernels of a
+  // replay only return, but cost 45 us.
+  const int left = loop_max - n_begin + 1;
+  const bool direct = c.profiler_on || left < kGraphIters;
+  const int batch = left < kGraphIters ? left + (left & 1) : kGraphIters;
   if (c.res_coef_n < loop_max + 2) {
     cudaFree(c.res_coef);
     c.res_coef = nullptr;
@@ -1640,21 +1667,8 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
       }
     }
   } else {
-  if (!c.res_graph && !c.profiler_on) {
-    cudaGraph_t graph = nullptr;
-    if (!check_cuda(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal),
-                    "graph capture"))
-      return -1;
-    enqueue_resident_iterations(c, batch, true_exit);
-    if (!check_cuda(cudaStreamEndCapture(c.stream, &graph), "graph capture end") ||
-        !check_cuda(cudaGraphInstantiate(&c.res_graph, graph, 0), "graph instantiate"))
-      return -1;
-    cudaGraphDestroy(graph);
-    c.res_graph_iters = batch;
-    c.res_graph_true_exit = true_exit;
-    c.res_graph_epoch = c.field_epoch;
-    c.res_graph_arith = c.arith;
-  }
+  cudaGraphExec_t graph = nullptr;
+  if (!direct && !(graph = cg_graph(c, true_exit))) return -1;
   // every batch runs at least one iteration until the loop stops, so the
   // loop needs at most this many batches; more means the state is corrupt
   const long long max_batches = (long long)(loop_max - n_begin) / batch + 3;
@@ -1663,8 +1677,8 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
       fail(24, "resident CG loop did not stop after %lld batches", nb);
       return -1;
     }
-    if (c.res_graph) {
-      if (!check_cuda(cudaGraphLaunch(c.res_graph, c.stream), "graph launch"))
+    if (graph) {
+      if (!check_cuda(cudaGraphLaunch(graph, c.stream), "graph launch"))
         return -1;
     } else {
       enqueue_resident_iterations(c, batch, true_exit);

@@ -1,6 +1,7 @@
 """Which form the resident driver takes (one launch, or kernels) by the work
 per SM: tiles of 16 rows count as four of 4, so grids on the far side of the
-change of tile height stay with the kernels."""
+change of tile height stay with the kernels; and how many kernels a single
+iteration queues."""
 import pytest
 
 from tealeaf_opencl_gb300 import decks, lib
@@ -59,3 +60,14 @@ def test_jacobi_form_follows_the_work_per_sm():
                                      summary_frequency=0)
         per_call = launches(deck, mode=lib.DRIVER_PER_CALL)
         assert launches(deck) == (per_call - 19 if one_launch else per_call)
+
+
+@pytest.mark.parametrize("prec", ["jac_diag", "jac_block"])
+def test_one_cg_iteration_queues_two_iterations_kernels(prec):
+    """PPCG's single CG iteration of the later timesteps, in the form of
+    separate kernels: two iterations of two kernels and the closing one, against
+    the one launch of the loop."""
+    deck = decks.five_state_deck(100, "ppcg", prec, steps=2, eps=1e-30, max_iters=200,
+                                 y_cells=70, inner_steps=4, presteps=10, summary_frequency=0,
+                                 extra="tl_ch_cg_epslim=1e30")
+    assert launches(deck, 1, steps=2) - launches(deck, 2, steps=2) == 4
