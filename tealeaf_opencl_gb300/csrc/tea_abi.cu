@@ -245,12 +245,18 @@ static void free_chunk(Chunk& c) {
   c.ready = false;
 }
 
-static bool alloc_field(Chunk& c, Field& f) {
+// optional: no memory for it is no error
+static bool alloc_field(Chunk& c, Field& f, bool optional = false) {
   // the offset makes padded column H of every row 256-byte aligned
   const long long off = (32 - (c.H % 32)) % 32;
   const size_t n = (size_t)(off + c.rows * c.S + 32);
-  if (!check_cuda(cudaMalloc(&f.base, n * sizeof(double)), "cudaMalloc field"))
+  const cudaError_t e = cudaMalloc(&f.base, n * sizeof(double));
+  if (e == cudaErrorMemoryAllocation && optional) {
+    cudaGetLastError();
+    f.base = nullptr;
     return false;
+  }
+  if (!check_cuda(e, "cudaMalloc field")) return false;
   if (!check_cuda(cudaMemsetAsync(f.base, 0, n * sizeof(double), c.stream),
                   "cudaMemset field"))
     return false;
@@ -415,6 +421,15 @@ bool ensure_alt_fields(Chunk& c) {
 
 bool ensure_u_alt(Chunk& c) { return c.u2.base || alloc_field(c, c.u2); }
 bool ensure_p_alt(Chunk& c) { return c.p2.base || alloc_field(c, c.p2); }
+
+// Asked once per chunk: a refused cudaMalloc in every call costs more than the
+// buffer saves.
+static bool have_alt(Chunk& c, Field& f, bool& refused) {
+  if (!f.base && !refused) refused = !alloc_field(c, f, true);
+  return f.base != nullptr;
+}
+bool have_u_alt(Chunk& c) { return have_alt(c, c.u2, c.u2_refused); }
+bool have_p_alt(Chunk& c) { return have_alt(c, c.p2, c.p2_refused); }
 
 void swap_alt_fields(Chunk& c) {
   std::swap(c.r, c.r2);
@@ -851,7 +866,12 @@ extern "C" void tea_leaf_cheby_iterate_kernel_ocl_(const int* cheby_calc_step) {
     return;
   }
   // calc_u folded into calc_p: the new u goes to the second buffer, which
-  // then becomes u
+  // then becomes u; without one a point preconditioner takes calc_p, calc_u
+  if (c.prec != PREC_JAC_BLOCK && !have_u_alt(c)) {
+    launch_cheby_calc_pu(c, c.cheby_alpha_h[s], c.cheby_beta_h[s], nullptr);
+    launch_cheby_calc_u(c);
+    return;
+  }
   if (!ensure_u_alt(c)) return;
   launch_cheby_calc_pu(c, c.cheby_alpha_h[s], c.cheby_beta_h[s], c.u2.f);
   std::swap(c.u, c.u2);
@@ -940,10 +960,23 @@ extern "C" void tea_leaf_jacobi_solve_kernel_ocl_(double* error) {
   *error = NAN;
   if (!need_chunk("tea_leaf_jacobi_solve_kernel_ocl_")) return;
   Chunk& c = chunk();
-  // the new u goes to the second buffer, which then becomes u
-  if (!ensure_u_alt(c)) return;
+  // the new u goes to the second buffer, which then becomes u; without one the
+  // sweep reads the copy that it leaves in un
+  if (!have_u_alt(c)) {
+    const long long first = (long long)c.H * c.S + c.H;
+    const size_t pitch = (size_t)c.S * sizeof(double);
+    if (!check_cuda(cudaMemcpy2DAsync(c.Mi.f + first, pitch, c.u.f + first, pitch,
+                                      c.x_max * sizeof(double), c.y_max,
+                                      cudaMemcpyDeviceToDevice, c.stream),
+                    "Jacobi copy of u"))
+      return;
+    arm_host_result(c);
+    launch_jacobi_sweep(c, c.Mi.f, c.u.f, nullptr);
+    fetch(1, error);
+    return;
+  }
   arm_host_result(c);
-  launch_jacobi_sweep(c, c.u2.f);
+  launch_jacobi_sweep(c, c.u.f, c.u2.f, c.Mi.f);
   std::swap(c.u, c.u2);
   c.field_epoch++;
   fetch(1, error);

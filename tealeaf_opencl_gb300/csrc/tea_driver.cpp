@@ -724,12 +724,14 @@ class Driver {
         cheby_calc_steps++;
       } else if (use_cg || use_cheby || use_ppcg) {
         if (mode == TEA_DRIVER_RESIDENT &&
-            (use_cg || (!D.verbose && !tea::kernels_timed()))) {
+            (use_cg || (!D.verbose && !tea::kernels_timed())) &&
+            ((use_cg && D.true_exit) || tea::have_p_alt(tea::chunk()))) {
           // The whole remaining CG loop, or the CG iterations before the
           // switch to Chebyshev or PPCG, on the device; it stops exactly
           // where this loop would (same tests, same arithmetic).  PPCG
           // switches after one iteration once the eigenvalues are known.
-          // While kernels are timed the latter stay the separate kernels.
+          // While kernels are timed the latter stay the separate kernels, as
+          // do both without memory for the loop's second p.
           int n_done = 0, conv = 0;
           tea::chunk().solver_checks = checks & TEA_CHECK_BREAKDOWN;
           const bool one = use_ppcg && !first;
@@ -763,7 +765,8 @@ class Driver {
         rro = rrn;
       } else if (use_jacobi && mode == TEA_DRIVER_RESIDENT && !D.verbose &&
                  !(checks & TEA_CHECK_BREAKDOWN) && !tea::kernels_timed() &&
-                 tea::jacobi_loop_fits(tea::chunk().dev(), tea::chunk().num_sms)) {
+                 tea::jacobi_loop_fits(tea::chunk().dev(), tea::chunk().num_sms) &&
+                 tea::have_u_alt(tea::chunk())) {
         int n_done = 0, conv = 0;
         if (tea::resident_jacobi_iterations(n, loop_max, D.eps * initial_residual, &error,
                                             &n_done, &conv) != 0)

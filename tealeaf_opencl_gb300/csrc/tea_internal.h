@@ -140,6 +140,7 @@ struct Chunk {
   // buffer it does not read; the two then trade places
   Field u2;
   Field p2;  // second p buffer of the resident CG loop (tea_cg_loop.cu)
+  bool u2_refused = false, p2_refused = false;  // no memory for them
   int inner_pairs = 0;      // run PPCG inner steps in fused pairs where they apply
   int field_epoch = 0;      // bumped whenever r/sd and r2/sd2 trade places
   int pending_inner = -1;   // a per-call inner step (0-based) not launched yet
@@ -213,14 +214,15 @@ void launch_cg_calc_p(Chunk& c, double beta);
 void launch_cheby_init_p(Chunk& c, double theta);
 void launch_cheby_calc_u(Chunk& c);
 // calc_p and calc_u of one Chebyshev iteration in one pass, the new u into un
+// (with a point preconditioner un may be null: calc_p alone)
 void launch_cheby_calc_pu(Chunk& c, double alpha, double beta, double* un);
 void launch_ppcg_init_sd(Chunk& c, double theta);
 void launch_ppcg_update_r(Chunk& c);
 // update_r and calc_sd of one inner step in one pass, sd read from sdi and the new sd written to sdo
 void launch_ppcg_step(Chunk& c, double alpha, double beta, const double* sdi, double* sdo);
 void launch_ppcg_calc_sd(Chunk& c, double alpha, double beta);
-// one Jacobi sweep, the new u into unew
-void launch_jacobi_sweep(Chunk& c, double* unew);
+// one Jacobi sweep from u, the new u into unew, u into un if there is one
+void launch_jacobi_sweep(Chunk& c, const double* u, double* unew, double* un);
 void launch_finalise(Chunk& c);
 void launch_field_summary(Chunk& c);
 void launch_update_halo(Chunk& c, int mask, int depth);
@@ -306,6 +308,9 @@ bool ensure_alt_fields(Chunk& c);
 // allocates u2 / p2 on first use
 bool ensure_u_alt(Chunk& c);
 bool ensure_p_alt(Chunk& c);
+// the same where the caller has a way without: no memory for it is no error
+bool have_u_alt(Chunk& c);
+bool have_p_alt(Chunk& c);
 // r/sd and r2/sd2 trade places (the fused pair has just written r2/sd2)
 void swap_alt_fields(Chunk& c);
 // launches a per-call PPCG inner step held back for pairing (tea_abi.cu)

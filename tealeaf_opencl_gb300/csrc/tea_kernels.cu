@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(kBlock, 3)
 
 // The same iteration without a preconditioner or with the diagonal one:
 // p = alpha p + beta r or alpha p + (beta Mi) r, u + p to the second u buffer.
-// One pass in place of calc_p and calc_u; 7 FP64 instructions per cell with the
+// One pass in place of calc_p and calc_u (without a second buffer calc_p alone); 7 FP64 instructions per cell with the
 // products on the integer pipes (bit-identical), 10 with all of them on the
 // FP64 pipe.
 template <int F, int MB, bool EMU>
@@ -613,10 +613,10 @@ __global__ void __launch_bounds__(kBlock, MB)
         w[c] = wl[j];
         r[c] = rl[j];
         p[c] = pn;
-        un[c] = uv[j + 1] + pn;
+        if (un) un[c] = uv[j + 1] + pn;
       }
   });
-  copy_halo_ring(d, d.u, un_);
+  if (un_) copy_halo_ring(d, d.u, un_);
 }
 
 // tea_leaf_cheby_solve_init_p (tea_leaf_cheby_cl.cl:4-64): w = A u,
@@ -997,13 +997,15 @@ __global__ void __launch_bounds__(kBlock, 1)
   });
 }
 
-// one Jacobi sweep (jacobi_tile)
+// one Jacobi sweep (jacobi_tile); without un, u is un's copy and unew keeps its
+// own halo ring
 template <int TH, bool EMU>
-__global__ void __launch_bounds__(kBlock) k_jacobi_sweep(Dev d, Red red, double* unew) {
+__global__ void __launch_bounds__(kBlock)
+    k_jacobi_sweep(Dev d, Red red, const double* u, double* unew, double* un) {
   tile_driver<TH, 1>(d, red, [&](int x, int y0, bool xin, double* acc) {
-    if (xin) acc[0] = jacobi_tile<TH, false, EMU>(d, d.u, unew, d.un, x, y0);
+    if (xin) acc[0] = jacobi_tile<TH, false, EMU>(d, u, unew, un, x, y0);
   });
-  copy_halo_ring(d, d.u, unew);
+  if (un) copy_halo_ring(d, u, unew);
 }
 
 // tea_leaf_finalise, tea_leaf_common_cl.cl:4-15
@@ -1253,14 +1255,14 @@ void launch_ppcg_calc_sd(Chunk& c, double alpha, double beta) {
               div_const(1.0), alpha, beta, (const ResState*)nullptr);
 }
 
-void launch_jacobi_sweep(Chunk& c, double* unew) {
+void launch_jacobi_sweep(Chunk& c, const double* u, double* unew, double* un) {
   const char* name = "tea_leaf_jacobi_solve";  // the same arithmetic in every form
   if (few_supertiles(c.dev(), c.num_sms))
-    launch_tile(c, name, k_jacobi_sweep<4, false>, c.dev(), c.red(), unew);
+    launch_tile(c, name, k_jacobi_sweep<4, false>, c.dev(), c.red(), u, unew, un);
   else if (c.TH == 4)
-    launch_tile(c, name, k_jacobi_sweep<4, true>, c.dev(), c.red(), unew);
+    launch_tile(c, name, k_jacobi_sweep<4, true>, c.dev(), c.red(), u, unew, un);
   else
-    launch_tile(c, name, k_jacobi_sweep<16, true>, c.dev(), c.red(), unew);
+    launch_tile(c, name, k_jacobi_sweep<16, true>, c.dev(), c.red(), u, unew, un);
 }
 
 void launch_finalise(Chunk& c) {
