@@ -88,10 +88,7 @@ FP64_PER_CELL = {
     ("tea_leaf_cg_solve_calc_ur", "jac_block", "chain"): 5.5,
     ("tea_leaf_cg_solve_calc_ur", "jac_block", "fused"): 5.5,
     # the Chebyshev step: operator 5 (chain) or 6 (fused), r = u0 - w 1,
-    # strip sweep 2.5, alpha p + beta z 1 (beta z on the integer pipes)
-    ("tea_leaf_cheby_solve_calc_p", "jac_block", "chain"): 9.5,
-    ("tea_leaf_cheby_solve_calc_p", "jac_block", "fused"): 10.5,
-    # the same with calc_u's u + p folded in
+    # strip sweep 2.5, alpha p + beta z 1 (beta z on the integer pipes), u + p 1
     ("tea_leaf_cheby_solve_calc_p_u", "jac_block", "chain"): 10.5,
     ("tea_leaf_cheby_solve_calc_p_u", "jac_block", "fused"): 11.5,
 }
@@ -414,15 +411,19 @@ def run_ours(args, dist):
 
 
 # algorithmic bytes per interior cell of each entry point's kernels: the
-# fields the reference kernel reads and writes, each once, FP64
+# fields the reference kernel reads and writes, each once, FP64; for the
+# one-pass Jacobi sweep and point-preconditioner inner step the fields of that
+# pass (the block-Jacobi rows of one-pass kernels are the reference's kernels
+# together, as step_bytes_per_cell_iteration counts them)
 KERNEL_BYTES = {
     "tea_leaf_cg_solve_calc_w": 32,       # r p Kx Ky, w w
     "tea_leaf_cg_solve_calc_ur": {"jac_diag": 64, "jac_block": 88, "none": 56},
     "tea_leaf_cg_solve_calc_p": 24,       # r z p, w p
     "tea_leaf_calc_2norm": 16,
     "tea_leaf_ppcg_solve_update_r": 56,   # r u r Kx Ky sd, w u r
-    # update_r and calc_sd in one pass (block Jacobi): the two kernels' fields
-    "tea_leaf_ppcg_solve_inner_step": {"jac_diag": 88, "jac_block": 112, "none": 80},
+    # update_r and calc_sd in one pass: sd u r Kx Ky (Mi), sd u r; block Jacobi:
+    # the two kernels' fields
+    "tea_leaf_ppcg_solve_inner_step": {"jac_diag": 72, "jac_block": 112, "none": 64},
     "tea_leaf_ppcg_solve_inner_pair": 88,  # two steps: r u r sd Kx Ky diag cp bfp, w u r sd
     "tea_leaf_ppcg_solve_calc_sd": {"jac_diag": 32, "jac_block": 56, "none": 24},
     "tea_leaf_cheby_solve_calc_p": {"jac_diag": 80, "jac_block": 96, "none": 72},
@@ -433,7 +434,7 @@ KERNEL_BYTES = {
     "tea_leaf_cg_solve_init_p": {"jac_diag": 32, "jac_block": 56, "none": 24},
     "tea_leaf_ppcg_solve_init_sd": {"jac_diag": 24, "jac_block": 48, "none": 16},
     "tea_leaf_cheby_solve_init_p": {"jac_diag": 72, "jac_block": 88, "none": 64},
-    "tea_leaf_jacobi_solve": 64,          # copy_u and solve in one pass: u, un; u0 un Kx Ky, u
+    "tea_leaf_jacobi_solve": 48,          # copy_u and solve in one pass: u u0 Kx Ky, u un
     "tea_leaf_finalise": 24,              # u density, energy1
     "field_summary": 32,                  # volume density energy1 u
     "tea_leaf_init_common": 24,           # density, Kx Ky

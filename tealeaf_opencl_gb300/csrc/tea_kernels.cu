@@ -923,9 +923,9 @@ __global__ void __launch_bounds__(kBlock, 3)
 
 // The same inner step without a preconditioner or with the diagonal one
 // (tea_leaf_ppcg_cl.cl:62-155): u += sd, r -= A sd, sd' = alpha sd + beta r or
-// alpha sd + (beta r) Mi, the new sd to the second buffer.  One pass of 80 (88)
-// algorithmic bytes and 7 FP64 instructions per cell in place of update_r and
-// calc_sd; the products run on the integer pipes (bit-identical).  Rows past
+// alpha sd + (beta r) Mi, the new sd to the second buffer.  One pass of 72 (80)
+// bytes, stored diagonal included, and 7 FP64 instructions per cell in place of
+// update_r and calc_sd; the products run on the integer pipes (bit-identical).  Rows past
 // the interior are clamped to the halo row, so every load is issued before the
 // first use; the values of such rows are not stored.
 template <int F, int MB, bool EMU>
