@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(kBlock, 3)
 // One pass in place of calc_p and calc_u (without a second buffer calc_p alone); 7 FP64 instructions per cell with the
 // products on the integer pipes (bit-identical), 10 with all of them on the
 // FP64 pipe.
-template <int F, int MB, bool EMU>
+template <int F, int MB, bool EMU, bool U = true>
 __global__ void __launch_bounds__(kBlock, MB)
     k_cheby_calc_pu_point(Dev d, Red red, double alpha, double beta, double* un_) {
   tile_driver<4, 0>(d, red, [&](int x, int y0, bool xin, double* acc) {
@@ -613,10 +613,10 @@ __global__ void __launch_bounds__(kBlock, MB)
         w[c] = wl[j];
         r[c] = rl[j];
         p[c] = pn;
-        if (un) un[c] = uv[j + 1] + pn;
+        if (U) un[c] = uv[j + 1] + pn;
       }
   });
-  if (un_) copy_halo_ring(d, d.u, un_);
+  if (U) copy_halo_ring(d, d.u, un_);
 }
 
 // tea_leaf_cheby_solve_init_p (tea_leaf_cheby_cl.cl:4-64): w = A u,
@@ -1192,6 +1192,14 @@ void launch_cheby_calc_pu(Chunk& c, double alpha, double beta, double* un) {
   if (c.prec != PREC_JAC_BLOCK) {
     const Dev d4 = dev4(c);
     const char* name = "tea_leaf_cheby_solve_calc_p_u";
+    if (!un) {
+      auto* const calc_p = c.arith == 2   ? k_cheby_calc_pu_point<2, 4, true, false>
+                           : c.arith == 1 ? k_cheby_calc_pu_point<1, 4, true, false>
+                                          : k_cheby_calc_pu_point<0, 4, true, false>;
+      launch_tile_ns(c, "tea_leaf_cheby_solve_calc_p", d4.ns, calc_p, d4, c.red(), alpha, beta,
+                     un);
+      return;
+    }
     auto* const kernel = c.arith == 2   ? TEA_POINT(k_cheby_calc_pu_point, 2, c)
                          : c.arith == 1 ? TEA_POINT(k_cheby_calc_pu_point, 1, c)
                                         : TEA_POINT(k_cheby_calc_pu_point, 0, c);
