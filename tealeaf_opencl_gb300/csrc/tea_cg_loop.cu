@@ -398,18 +398,23 @@ bool launch_jacobi_loop(const LaunchCtx& l, const Dev& d_, double* u2, const Red
 // 8-10 us (start, drain, the last block's sum), a grid barrier with the sum in
 // every block 2.5 us; but the cooperative kernel's passes share one register
 // budget (16 warps per SM), so long passes run at 0.8-0.95 of the rate of their
-// own kernels.  us per CG iteration, graph / one launch, at 1501 columns:
-//   per SM                  7.9         9.9         10.4        11.9        13.9        14.9
-//   diagonal, fused     43.7 / 40.5 55.2 / 55.2 59.1 / 61.6 64.6 / 65.7 71.6 / 74.3 76.1 / 81.3
-//   block, fused        49.6 / 45.1 61.4 / 60.2 65.2 / 67.3 71.5 / 71.9 79.4 / 81.6 85.2 / 89.1
-//   none, fused         41.7 / 36.6 51.2 / 47.1 55.4 / 52.8 61.6 / 59.1 68.8 / 68.5 72.9 / 75.1
-//   block, exact form   81.1 / 70.2 96.4 / 90.3 98.4 / 99.7  109 / 107   130 / 122   133 / 132
-// (the exact form's strip divides keep both forms on the FP64 pipe).  In 16-row
-// tiles, 32 per SM and more, the graph is ahead throughout: diagonal fused 2176^2
-// 143 / 149, 2500^2 172 / 186, 2800^2 208 / 219.
+// own kernels, and a block takes supertiles two at a time, so its time steps up
+// where a further round begins.  us per CG iteration, graph / one launch, at 1501
+// columns (2 per SM are a round):
+//   per SM, within 0.2      9.0         10.0        11.1        12.0        12.2        13.9
+//   diagonal, chain     50.3 / 49.4 55.1 / 53.6 60.7 / 61.2 62.7 / 63.2 65.5 / 69.5 69.7 / 71.5
+//   block, chain        56.6 / 54.7 61.3 / 59.0 67.6 / 67.2 69.2 / 69.4 72.6 / 76.1
+//   block, fused        57.8 / 56.8 62.9 / 61.1 69.2 / 69.6 71.1 / 71.8 74.8 / 79.1 79.4 / 81.6
+//   none, chain         47.9 / 42.0 50.3 / 45.0 55.5 / 52.6 59.9 / 56.8             66.9 / 65.7
+//   block, exact        84.2 / 83.0 96.4 / 90.3  105 / 101   109 / 107   116 / 116   130 / 122
+// So the line is where the seventh round begins; without a preconditioner and in
+// the exact form (whose strip divides take both forms' time) the seventh round
+// still gains, and the eighth does not (14.9 per SM: 72.9 / 75.1 none fused, 133 /
+// 132 block exact).  In 16-row tiles, 32 per SM and more, the graph is ahead
+// throughout: diagonal fused 2176^2 143 / 149, 2500^2 172 / 186, 2800^2 208 / 219.
 static int rows4_supertiles(const Dev& d) { return d.ns * (d.th / 4); }
 bool cg_loop_fits(const Dev& d, int num_sms, int arith) {
-  const int per_sm = arith != 0 && d.prec != PREC_NONE ? 10 : 14;
+  const int per_sm = arith != 0 && d.prec != PREC_NONE ? 12 : 14;
   return rows4_supertiles(d) <= per_sm * num_sms;
 }
 

@@ -30,7 +30,7 @@ def sms():
 
 
 # 4-row supertiles of 1501 columns: six a row of tiles
-@pytest.mark.parametrize("prec,form,lo,hi", [("jac_diag", "fused", 10, 10), ("none", "chain", 14, 14),
+@pytest.mark.parametrize("prec,form,lo,hi", [("jac_diag", "fused", 12, 12), ("none", "chain", 14, 14),
                                              ("jac_block", "exact", 14, 14)])
 def test_cg_form_follows_the_work_per_sm(prec, form, lo, hi):
     for per_sm, one_launch in ((lo, True), (hi + 0.2, False)):
