@@ -723,23 +723,24 @@ class Driver {
         }
         cheby_calc_steps++;
       } else if (use_cg || use_cheby || use_ppcg) {
+        // PPCG switches after one iteration once the eigenvalues are known: the
+        // upload and read-backs of a device loop would cost 20 us more than the
+        // three calls of that one
+        const bool one = use_ppcg && !first;
         if (mode == TEA_DRIVER_RESIDENT &&
-            (use_cg || (!D.verbose && !tea::kernels_timed())) &&
+            (use_cg || (!one && !D.verbose && !tea::kernels_timed())) &&
             ((use_cg && D.true_exit) || tea::have_p_alt(tea::chunk()))) {
           // The whole remaining CG loop, or the CG iterations before the
           // switch to Chebyshev or PPCG, on the device; it stops exactly
-          // where this loop would (same tests, same arithmetic).  PPCG
-          // switches after one iteration once the eigenvalues are known.
-          // While kernels are timed the latter stay the separate kernels, as
-          // do both without memory for the loop's second p.
+          // where this loop would (same tests, same arithmetic).  While
+          // kernels are timed the latter stay the separate kernels, as do
+          // both without memory for the loop's second p.
           int n_done = 0, conv = 0;
           tea::chunk().solver_checks = checks & TEA_CHECK_BREAKDOWN;
-          const bool one = use_ppcg && !first;
-          if (tea::resident_cg_iterations(n, one ? std::min(loop_max, std::max(n, 1)) : loop_max,
-                                          rro, D.eps * initial_residual, &rro, &error, &n_done,
-                                          &conv, cg_alphas.data(), cg_betas.data(),
-                                          use_cg && D.true_exit,
-                                          use_cg || one ? 0 : std::max(D.presteps, 1),
+          if (tea::resident_cg_iterations(n, loop_max, rro, D.eps * initial_residual, &rro,
+                                          &error, &n_done, &conv, cg_alphas.data(),
+                                          cg_betas.data(), use_cg && D.true_exit,
+                                          use_cg ? 0 : std::max(D.presteps, 1),
                                           D.epslim) != 0 ||
               !resident_breakdown_ok())
             return -1;

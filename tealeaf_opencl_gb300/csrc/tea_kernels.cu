@@ -1578,7 +1578,7 @@ static bool ensure_resident_state(Chunk& c) {
   return true;
 }
 
-constexpr int kGraphIters = 16;  // iterations of one graph replay (even)
+constexpr int kGraphIters = 16;  // iterations of one batch (even)
 
 // The graph of kGraphIters iterations on the current buffers in the current
 // form, captured unless one of the two kept is that (one per buffer of u).
@@ -1624,12 +1624,6 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
                            double switch_eps) {
   Chunk& c = chunk();
   flush_pending_inner(c);
-  // Fewer iterations than a replay makes (PPCG's single one in the timesteps
-  // after its first) are queued without a graph: the 30 further kernels of a
-  // replay only return, but cost 45 us.
-  const int left = loop_max - n_begin + 1;
-  const bool direct = c.profiler_on || left < kGraphIters;
-  const int batch = left < kGraphIters ? left + (left & 1) : kGraphIters;
   if (c.res_coef_n < loop_max + 2) {
     cudaFree(c.res_coef);
     c.res_coef = nullptr;
@@ -1678,10 +1672,10 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
     }
   } else {
   cudaGraphExec_t graph = nullptr;
-  if (!direct && !(graph = cg_graph(c, true_exit))) return -1;
+  if (!c.profiler_on && !(graph = cg_graph(c, true_exit))) return -1;
   // every batch runs at least one iteration until the loop stops, so the
   // loop needs at most this many batches; more means the state is corrupt
-  const long long max_batches = (long long)(loop_max - n_begin) / batch + 3;
+  const long long max_batches = (long long)(loop_max - n_begin) / kGraphIters + 3;
   for (long long nb = 0;; nb++) {
     if (nb >= max_batches) {
       fail(24, "resident CG loop did not stop after %lld batches", nb);
@@ -1691,10 +1685,10 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
       if (!check_cuda(cudaGraphLaunch(graph, c.stream), "graph launch"))
         return -1;
     } else {
-      enqueue_resident_iterations(c, batch, true_exit);
+      enqueue_resident_iterations(c, kGraphIters, true_exit);
       check_cuda(cudaGetLastError(), "resident launch");
     }
-    count_launches(2 * batch + 1);
+    count_launches(2 * kGraphIters + 1);
     if (!check_cuda(cudaMemcpyAsync(&h, c.res_state, sizeof(ResState),
                                     cudaMemcpyDeviceToHost, c.stream),
                     "resident state read") ||
