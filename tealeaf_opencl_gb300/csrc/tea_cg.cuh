@@ -201,9 +201,12 @@ __device__ __forceinline__ void cg_p_tile(const Dev& d, int x, int y0, bool xin,
 
 // ---- the two-pass CG iteration (tea_cg_loop.cu, tea_batch.cu) ----
 
-template <int F>
+// The exact form's product is one FP64 instruction more, and pass w forms p' of
+// the cells around a tile a second time: on the integer pipes (bit-identical)
+// it leaves the two passes ahead of three kernels, see k_cg_pass_r.
+template <int F, bool EMU = false>
 __device__ __forceinline__ double p_next(double beta, double p, double z) {
-  return F ? __fma_rn(beta, p, z) : z + beta * p;
+  return F ? __fma_rn(beta, p, z) : z + mul_e<EMU>(beta, p);
 }
 
 // Pass A on one tile: lane column x, rows y0 .. y0+TH-1.  p' of the rows
@@ -237,7 +240,7 @@ __device__ __forceinline__ double loop_w_tile(const Dev& d, const double* __rest
   const double* __restrict__ pcol = xin ? pin : hal;
   // p' from the old p and z; halo cells keep p
   auto fresh = [&](double po, double zv, bool in) {
-    return first || !in ? po : p_next<F>(beta, po, zv);
+    return first || !in ? po : p_next<F, EMU>(beta, po, zv);
   };
   double acc = 0.0;
   double pm = 0.0, pc = 0.0, pco = 0.0;  // p' of rows g-1 and g, old p of row g
@@ -316,8 +319,9 @@ __device__ __forceinline__ double loop_w_tile(const Dev& d, const double* __rest
 
 // Pass B on one tile: r -= alpha w, z = M^-1 r and the lane's share of r.z
 // (cg_ur_tile_r without u, which pass A updates).  A lane reads back only
-// the r and w that it wrote itself.
-template <int TH, int F, int NV = 1, bool EMU = true>
+// the r and w that it wrote itself.  RE: the exact form's alpha w on the integer
+// pipes.
+template <int TH, int F, int NV = 1, bool EMU = true, bool RE = false>
 __device__ __forceinline__ void loop_r_tile(const Dev& d, int x, int y0, double alpha,
                                             double* acc) {
   double* __restrict__ r = d.r;
@@ -326,6 +330,9 @@ __device__ __forceinline__ void loop_r_tile(const Dev& d, int x, int y0, double 
   const long long S = d.S;
   if (x >= d.x_max) return;
   const int rows = min(TH, d.y_max - y0);
+  auto r_next = [&](double rr, double ww) {
+    return F ? __fma_rn(-alpha, ww, rr) : rr - mul_e<RE>(alpha, ww);
+  };
 #pragma unroll 1
   for (int g = 0; g < rows; g += 4) {
     const long long c0 = cidx(d, x, y0 + g);
@@ -350,7 +357,7 @@ __device__ __forceinline__ void loop_r_tile(const Dev& d, int x, int y0, double 
       const double d0 = F ? 0.0 : __ldg(d.diag + c0);
 #pragma unroll
       for (int j = 0; j < 4; j++)
-        rv[j] = g + j >= rows ? 0.0 : F ? __fma_rn(-alpha, wv[j], rv[j]) : rv[j] - alpha * wv[j];
+        rv[j] = g + j >= rows ? 0.0 : r_next(rv[j], wv[j]);
       if (upper == 4)
         strip_solve_v<F, false, true>(4, rv, bl, kl, cl, d0, zv);
       else
@@ -358,7 +365,7 @@ __device__ __forceinline__ void loop_r_tile(const Dev& d, int x, int y0, double 
     } else {
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        rv[j] = F ? __fma_rn(-alpha, wv[j], rv[j]) : rv[j] - alpha * wv[j];
+        rv[j] = r_next(rv[j], wv[j]);
         zv[j] = d.prec == PREC_JAC_DIAG ? mul_e<EMU>(rv[j], mv[j]) : rv[j];
       }
     }

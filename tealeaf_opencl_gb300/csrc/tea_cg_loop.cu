@@ -271,6 +271,11 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
 // at 4096^2 diagonal, 474 and 504 at three and four blocks; pass B streams at
 // four (392, 412 at three, two).  The exact form's pass B needs more registers
 // (its strip divides): three blocks, 3000^2 block Jacobi 468 -> 458 us.
+// In that form, bound by the FP64 pipe throughout, the two passes fell behind
+// the three kernels on large grids until beta p and alpha w moved to the integer
+// pipes; us per iteration, three kernels / two passes before / after: 3000x2900
+// none 356 / 374 / 346, block 431 / 447 / 421, none with the true-residual exit
+// 399 / 416 / 386; 1800x1700 none 160 / 164 / 158, block 192 / 195 / 189.
 
 // Pass A.  An iteration whose predecessor has run (p_pending) forms p' and
 // finishes u; the first one copies p, so that p alternates between the two
@@ -299,7 +304,7 @@ __global__ void __launch_bounds__(kBlock, F ? 4 : 3) k_cg_pass_r(Dev d, Red red,
   if (*(volatile int*)&st->stop) return;
   const double alpha = st->alpha;
   const bool last = tile_driver<TH, NV>(d, red, [&](int x, int y0, bool, double* acc) {
-    loop_r_tile<TH, F, NV>(d, x, y0, alpha, acc);
+    loop_r_tile<TH, F, NV, true, true>(d, x, y0, alpha, acc);
   });
   if (last && threadIdx.x == 0) cg_scalar_step<NV>(st, alpha, red.result);
 }
