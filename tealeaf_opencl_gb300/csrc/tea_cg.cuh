@@ -220,7 +220,8 @@ __device__ __forceinline__ double p_next(double beta, double p, double z) {
 // L2.  All loads of four rows are issued before anything waits for one; rows
 // past the interior are clamped to the halo row above it and lanes past the
 // last column read the row's padding, and neither is used.
-template <int TH, int F, bool COPY = false, bool EMU = true>
+// PE: the exact form's alpha p and beta p on the integer pipes.
+template <int TH, int F, bool COPY = false, bool EMU = true, bool PE = EMU>
 __device__ __forceinline__ double loop_w_tile(const Dev& d, const double* __restrict__ pin,
                                               double* __restrict__ pout,
                                               const double* __restrict__ zsrc, int x, int y0,
@@ -240,7 +241,7 @@ __device__ __forceinline__ double loop_w_tile(const Dev& d, const double* __rest
   const double* __restrict__ pcol = xin ? pin : hal;
   // p' from the old p and z; halo cells keep p
   auto fresh = [&](double po, double zv, bool in) {
-    return first || !in ? po : p_next<F, EMU>(beta, po, zv);
+    return first || !in ? po : p_next<F, PE>(beta, po, zv);
   };
   double acc = 0.0;
   double pm = 0.0, pc = 0.0, pco = 0.0;  // p' of rows g-1 and g, old p of row g
@@ -294,7 +295,7 @@ __device__ __forceinline__ double loop_w_tile(const Dev& d, const double* __rest
       const long long c = c0 + (g + j) * S;
       const bool own = xin && g + j < rows;
       if (own && !first)
-        u[c] = F ? __fma_rn(alpha, po[j + 1], uv[j]) : uv[j] + alpha * po[j + 1];
+        u[c] = F ? __fma_rn(alpha, po[j + 1], uv[j]) : uv[j] + mul_e<PE>(alpha, po[j + 1]);
       double pe = __shfl_down_sync(0xffffffffu, pv[j + 1], 1);
       double pw = __shfl_up_sync(0xffffffffu, pv[j + 1], 1);
       const double e = __shfl_sync(0xffffffffu, ev, 2 * j + 1);
@@ -375,10 +376,11 @@ __device__ __forceinline__ void loop_r_tile(const Dev& d, int x, int y0, double 
         r[c0 + j * S] = rv[j];
         if (d.prec != PREC_NONE) z[c0 + j * S] = zv[j];
         acc[0] = accum<F>(acc[0], rv[j], zv[j]);
-        if (NV > 1) acc[NV - 1] = accum<F>(acc[NV - 1], rv[j], rv[j]);
+        if (NV > 1 && d.prec != PREC_NONE) acc[NV - 1] = accum<F>(acc[NV - 1], rv[j], rv[j]);
       }
     }
   }
+  if (NV > 1 && d.prec == PREC_NONE) acc[NV - 1] = acc[0];  // z is r
 }
 
 // tea_leaf_jacobi_copy_u and tea_leaf_jacobi_solve in one pass

@@ -271,24 +271,27 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
 // at 4096^2 diagonal, 474 and 504 at three and four blocks; pass B streams at
 // four (392, 412 at three, two).  The exact form's pass B needs more registers
 // (its strip divides): three blocks, 3000^2 block Jacobi 468 -> 458 us.
-// In that form, bound by the FP64 pipe throughout, the two passes fell behind
-// the three kernels on large grids until beta p and alpha w moved to the integer
-// pipes; us per iteration, three kernels / two passes before / after: 3000x2900
-// none 356 / 374 / 346, block 431 / 447 / 421, none with the true-residual exit
-// 399 / 416 / 386; 1800x1700 none 160 / 164 / 158, block 192 / 195 / 189.
+//
+// In the exact form, bound by the FP64 pipe throughout, the two passes fell
+// behind three kernels on large grids until the products by alpha and beta moved
+// to the integer pipes (PE), but for few supertiles, where the FP64 pipe's own
+// are quicker (few_supertiles).  us per iteration, three kernels / two passes
+// before / after: 3000x2900 none 355 / 374 / 334, block 430 / 447 / 410;
+// 1800x1700 none 160 / 164 / 154, block 192 / 194 / 184; with the true-residual
+// exit 3000x2900 none 399 / 416 / 374, 1800x1700 none 169 / 182 / 170.
 
 // Pass A.  An iteration whose predecessor has run (p_pending) forms p' and
 // finishes u; the first one copies p, so that p alternates between the two
 // buffers whatever happens.
-template <int TH, int F>
-__global__ void __launch_bounds__(kBlock, F || TH == 16 ? 2 : 3)
+template <int TH, int F, bool PE>
+__global__ void __launch_bounds__(kBlock, 2)
     k_cg_pass_w(Dev d, Red red, ResState* st, const double* pin, double* pout) {
   if (*(volatile int*)&st->stop) return;
   const bool first = !*(volatile int*)&st->p_pending;
   const double alpha = st->alpha, beta = st->beta;
   const double* zsrc = d.prec != PREC_NONE ? d.z : d.r;
   const bool last = tile_driver<TH, 1>(d, red, [&](int x, int y0, bool, double* acc) {
-    acc[0] = loop_w_tile<TH, F, true>(d, pin, pout, zsrc, x, y0, alpha, beta, first);
+    acc[0] = loop_w_tile<TH, F, true, true, PE>(d, pin, pout, zsrc, x, y0, alpha, beta, first);
   });
   if (last && threadIdx.x == 0) {
     const double pw = red.result[0];
@@ -299,12 +302,12 @@ __global__ void __launch_bounds__(kBlock, F || TH == 16 ? 2 : 3)
 
 // Pass B and the scalar step; with NV = 2 also r.r for the exit test on the
 // unpreconditioned residual.
-template <int TH, int F, int NV>
+template <int TH, int F, int NV, bool PE>
 __global__ void __launch_bounds__(kBlock, F ? 4 : 3) k_cg_pass_r(Dev d, Red red, ResState* st) {
   if (*(volatile int*)&st->stop) return;
   const double alpha = st->alpha;
   const bool last = tile_driver<TH, NV>(d, red, [&](int x, int y0, bool, double* acc) {
-    loop_r_tile<TH, F, NV, true, true>(d, x, y0, alpha, acc);
+    loop_r_tile<TH, F, NV, true, PE>(d, x, y0, alpha, acc);
   });
   if (last && threadIdx.x == 0) cg_scalar_step<NV>(st, alpha, red.result);
 }
@@ -348,14 +351,21 @@ int pass_grid(const LaunchCtx& l, const Dev& d, void (*kernel)(KArgs...)) {
 template <int TH, int F, int NV>
 void enqueue_passes_t(const LaunchCtx& l, const Dev& d, double* p2, const Red& red,
                       ResState* st, unsigned int* counter, int iters) {
-  const int gw = pass_grid(l, d, k_cg_pass_w<TH, F>);
-  const int gr = pass_grid(l, d, k_cg_pass_r<TH, F, NV>);
+  auto* pass_w = k_cg_pass_w<TH, F, F == 0>;
+  auto* pass_r = k_cg_pass_r<TH, F, NV, F == 0>;
+  if constexpr (F == 0 && TH == 4)
+    if (few_supertiles(d, l.num_sms)) {
+      pass_w = k_cg_pass_w<TH, F, false>;
+      pass_r = k_cg_pass_r<TH, F, NV, false>;
+    }
+  const int gw = pass_grid(l, d, pass_w);
+  const int gr = pass_grid(l, d, pass_r);
   const int ge = pass_grid(l, d, k_cg_pass_end<TH, F>);
   for (int i = 0; i < iters; i += 2) {
-    k_cg_pass_w<TH, F><<<gw, kBlock, 0, l.stream>>>(d, red, st, d.p, p2);
-    k_cg_pass_r<TH, F, NV><<<gr, kBlock, 0, l.stream>>>(d, red, st);
-    k_cg_pass_w<TH, F><<<gw, kBlock, 0, l.stream>>>(d, red, st, p2, d.p);
-    k_cg_pass_r<TH, F, NV><<<gr, kBlock, 0, l.stream>>>(d, red, st);
+    pass_w<<<gw, kBlock, 0, l.stream>>>(d, red, st, d.p, p2);
+    pass_r<<<gr, kBlock, 0, l.stream>>>(d, red, st);
+    pass_w<<<gw, kBlock, 0, l.stream>>>(d, red, st, p2, d.p);
+    pass_r<<<gr, kBlock, 0, l.stream>>>(d, red, st);
   }
   k_cg_pass_end<TH, F><<<ge, kBlock, 0, l.stream>>>(d, red, st, p2, counter);
 }
@@ -411,11 +421,11 @@ bool launch_jacobi_loop(const LaunchCtx& l, const Dev& d_, double* u2, const Red
 //   block, chain        56.6 / 54.7 61.3 / 59.0 67.6 / 67.2 69.2 / 69.4 72.6 / 76.1
 //   block, fused        57.8 / 56.8 62.9 / 61.1 69.2 / 69.6 71.1 / 71.8 74.8 / 79.1 79.4 / 81.6
 //   none, chain         47.9 / 42.0 50.3 / 45.0 55.5 / 52.6 59.9 / 56.8             66.9 / 65.7
-//   block, exact        84.2 / 83.0 96.4 / 90.3  105 / 101   109 / 107   116 / 116   130 / 122
+//   block, exact        85.5 / 82.9 97.1 / 90.4  105 / 100   107 / 106   116 / 115   129 / 122
 // So the line is where the seventh round begins; without a preconditioner and in
-// the exact form (whose strip divides take both forms' time) the seventh round
-// still gains, and the eighth does not (14.9 per SM: 72.9 / 75.1 none fused, 133 /
-// 132 block exact).  In 16-row tiles, 32 per SM and more, the graph is ahead
+// the exact form (FP64-bound either way) it is where the eighth does, from which
+// the two are within 3 % (15.0 per SM: none fused 73.6 / 75.4, block exact 132 /
+// 131).  In 16-row tiles, 32 per SM and more, the graph is ahead
 // throughout: diagonal fused 2176^2 143 / 149, 2500^2 172 / 186, 2800^2 208 / 219.
 static int rows4_supertiles(const Dev& d) { return d.ns * (d.th / 4); }
 bool cg_loop_fits(const Dev& d, int num_sms, int arith) {

@@ -33,3 +33,17 @@ def test_exact_passes_match_per_call(x, y, prec, iters, extra):
         assert got[0] == want[0]
         for a, b in zip(got[1], want[1]):
             assert np.array_equal(a.view(np.int64), b.view(np.int64)), resident_mode
+
+
+@pytest.mark.parametrize("form", ["exact", "fused", "chain"])
+@pytest.mark.parametrize("x,y", [(70, 45), (611, 607), (2049, 2434)])
+def test_true_residual_exit_without_preconditioner_is_the_plain_exit(form, x, y):
+    """r.z is r.r without a preconditioner, so both exits end at one iteration."""
+    extra = "tl_arithmetic %s\n" % form
+    deck = decks.five_state_deck(x, "cg", "none", steps=2, eps=1e-3, max_iters=60, y_cells=y,
+                                 extra=extra)
+    want = run(deck, lib.DRIVER_RESIDENT, 1)
+    got = run(deck.replace(extra, extra + "tl_exit_true_residual\n"), lib.DRIVER_RESIDENT)
+    assert got[0] == want[0] and max(want[0]) > 1
+    for a, b in zip(got[1], want[1]):
+        assert np.array_equal(a.view(np.int64), b.view(np.int64))
