@@ -421,11 +421,10 @@ bool launch_jacobi_loop(const LaunchCtx& l, const Dev& d_, double* u2, const Red
 //   block, chain        56.6 / 54.7 61.3 / 59.0 67.6 / 67.2 69.2 / 69.4 72.6 / 76.1
 //   block, fused        57.8 / 56.8 62.9 / 61.1 69.2 / 69.6 71.1 / 71.8 74.8 / 79.1 79.4 / 81.6
 //   none, chain         47.9 / 42.0 50.3 / 45.0 55.5 / 52.6 59.9 / 56.8             66.9 / 65.7
-//   block, exact        85.5 / 82.9 97.1 / 90.4  105 / 100   107 / 106   116 / 115   129 / 122
+//   block, exact        84.5 / 81.5 91.4 / 88.6  101 / 98.3  104 / 104   111 / 113   121 / 119
 // So the line is where the seventh round begins; without a preconditioner and in
-// the exact form (FP64-bound either way) it is where the eighth does, from which
-// the two are within 3 % (15.0 per SM: none fused 73.6 / 75.4, block exact 132 /
-// 131).  In 16-row tiles, 32 per SM and more, the graph is ahead
+// the exact form it is where the eighth does (14.2 per SM: none fused 71.3 / 74.2,
+// block exact 124 / 127).  In 16-row tiles, 32 per SM and more, the graph is ahead
 // throughout: diagonal fused 2176^2 143 / 149, 2500^2 172 / 186, 2800^2 208 / 219.
 static int rows4_supertiles(const Dev& d) { return d.ns * (d.th / 4); }
 bool cg_loop_fits(const Dev& d, int num_sms, int arith) {
