@@ -944,7 +944,7 @@ def main():
     ap.add_argument("--ref-cells", type=int, default=32,
                     help="--mode adjoint: side of the FP64 reference-gradient problem")
     ap.add_argument("--batch-launch", default="auto", choices=["auto", "kernels", "persistent"],
-                    help="--mode batch: the autotuner's launch mode, or three kernels per "
+                    help="--mode batch: the autotuner's launch mode, or two kernels per "
                          "CG iteration, or one persistent launch per graph replay")
     ap.add_argument("--sequential", type=int, default=32,
                     help="--mode batch: problems also run one by one for comparison")

@@ -7,9 +7,10 @@
 //           the tile sums of p'.w
 //   pass B  r -= alpha w, z = M^-1 r, the tile sums of r.z
 //
-// Every value is computed by the expressions of the three kernels of the
-// graph loop from the same operands, and every sum takes the fixed order of
-// tea_device.cuh, so the results are theirs bit for bit.
+// Every value is computed by the expressions of the per-call kernels (calc_w,
+// calc_ur, calc_p) from the same operands, and every sum takes the fixed order
+// of tea_device.cuh, so the results are theirs bit for bit.  The same passes as
+// kernels of their own, for larger grids, are at the end of the file.
 #include <string.h>
 
 #include <algorithm>

@@ -1572,7 +1572,7 @@ static bool ensure_resident_state(Chunk& c) {
   if (!check_cuda(cudaMalloc(&c.res_state, sizeof(ResState)), "cudaMalloc state") ||
       !check_cuda(cudaMallocHost(&c.res_state_h, sizeof(ResState)), "cudaMallocHost state") ||
       !check_cuda(cudaMalloc(&c.res_counter, sizeof(unsigned int)), "cudaMalloc counter") ||
-      !check_cuda(cudaMalloc(&c.res_bar, 3 * sizeof(unsigned int)), "cudaMalloc barrier"))
+      !check_cuda(cudaMalloc(&c.res_bar, 2 * sizeof(unsigned int)), "cudaMalloc barrier"))
     return false;
   cudaMemsetAsync(c.res_counter, 0, sizeof(unsigned int), c.stream);
   return true;

@@ -21,7 +21,8 @@ def harness(tmp_path_factory):
         pytest.skip("no host C++ compiler or CUDA headers")
     out = str(tmp_path_factory.mktemp("launch") / "launch.so")
     include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
-    subprocess.run([cxx, "-O1", "-shared", "-fPIC", "-I", CSRC, "-I", include,
+    # -Bsymbolic: its own cudaGetLastError, not one that the process has loaded
+    subprocess.run([cxx, "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", CSRC, "-I", include,
                     os.path.join(HERE, "native", "resident_launch_harness.cpp"), "-o", out],
                    check=True)
     return ctypes.CDLL(out)
