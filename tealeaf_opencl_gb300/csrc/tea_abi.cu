@@ -204,17 +204,22 @@ Red Chunk::red() const {
   return rr;
 }
 
+static void free_fields(Chunk& c) {
+  Field* l[] = {&c.density, &c.energy0, &c.energy1, &c.volume, &c.u, &c.u0,
+                &c.p,       &c.r,       &c.w,       &c.Mi,     &c.Kx, &c.Ky,
+                &c.sd,      &c.z,       &c.cp,      &c.bfp,    &c.diag,
+                &c.r2,      &c.sd2,     &c.u2};
+  for (Field* f : l) {
+    cudaFree(f->base);
+    *f = Field();
+  }
+}
+
 static void free_chunk(Chunk& c) {
   if (!c.ready) return;
   resident_release();
   mixed_release();
-  Field* l[] = {&c.density, &c.energy0, &c.energy1, &c.volume, &c.u, &c.u0,
-                &c.p,       &c.r,       &c.w,       &c.Mi,     &c.Kx, &c.Ky,
-                &c.sd,      &c.z,       &c.cp,      &c.bfp,    &c.diag};
-  for (Field* f : l) {
-    cudaFree(f->base);
-    f->base = f->f = nullptr;
-  }
+  free_fields(c);
   double** one[] = {&c.cellx,   &c.celly,   &c.celldx,   &c.celldy,
                     &c.vertexx, &c.vertexy, &c.vertexdx, &c.vertexdy,
                     &c.red_partials, &c.red_result};
@@ -222,10 +227,11 @@ static void free_chunk(Chunk& c) {
     cudaFree(*p);
     *p = nullptr;
   }
-  cudaFree(c.red_counter);
-  c.red_counter = nullptr;
+  c.red_counter = c.res_counter = c.res_bar = nullptr;
+  c.res_state = nullptr;
   cudaFreeHost(c.host_result);
   c.host_result = nullptr;
+  c.res_state_h = nullptr;
   cudaFreeHost(c.host_map);
   c.host_map = c.host_map_dev = nullptr;
   c.red_to_host = false;
@@ -234,11 +240,6 @@ static void free_chunk(Chunk& c) {
   free(c.ppcg_alpha_h);
   free(c.ppcg_beta_h);
   c.cheby_alpha_h = c.cheby_beta_h = c.ppcg_alpha_h = c.ppcg_beta_h = nullptr;
-  cudaFree(c.r2.base);
-  cudaFree(c.sd2.base);
-  cudaFree(c.u2.base);
-  cudaFree(c.p2.base);
-  c.r2 = c.sd2 = c.u2 = c.p2 = Field();
   c.pending_inner = -1;
   tb_release();
   if (c.stream) cudaStreamDestroy(c.stream);
@@ -246,22 +247,46 @@ static void free_chunk(Chunk& c) {
   c.ready = false;
 }
 
-// optional: no memory for it is no error
-static bool alloc_field(Chunk& c, Field& f, bool optional = false) {
-  // the offset makes padded column H of every row 256-byte aligned
-  const long long off = (32 - (c.H % 32)) % 32;
-  const size_t n = (size_t)(off + c.rows * c.S + 32);
-  const cudaError_t e = cudaMalloc(&f.base, n * sizeof(double));
+// doubles of a field's allocation; element (0,0) is at field_offset, which makes
+// padded column H of every row 256-byte aligned
+static long long field_offset(const Chunk& c) { return (32 - (c.H % 32)) % 32; }
+static size_t field_doubles(const Chunk& c) {
+  return (size_t)((field_offset(c) + c.rows * c.S + 32 + 31) / 32 * 32);
+}
+
+// A zero field, with a second one behind it in the same allocation if asked for
+// (one cudaMalloc less, 80 us).  optional: no memory for it is no error.
+static bool alloc_field(Chunk& c, Field& f, bool optional = false, Field* second = nullptr) {
+  const size_t n = field_doubles(c), all = (second ? 2 : 1) * n * sizeof(double);
+  const cudaError_t e = cudaMalloc(&f.base, all);
   if (e == cudaErrorMemoryAllocation && optional) {
     cudaGetLastError();
-    f.base = nullptr;
+    f = Field();
     return false;
   }
   if (!check_cuda(e, "cudaMalloc field")) return false;
-  if (!check_cuda(cudaMemsetAsync(f.base, 0, n * sizeof(double), c.stream),
-                  "cudaMemset field"))
-    return false;
-  f.f = f.base + off;
+  if (!check_cuda(cudaMemsetAsync(f.base, 0, all, c.stream), "cudaMemset field")) return false;
+  f.f = f.base + field_offset(c);
+  if (second) second->f = f.f + n;
+  return true;
+}
+
+// Every field of a chunk.  With the spare buffer (and PPCG's second sd), too
+// little memory is no error.
+static bool alloc_fields(Chunk& c, bool spare) {
+  Field* l[] = {&c.density, &c.energy0, &c.energy1, &c.volume, &c.u, &c.u0,
+                &c.p,       &c.r,       &c.w,       &c.Mi,     &c.Kx, &c.Ky,
+                &c.sd,      &c.z,       &c.cp,      &c.bfp,    &c.diag};
+  for (Field* f : l) {
+    Field* const second = !spare                                  ? nullptr
+                          : f == &c.u                             ? &c.u2
+                          : f == &c.sd && c.solver == SOLVER_PPCG ? &c.sd2
+                                                                  : nullptr;
+    if (!alloc_field(c, *f, spare, second)) {
+      free_fields(c);
+      return false;
+    }
+  }
   return true;
 }
 
@@ -332,6 +357,9 @@ static bool config_from_tea_in(Config* cfg) {
   return true;
 }
 
+constexpr size_t kSmallBytes = 1024;  // results, counters and loop state of a chunk
+static_assert(64 * sizeof(double) + sizeof(ResState) <= kSmallBytes, "loop state");
+
 static bool init_chunk(int x_max, int y_max, const Config& cfg) {
   Chunk& c = chunk();
   free_chunk(c);
@@ -360,11 +388,9 @@ static bool init_chunk(int x_max, int y_max, const Config& cfg) {
                   "cudaStreamCreate"))
     return false;
   c.ready = true;  // so that free_chunk releases partial allocations
-  Field* l[] = {&c.density, &c.energy0, &c.energy1, &c.volume, &c.u, &c.u0,
-                &c.p,       &c.r,       &c.w,       &c.Mi,     &c.Kx, &c.Ky,
-                &c.sd,      &c.z,       &c.cp,      &c.bfp,    &c.diag};
-  for (Field* f : l)
-    if (!alloc_field(c, *f)) return false;
+  // with the spare buffer behind u, or without it where memory is short
+  const long long errors = error_count();
+  if (!alloc_fields(c, true) && (error_count() != errors || !alloc_fields(c, false))) return false;
   const int n1 = std::max(x_max, y_max) + 2 * c.H + 2;
   double** one[] = {&c.cellx,   &c.celly,   &c.celldx,   &c.celldy,
                     &c.vertexx, &c.vertexy, &c.vertexdx, &c.vertexdy};
@@ -379,11 +405,8 @@ static bool init_chunk(int x_max, int y_max, const Config& cfg) {
   c.red_stride = nsx * ((y_max + 3) / 4) + 1;
   if (!check_cuda(cudaMalloc(&c.red_partials, 8 * c.red_stride * sizeof(double)),
                   "cudaMalloc partials") ||
-      !check_cuda(cudaMalloc(&c.red_result, 8 * sizeof(double)),
-                  "cudaMalloc result") ||
-      !check_cuda(cudaMalloc(&c.red_counter, 8 * sizeof(unsigned int)),
-                  "cudaMalloc counter") ||
-      !check_cuda(cudaMallocHost(&c.host_result, 8 * sizeof(double)),
+      !check_cuda(cudaMalloc(&c.red_result, kSmallBytes), "cudaMalloc result") ||
+      !check_cuda(cudaMallocHost(&c.host_result, 8 * sizeof(double) + sizeof(ResState)),
                   "cudaMallocHost") ||
       !check_cuda(cudaHostAlloc(&c.host_map, 8 * sizeof(unsigned long long),
                                 cudaHostAllocMapped),
@@ -391,8 +414,13 @@ static bool init_chunk(int x_max, int y_max, const Config& cfg) {
       !check_cuda(cudaHostGetDevicePointer(&c.host_map_dev, c.host_map, 0),
                   "cudaHostGetDevicePointer"))
     return false;
-  cudaMemsetAsync(c.red_counter, 0, 8 * sizeof(unsigned int), c.stream);
-  cudaMemsetAsync(c.red_result, 0, 8 * sizeof(double), c.stream);
+  cudaMemsetAsync(c.red_result, 0, kSmallBytes, c.stream);
+  // counters, grid barrier and loop state behind the results, a 128-byte line each
+  c.red_counter = (unsigned int*)(c.red_result + 16);
+  c.res_counter = (unsigned int*)(c.red_result + 32);
+  c.res_bar = (unsigned int*)(c.red_result + 48);
+  c.res_state = (ResState*)(c.red_result + 64);
+  c.res_state_h = (ResState*)(c.host_result + 8);
   return check_cuda(cudaStreamSynchronize(c.stream), "chunk allocation");
 }
 
@@ -409,28 +437,28 @@ static bool need_chunk(const char* who) {
   return true;
 }
 
-bool ensure_alt_fields(Chunk& c) {
-  if (c.r2.base) return true;
-  if (!alloc_field(c, c.r2) || !alloc_field(c, c.sd2)) return false;
-  // the halos (never written by the solve) must match the live pair's
-  const size_t n = (size_t)((32 - (c.H % 32)) % 32 + c.rows * c.S + 32) * sizeof(double);
-  return check_cuda(cudaMemcpyAsync(c.r2.base, c.r.base, n, cudaMemcpyDeviceToDevice, c.stream),
-                    "alt r copy") &&
-         check_cuda(cudaMemcpyAsync(c.sd2.base, c.sd.base, n, cudaMemcpyDeviceToDevice, c.stream),
-                    "alt sd copy");
+// A second buffer with the live one's contents: its halo, which the solve never
+// writes, must match.
+static bool ensure_copy(Chunk& c, const Field& live, Field& second) {
+  if (second.f) return true;
+  const size_t n = field_doubles(c) * sizeof(double);
+  if (!check_cuda(cudaMalloc(&second.base, n), "cudaMalloc field")) return false;
+  second.f = second.base + field_offset(c);
+  return check_cuda(cudaMemcpyAsync(second.base, live.f - field_offset(c), n,
+                                    cudaMemcpyDeviceToDevice, c.stream),
+                    "second buffer copy");
 }
 
-bool ensure_u_alt(Chunk& c) { return c.u2.base || alloc_field(c, c.u2); }
-bool ensure_p_alt(Chunk& c) { return c.p2.base || alloc_field(c, c.p2); }
+bool ensure_sd_alt(Chunk& c) { return ensure_copy(c, c.sd, c.sd2); }
+bool ensure_alt_fields(Chunk& c) { return ensure_sd_alt(c) && ensure_copy(c, c.r, c.r2); }
+bool ensure_spare(Chunk& c) { return c.u2.f || alloc_field(c, c.u2); }
 
 // Asked once per chunk: a refused cudaMalloc in every call costs more than the
 // buffer saves.
-static bool have_alt(Chunk& c, Field& f, bool& refused) {
-  if (!f.base && !refused) refused = !alloc_field(c, f, true);
-  return f.base != nullptr;
+bool have_spare(Chunk& c) {
+  if (!c.u2.f && !c.u2_refused) c.u2_refused = !alloc_field(c, c.u2, true);
+  return c.u2.f != nullptr;
 }
-bool have_u_alt(Chunk& c) { return have_alt(c, c.u2, c.u2_refused); }
-bool have_p_alt(Chunk& c) { return have_alt(c, c.p2, c.p2_refused); }
 
 void swap_alt_fields(Chunk& c) {
   std::swap(c.r, c.r2);
@@ -773,7 +801,7 @@ extern "C" void tea_leaf_cg_calc_ur_kernel_ocl_(double* alpha, double* rrn) {
   // the r and z made here.  This pass forms it too, from its own z, into the
   // spare sd buffer; init_sd then only makes that buffer current, provided no
   // other call came in between (the current sd is untouched until then).
-  if (c.solver == SOLVER_PPCG && c.n_ppcg > 0 && ensure_alt_fields(c)) {
+  if (c.solver == SOLVER_PPCG && c.n_ppcg > 0 && ensure_sd_alt(c)) {
     launch_cg_calc_ur_sd(c, a, c.ppcg_theta, c.sd2.f);
     c.spec_sd_call = c.abi_calls;
     c.spec_sd_theta = c.ppcg_theta;
@@ -818,12 +846,12 @@ extern "C" void tea_leaf_cheby_iterate_kernel_ocl_(const int* cheby_calc_step) {
   }
   // calc_u folded into calc_p: the new u goes to the second buffer, which
   // then becomes u; without one a point preconditioner takes calc_p, calc_u
-  if (c.prec != PREC_JAC_BLOCK && !have_u_alt(c)) {
+  if (c.prec != PREC_JAC_BLOCK && !have_spare(c)) {
     launch_cheby_calc_pu(c, c.cheby_alpha_h[s], c.cheby_beta_h[s], nullptr);
     launch_cheby_calc_u(c);
     return;
   }
-  if (!ensure_u_alt(c)) return;
+  if (!ensure_spare(c)) return;
   launch_cheby_calc_pu(c, c.cheby_alpha_h[s], c.cheby_beta_h[s], c.u2.f);
   std::swap(c.u, c.u2);
   c.field_epoch++;
@@ -901,7 +929,7 @@ extern "C" void tea_leaf_ppcg_inner_kernel_ocl_(int* inner_step,
   flush_pending_inner(c);
   // update_r and calc_sd in one pass: the new sd goes to the second buffer,
   // which then becomes sd
-  if (!ensure_alt_fields(c)) return;
+  if (!ensure_sd_alt(c)) return;
   launch_ppcg_step(c, c.ppcg_alpha_h[s], c.ppcg_beta_h[s], c.sd.f, c.sd2.f);
   std::swap(c.sd, c.sd2);
   c.field_epoch++;
@@ -913,7 +941,7 @@ extern "C" void tea_leaf_jacobi_solve_kernel_ocl_(double* error) {
   Chunk& c = chunk();
   // the new u goes to the second buffer, which then becomes u; without one the
   // sweep reads the copy that it leaves in un
-  if (!have_u_alt(c)) {
+  if (!have_spare(c)) {
     const long long first = (long long)c.H * c.S + c.H;
     const size_t pitch = (size_t)c.S * sizeof(double);
     if (!check_cuda(cudaMemcpy2DAsync(c.Mi.f + first, pitch, c.u.f + first, pitch,
@@ -1079,7 +1107,7 @@ static int copy_field(int id, double* host, const double* in, bool padded) {
   // the second r/sd buffer keeps the same halo (the fused PPCG inner steps
   // read halos from whichever buffer is live)
   Field* alt = f == &c.r ? &c.r2 : f == &c.sd ? &c.sd2 : nullptr;
-  if (in && padded && alt && alt->base &&
+  if (in && padded && alt && alt->f &&
       !check_cuda(cudaMemcpy2DAsync(alt->f, c.S * sizeof(double), in, w * sizeof(double),
                                     w * sizeof(double), h, cudaMemcpyHostToDevice, c.stream),
                   "field copy (second buffer)"))

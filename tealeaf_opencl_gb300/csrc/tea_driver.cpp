@@ -729,12 +729,12 @@ class Driver {
         const bool one = use_ppcg && !first;
         if (mode == TEA_DRIVER_RESIDENT &&
             (use_cg || (!one && !D.verbose && !tea::kernels_timed())) &&
-            ((use_cg && D.true_exit) || tea::have_p_alt(tea::chunk()))) {
+            ((use_cg && D.true_exit) || tea::have_spare(tea::chunk()))) {
           // The whole remaining CG loop, or the CG iterations before the
           // switch to Chebyshev or PPCG, on the device; it stops exactly
           // where this loop would (same tests, same arithmetic).  While
           // kernels are timed the latter stay the separate kernels, as do
-          // both without memory for the loop's second p.
+          // both without memory for the spare buffer.
           int n_done = 0, conv = 0;
           tea::chunk().solver_checks = checks & TEA_CHECK_BREAKDOWN;
           if (tea::resident_cg_iterations(n, loop_max, rro, D.eps * initial_residual, &rro,
@@ -767,7 +767,7 @@ class Driver {
       } else if (use_jacobi && mode == TEA_DRIVER_RESIDENT && !D.verbose &&
                  !(checks & TEA_CHECK_BREAKDOWN) && !tea::kernels_timed() &&
                  tea::jacobi_loop_fits(tea::chunk().dev(), tea::chunk().num_sms) &&
-                 tea::have_u_alt(tea::chunk())) {
+                 tea::have_spare(tea::chunk())) {
         int n_done = 0, conv = 0;
         if (tea::resident_jacobi_iterations(n, loop_max, D.eps * initial_residual, &error,
                                             &n_done, &conv) != 0)

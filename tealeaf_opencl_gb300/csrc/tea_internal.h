@@ -80,7 +80,7 @@ struct ResState {
 };
 
 struct Field {
-  double* base = nullptr;  // cudaMalloc'd allocation
+  double* base = nullptr;  // cudaMalloc'd allocation; null if behind another's
   double* f = nullptr;     // element (0,0) of the padded layout
 };
 
@@ -106,8 +106,8 @@ struct Chunk {
   double* red_partials = nullptr;
   long long red_stride = 0;
   unsigned int* red_counter = nullptr;
-  double* red_result = nullptr;
-  double* host_result = nullptr;  // pinned, 8 doubles
+  double* red_result = nullptr;  // and behind it the counters and res_* below
+  double* host_result = nullptr;  // pinned, 8 doubles, then res_state_h
   unsigned long long* host_map = nullptr;      // mapped pinned: 8 results
   unsigned long long* host_map_dev = nullptr;  // its device address
   bool red_to_host = false;        // next c.red() copies its result to host_map
@@ -131,16 +131,17 @@ struct Chunk {
   cudaGraphExec_t res_ppcg_graph = nullptr;  // resident PPCG iterations
   std::vector<double> res_ppcg_key;          // theta, coefficients, form of it
   int resident_mode = 0;               // 0 by size, 1 graph replay, 2 cooperative loop
-  // second r and sd buffers for the fused pair of PPCG inner steps
-  // (tea_ppcg_tb.cu), which writes r and sd to the pair it does not read;
-  // allocated on first use, with the halos of the live pair
+  // second r and sd buffers: the one-pass inner step writes sd, the fused pair
+  // of inner steps (tea_ppcg_tb.cu) r and sd, to the buffer it does not read;
+  // made on first use, with the halos of the live ones
   Field r2, sd2;
-  // second u buffer of the Chebyshev iteration with calc_u folded into
-  // calc_p and of the Jacobi sweep, which write the new u, halo included, to the
-  // buffer it does not read; the two then trade places
+  // The spare buffer.  The Chebyshev iteration with calc_u folded into calc_p
+  // and the Jacobi sweep write the new u, halo included, to it; the two then
+  // trade places.  The resident CG loop keeps every second p in it
+  // (tea_cg_loop.cu).  Between calls it holds nothing.  Allocated with u where
+  // there is room for it.
   Field u2;
-  Field p2;  // second p buffer of the resident CG loop (tea_cg_loop.cu)
-  bool u2_refused = false, p2_refused = false;  // no memory for them
+  bool u2_refused = false;  // no memory for it
   int inner_pairs = 0;      // run PPCG inner steps in fused pairs where they apply
   int field_epoch = 0;      // bumped whenever r/sd and r2/sd2 trade places
   int pending_inner = -1;   // a per-call inner step (0-based) not launched yet
@@ -302,15 +303,14 @@ bool launch_ppcg_inner_pair(Chunk& c, int s, const ResState* st, double* r_in,
                             double* sd_in, double* r_out, double* sd_out);
 int tb_error();
 void tb_release();
-// the second r/sd buffers (tea_abi.cu): allocated and given the live
+// the second sd, or r and sd, buffers (tea_abi.cu): allocated and given the live
 // buffers' contents once; false on failure
+bool ensure_sd_alt(Chunk& c);
 bool ensure_alt_fields(Chunk& c);
-// allocates u2 / p2 on first use
-bool ensure_u_alt(Chunk& c);
-bool ensure_p_alt(Chunk& c);
-// the same where the caller has a way without: no memory for it is no error
-bool have_u_alt(Chunk& c);
-bool have_p_alt(Chunk& c);
+// allocates the spare buffer on first use; have_spare where the caller has a way
+// without: no memory for it is no error
+bool ensure_spare(Chunk& c);
+bool have_spare(Chunk& c);
 // r/sd and r2/sd2 trade places (the fused pair has just written r2/sd2)
 void swap_alt_fields(Chunk& c);
 // launches a per-call PPCG inner step held back for pairing (tea_abi.cu)

@@ -573,9 +573,9 @@ __global__ void __launch_bounds__(kBlock, 3)
 
 // The same iteration without a preconditioner or with the diagonal one:
 // p = alpha p + beta r or alpha p + (beta Mi) r, u + p to the second u buffer.
-// One pass in place of calc_p and calc_u (without a second buffer calc_p alone); 7 FP64 instructions per cell with the
-// products on the integer pipes (bit-identical), 10 with all of them on the
-// FP64 pipe.
+// One pass in place of calc_p and calc_u (U = false, without a second buffer:
+// calc_p alone); 7 FP64 instructions per cell with the products on the integer
+// pipes (bit-identical), 10 with all of them on the FP64 pipe.
 template <int F, int MB, bool EMU, bool U = true>
 __global__ void __launch_bounds__(kBlock, MB)
     k_cheby_calc_pu_point(Dev d, Red red, double alpha, double beta, double* un_) {
@@ -1541,7 +1541,7 @@ static void enqueue_ppcg_iterations(Chunk& c, int iters) {
 }
 
 static void enqueue_resident_iterations(Chunk& c, int iters, bool true_exit) {
-  enqueue_cg_passes(LaunchCtx{c.stream, c.num_sms, c.arith}, c.dev(), c.p2.f, c.red(),
+  enqueue_cg_passes(LaunchCtx{c.stream, c.num_sms, c.arith}, c.dev(), c.u2.f, c.red(),
                     c.res_state, c.res_counter, iters, true_exit);
 }
 
@@ -1551,31 +1551,12 @@ void resident_release() {
     if (g.exec) cudaGraphExecDestroy(g.exec);
     g = Chunk::CgGraph();
   }
-  cudaFree(c.res_state);
   cudaFree(c.res_coef);
-  cudaFree(c.res_counter);
-  cudaFree(c.res_bar);
-  c.res_bar = nullptr;
   if (c.res_ppcg_graph) cudaGraphExecDestroy(c.res_ppcg_graph);
   c.res_ppcg_graph = nullptr;
   c.res_ppcg_key.clear();
-  cudaFreeHost(c.res_state_h);
-  c.res_state = nullptr;
   c.res_coef = nullptr;
-  c.res_counter = nullptr;
-  c.res_state_h = nullptr;
   c.res_coef_n = 0;
-}
-
-static bool ensure_resident_state(Chunk& c) {
-  if (c.res_state) return true;
-  if (!check_cuda(cudaMalloc(&c.res_state, sizeof(ResState)), "cudaMalloc state") ||
-      !check_cuda(cudaMallocHost(&c.res_state_h, sizeof(ResState)), "cudaMallocHost state") ||
-      !check_cuda(cudaMalloc(&c.res_counter, sizeof(unsigned int)), "cudaMalloc counter") ||
-      !check_cuda(cudaMalloc(&c.res_bar, 2 * sizeof(unsigned int)), "cudaMalloc barrier"))
-    return false;
-  cudaMemsetAsync(c.res_counter, 0, sizeof(unsigned int), c.stream);
-  return true;
 }
 
 constexpr int kGraphIters = 16;  // iterations of one batch (even)
@@ -1632,7 +1613,6 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
       return -1;
     c.res_coef_n = loop_max + 2;
   }
-  if (!ensure_resident_state(c)) return -1;
   ResState& h = *c.res_state_h;
   memset(&h, 0, sizeof(h));
   h.rro = rro_in;
@@ -1648,12 +1628,12 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
                                   cudaMemcpyHostToDevice, c.stream),
                   "resident state upload"))
     return -1;
-  if (!ensure_p_alt(c)) return -1;
+  if (!ensure_spare(c)) return -1;
   if (use_cg_loop(c, true_exit)) {
     const LaunchCtx l{c.stream, c.num_sms, c.arith};
     const long long launches = (long long)(loop_max - n_begin) / kLoopLaunchIters + 2;
     for (long long k = 0;; k++) {
-      if (!launch_cg_loop(l, c.dev(), c.p2.f, c.red(), c.res_state, c.res_bar,
+      if (!launch_cg_loop(l, c.dev(), c.u2.f, c.red(), c.res_state, c.res_bar,
                           c.barrier_spin_limit, (unsigned int)c.barrier_extra) ||
           !check_cuda(cudaMemcpyAsync(&h, c.res_state, sizeof(ResState),
                                       cudaMemcpyDeviceToHost, c.stream),
@@ -1721,7 +1701,7 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
 int resident_jacobi_iterations(int n_begin, int loop_max, double eps_target, double* error_out,
                                int* n_done, int* converged) {
   Chunk& c = chunk();
-  if (!ensure_resident_state(c) || !ensure_u_alt(c)) return -1;
+  if (!ensure_spare(c)) return -1;
   ResState& h = *c.res_state_h;
   memset(&h, 0, sizeof(h));
   h.eps_target = eps_target;
@@ -1774,12 +1754,11 @@ int resident_ppcg_iterations(int n_begin, int loop_max, double rro_in,
     return -1;
   }
   const int batch = 4;
-  if (!ensure_resident_state(c)) return -1;
   flush_pending_inner(c);
   const bool pairs = resident_pairs(c);
   if (pairs && (!ensure_alt_fields(c) || !tb_prepare(c))) return -1;
   // the one-pass inner steps write sd to the second buffer
-  if (!ensure_alt_fields(c)) return -1;
+  if (!ensure_sd_alt(c)) return -1;
   std::vector<double> key = {c.ppcg_theta, (double)c.arith, (double)c.n_ppcg,
                              (double)c.field_epoch, pairs ? 1.0 : 0.0};
   key.insert(key.end(), c.ppcg_alpha_h, c.ppcg_alpha_h + c.n_ppcg);
@@ -1840,10 +1819,10 @@ int resident_ppcg_iterations(int n_begin, int loop_max, double rro_in,
   }
   if (pairs && ((long long)(h.n - n_begin + 1) * (c.n_ppcg / 2)) % 2 != 0) {
     // an odd number of fused pairs ran: the results are in r2/sd2
-    const size_t n = (size_t)((32 - (c.H % 32)) % 32 + c.rows * c.S + 32) * sizeof(double);
-    if (!check_cuda(cudaMemcpyAsync(c.r.base, c.r2.base, n, cudaMemcpyDeviceToDevice, c.stream),
+    const size_t n = (size_t)(c.rows * c.S) * sizeof(double);
+    if (!check_cuda(cudaMemcpyAsync(c.r.f, c.r2.f, n, cudaMemcpyDeviceToDevice, c.stream),
                     "resident PPCG r copy back") ||
-        !check_cuda(cudaMemcpyAsync(c.sd.base, c.sd2.base, n, cudaMemcpyDeviceToDevice,
+        !check_cuda(cudaMemcpyAsync(c.sd.f, c.sd2.f, n, cudaMemcpyDeviceToDevice,
                                     c.stream),
                     "resident PPCG sd copy back"))
       return -1;
