@@ -165,6 +165,7 @@ struct Chunk {
     int arith = 0;
     bool true_exit = false;
   } res_graph[2];
+  bool presteps_made = false;  // the loop has made CG iterations before a switch
   double res_last_rr_true = 0.0;
 
   Dev dev() const;

@@ -1559,7 +1559,7 @@ void resident_release() {
   c.res_coef_n = 0;
 }
 
-constexpr int kGraphIters = 16;  // iterations of one batch (even)
+constexpr int kGraphIters = 16;  // iterations of one replay (even)
 
 // The graph of kGraphIters iterations on the current buffers in the current
 // form, captured unless one of the two kept is that (one per buffer of u).
@@ -1651,11 +1651,19 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
       }
     }
   } else {
+  // A chunk's first iterations before a switch (PPCG makes no others here) are
+  // queued as they are: as many as there must be, then eight at a time.  For 2 to
+  // 30 of them a graph costs more than it saves (0.2 ms to make).
+  const bool direct = c.profiler_on || (switch_n > 0 && !c.presteps_made);
+  if (switch_n > 0) c.presteps_made = true;
+  int batch = kGraphIters;
+  if (direct && switch_n > 0)
+    batch = std::min(std::max(2, (std::min(switch_n, loop_max) - n_begin + 1) & ~1), 64);
   cudaGraphExec_t graph = nullptr;
-  if (!c.profiler_on && !(graph = cg_graph(c, true_exit))) return -1;
-  // every batch runs at least one iteration until the loop stops, so the
+  if (!direct && !(graph = cg_graph(c, true_exit))) return -1;
+  // every batch runs at least two iterations until the loop stops, so the
   // loop needs at most this many batches; more means the state is corrupt
-  const long long max_batches = (long long)(loop_max - n_begin) / kGraphIters + 3;
+  const long long max_batches = (long long)(loop_max - n_begin) / 2 + 3;
   for (long long nb = 0;; nb++) {
     if (nb >= max_batches) {
       fail(24, "resident CG loop did not stop after %lld batches", nb);
@@ -1665,16 +1673,17 @@ int resident_cg_iterations(int n_begin, int loop_max, double rro_in,
       if (!check_cuda(cudaGraphLaunch(graph, c.stream), "graph launch"))
         return -1;
     } else {
-      enqueue_resident_iterations(c, kGraphIters, true_exit);
+      enqueue_resident_iterations(c, batch, true_exit);
       check_cuda(cudaGetLastError(), "resident launch");
     }
-    count_launches(2 * kGraphIters + 1);
+    count_launches(2 * batch + 1);
     if (!check_cuda(cudaMemcpyAsync(&h, c.res_state, sizeof(ResState),
                                     cudaMemcpyDeviceToHost, c.stream),
                     "resident state read") ||
         !check_cuda(cudaStreamSynchronize(c.stream), "resident sync"))
       return -1;
     if (h.stop && !h.p_pending) break;
+    if (direct && switch_n > 0) batch = 8;
   }
   }
   *rro_out = h.rro;
